@@ -84,6 +84,39 @@ extern "C" void pn_params_default(pn_params *p) {
 bool pn::is_f32(const pn_ctx *c) { return c->p.precision == PN_PREC_MIXED; }
 int pn::force_mode(const pn_ctx *c) { return c->p.inv_c2 != 0.0 ? MODE_FORCE : MODE_NEWTON; }
 
+bool pn::fix_units(double eps, FixUnits *u) {
+    *u = FixUnits{};
+    if (!std::isfinite(eps)) return false;
+    u->eL = std::ilogb(eps);
+    if (u->eL < -60 || u->eL > 60) return false;
+    const double e = std::ldexp(eps, -u->eL);
+    u->eps60 = (unsigned long long)std::ldexp(e * e, 60);
+    u->inv_len = std::ldexp(1.0, -u->eL);
+    u->inv_eps = 1.0 / eps;
+    u->inv_eps3 = (double)(1.0L / ((long double)eps * eps * eps));
+    return true;
+}
+
+// Shape of the fixed-point FP64 sweep: lanes per star and j-range splits.
+static void choose_fix(PairCfg *k, int nstar, int sms) {
+    k->ipt = 1;
+    k->tj = 128;
+    k->x2 = 1;
+    const int ntiles = (nstar + 127) / 128, slots = 3 * sms;
+    double best = 1e300;
+    for (int js = 1; js <= 16; js *= 2)
+        for (int g = 1; g <= 16 && g <= ntiles; ++g) {
+            const int ctas = (nstar * js + 127) / 128 * g;
+            const double waves = (ctas + slots - 1) / slots;
+            const double cost = waves * ((double)((ntiles + g - 1) / g) * (128.0 / js + 4.0) + 6.0) + 0.5 * g;
+            if (cost < best) {
+                best = cost;
+                k->js = js;
+                k->gsplit = g;
+            }
+        }
+}
+
 // Launch shape of the pair sweep: explicit parameters win; otherwise a heuristic sized for
 // GB300 (152 SMs): enough CTAs for several waves, split along j when there are few i-blocks.
 static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
@@ -114,6 +147,11 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
         const int ntiles_t = (nstar + tuned.tj - 1) / tuned.tj;
         if (tuned.gsplit > ntiles_t) tuned.gsplit = ntiles_t;
         return tuned;
+    }
+    FixUnits fu;
+    if (!f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, &fu)) {
+        choose_fix(&k, nstar, c->sms);
+        return k;
     }
     if ((pv == PN_PAIR_F32X2 || pv == PN_PAIR_F32X2_OCC3 || pv == PN_PAIR_F32X2_OCC4) && f32) {
         if (k.ipt > 2) k.ipt = 2;
@@ -169,7 +207,7 @@ static void free_ctx(pn_ctx *c) {
     if (!c) return;
     free_adjoint(c);
     if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
-    void *bufs[] = {c->state_buf, c->a_aos, c->in_aos, c->spos, c->pack, c->pack2, c->ipack, c->torg, c->acc,
+    void *bufs[] = {c->state_buf, c->a_aos, c->in_aos, c->spos, c->pack, c->pack2, c->ipack, c->fpack, c->fix_bad, c->torg, c->acc,
                     c->part, c->glob, c->eout, c->tickets, c->err};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -243,6 +281,9 @@ extern "C" int pn_create(pn_ctx **out, int nmax, const pn_params *p) {
     if (cudaMalloc(&c->pack, 6 * np * 16) != cudaSuccess) return fail("pack");
     if (cudaMalloc(&c->pack2, 7 * (np / 2) * 16) != cudaSuccess) return fail("pack2");
     if (cudaMalloc(&c->ipack, np * 16) != cudaSuccess) return fail("ipack");
+    if (cudaMalloc(&c->fpack, FIX_GROUPS * np * 16) != cudaSuccess) return fail("fpack");
+    if (cudaMalloc(&c->fix_bad, sizeof(int)) != cudaSuccess) return fail("fix_bad");
+    if (cudaMemset(c->fix_bad, 0, sizeof(int)) != cudaSuccess) return fail("memset");
     if (cudaMemset(c->pack2, 0, 7 * (np / 2) * 16) != cudaSuccess) return fail("memset");
     if (cudaMalloc(&c->torg, (np / 32 + 1) * sizeof(TileOrigin)) != cudaSuccess) return fail("torg");
     const size_t nblk = np / 256 + 2;
@@ -316,6 +357,9 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
         pa.ipack = c->ipack;
         if (k.x2) pa.pack = nullptr;  // the packed sweep reads the paired pack only
     }
+    FixUnits fu{};
+    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
+    if (!pa.f32 && k.x2) { pa.fpack = c->fpack; pa.fix_bad = c->fix_bad; pa.fu = fu; }
     pa.part = c->part; pa.glob = c->glob; pa.ticket = &c->tickets[0];
     CU(launch_prep(pa, s));
 
@@ -323,6 +367,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     qa.pack = c->pack; qa.torg = c->torg; qa.spos = c->spos; qa.pack2 = c->pack2; qa.ipack = c->ipack; qa.out = c->acc; qa.err = c->err;
     qa.nstar = nstar; qa.npad = c->npad; qa.tj = k.tj; qa.ntiles = (nstar + k.tj - 1) / k.tj;
     qa.gsplit = k.gsplit; qa.eps2 = eps2;
+    qa.fpack = pa.fpack; qa.fix_bad = pa.fix_bad; qa.fu = fu; qa.m = m; qa.v = v; qa.vsp = sp; qa.vsk = sk;
     if (timed) CU(cudaEventRecord(c->ev0, s));
     // external event nodes, so that the events are really recorded when a captured step replays
     // (the flag is valid only while the stream is being captured)
@@ -334,6 +379,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     if (tslot >= 0) CU(cudaEventRecordWithFlags(c->evp[2 * tslot], s, cudaEventRecordExternal));
     if (nstar > 0) {
         if (is_f32(c)) CU(launch_pair_f32(mode, k, qa, s));
+        else if (k.x2) CU(launch_pair_fix(mode, k, qa, s));
         else CU(launch_pair_f64(mode, k, qa, s));
     }
     if (tslot >= 0) CU(cudaEventRecordWithFlags(c->evp[2 * tslot + 1], s, cudaEventRecordExternal));
@@ -359,7 +405,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     fa.a = a_out; fa.asp = asp; fa.ask = ask;
     fa.stage = stage; fa.st = c->st; fa.ld = c->ld; fa.sums_out = sums_out;
     fa.part = c->part + (size_t)(c->npad / 256 + 2) * 8;
-    fa.ticket = &c->tickets[1]; fa.err = c->err;
+    fa.ticket = &c->tickets[1]; fa.err = c->err; fa.fix_bad = pa.fix_bad;
     CU(launch_finish(fa, s));
     if (timed) CU(cudaEventRecord(c->ev2, s));
     c->stats.tile_j = k.tj; c->stats.i_per_thread = k.ipt; c->stats.j_split = k.js;
@@ -679,14 +725,19 @@ static int eval_energy(pn_ctx *c, const double *x, const double *v, const double
     pa.tj = k.tj; pa.f32 = is_f32(c); pa.eps2 = eps2;
     pa.pack = c->pack; pa.torg = c->torg; pa.spos = c->spos;
     if (pa.f32) { pa.pack2 = c->pack2; pa.ipack = c->ipack; }
+    FixUnits fu{};
+    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
+    if (!pa.f32 && k.x2) { pa.fpack = c->fpack; pa.fix_bad = c->fix_bad; pa.fu = fu; }
     pa.part = c->part; pa.glob = c->glob; pa.ticket = &c->tickets[0];
     CU(launch_prep(pa, s));
     PairArgs qa{};
     qa.pack = c->pack; qa.torg = c->torg; qa.spos = c->spos; qa.pack2 = c->pack2; qa.ipack = c->ipack; qa.out = c->acc; qa.err = c->err;
     qa.nstar = nstar; qa.npad = c->npad; qa.tj = k.tj; qa.ntiles = (nstar + k.tj - 1) / k.tj;
     qa.gsplit = k.gsplit; qa.eps2 = eps2;
+    qa.fpack = pa.fpack; qa.fix_bad = pa.fix_bad; qa.fu = fu; qa.m = m; qa.v = v; qa.vsp = sp; qa.vsk = sk;
     if (nstar > 0) {
         if (is_f32(c)) CU(launch_pair_f32(MODE_ENERGY, k, qa, s));
+        else if (k.x2) CU(launch_pair_fix(MODE_ENERGY, k, qa, s));
         else CU(launch_pair_f64(MODE_ENERGY, k, qa, s));
     }
     EnergyArgs ea{};
@@ -696,7 +747,7 @@ static int eval_energy(pn_ctx *c, const double *x, const double *v, const double
     ea.nacc = pair_nacc(MODE_ENERGY); ea.sphi = E_PHI; ea.spsi = E_PSI;
     ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2;
     ea.part = c->part + (size_t)(c->npad / 256 + 2) * 8;
-    ea.out = c->eout; ea.ticket = &c->tickets[2];
+    ea.out = c->eout; ea.ticket = &c->tickets[2]; ea.fix_bad = pa.fix_bad;
     CU(launch_energy_finish(ea, s));
     return read_energy(c, e);
 }

@@ -24,6 +24,8 @@ struct pn_ctx {
     void *pack = nullptr;
     float4 *pack2 = nullptr;      // paired pack of the f32x2 sweep [7][npad/2]
     float4 *ipack = nullptr;      // [npad] (v.xyz, qe)
+    uint4 *fpack = nullptr;       // pack of the fixed-point FP64 sweep [FIX_GROUPS][npad]
+    int *fix_bad = nullptr;       // raised by k_prep for a system outside that sweep's range
     pn::TileOrigin *torg = nullptr;
     double *acc = nullptr;
     int acc_splits = 0;

@@ -12,14 +12,21 @@ struct PairCfg {
     int js = 1;      // lanes sharing one i-set
     int tj = 128;    // stars per j-tile
     int gsplit = 1;  // j-range splits across CTAs
-    int x2 = 0;      // FP32 only: the packed f32x2 sweep (pn_pair2.cuh; js = 1, ipt 1 or 2);
+    int x2 = 0;      // FP32: the packed f32x2 sweep (pn_pair2.cuh; js = 1, ipt 1 or 2);
                      // 2 / 3 = the same sized for 3 / 4 CTAs per SM (ipt 2, force sweeps)
+                     // FP64: 1 = the fixed-point sweep (pn_pairfix.cuh; ipt 1, tj 128)
 };
 
 // Launches k_pair for the given precision/mode/shape (returns cudaErrorInvalidValue for an
 // unsupported (ipt, js) combination).  Implemented in pn_pair_f32.cu / pn_pair_f64.cu.
 cudaError_t launch_pair_f32(int mode, const PairCfg &c, const PairArgs &a, cudaStream_t s);
 cudaError_t launch_pair_f64(int mode, const PairCfg &c, const PairArgs &a, cudaStream_t s);
+// The FP64 sweep on the integer pipes (PairCfg::x2 = 1 in FP64; pn_pair_fix.cu): ipt 1, js 1..16,
+// tiles of 128.
+cudaError_t launch_pair_fix(int mode, const PairCfg &c, const PairArgs &a, cudaStream_t s);
+constexpr int FIX_GROUPS = 11;  // 16-byte groups per star of its pack
+// Its units for a softening; false where its range does not cover it.
+bool fix_units(double eps, FixUnits *u);
 bool pair_shape_supported(int ipt, int js);
 
 // Persistent ensemble sweep (k_pair_ens): (ipt, js) in {(1,1), (2,1), (1,4)}; tjmax = the

@@ -11,6 +11,7 @@
 // the ticket, so results do not depend on scheduling.
 #include <cstdio>
 
+#include "pn_fix.cuh"
 #include "pn_kernels.h"
 
 namespace pn {
@@ -96,6 +97,58 @@ __device__ __forceinline__ bool last_block(unsigned *ticket, int nblk) {
 }
 
 // ------------------------------------------------------------------ prep
+// The fixed-point sweep's pack of star j (pn_pairfix.cuh): s, its tile's origin o and velocity unit
+// 2^ev, v, m, mu3 and the FP64 coefficients of the W sum.  A padding star has no mass and sits at its tile's origin.
+__device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, const double *s, const double *o,
+                                         const double *v, double v2, int ev, double m, double mu3, double c1,
+                                         double c3, double k35, double qe, double m0) {
+    using namespace fix;
+    const FixUnits &u = a.fu;
+    const int e0 = expo(m0);
+    const double mscale = __hiloint2double((1023 - e0) << 20, 0);
+    constexpr double reach = (double)(1 << POS_BITS);
+    bool in = m0 > 1e-290 && m0 < 1e290 && v2 < 1e180 && fabs(s[0]) * u.inv_len < reach &&
+              fabs(s[1]) * u.inv_len < reach && fabs(s[2]) * u.inv_len < reach;
+    in = in && (m == 0.0 || (m >= m0 * 2.328306436538696e-10 && m <= m0 * 5.764607523034235e17));  // 2^-32, 2^59
+    if (real && !in) atomicOr(a.fix_bad, 1);
+    if (!in) return;
+    float hi[3], lo[3];
+    X96 x[3];
+    B2 w[3], q[3];
+    for (int k = 0; k < 3; ++k) {
+        const double r = real ? (s[k] - o[k]) * u.inv_len : 0.0;
+        hi[k] = (float)r;
+        lo[k] = (float)(r - (double)hi[k]);
+        x[k] = to_x96(real ? s[k] : o[k], u.eL);
+        w[k] = bal(to_scaled(v[k], W_MANT, 63, 60, ev));
+        q[k] = bal(to_scaled(v[k], U_MANT, 62, 62, ev));
+    }
+    int em, em3;
+    const u64 mm = mantissa(m, em), mm3 = mantissa(mu3, em3);
+    em = mm ? em - e0 : -8192;
+    em3 = mm3 ? em3 - e0 + 3 * u.eL : -8192;
+    const double gsc = __hiloint2double((1023 - 62 - 2 * u.eL) << 20, 0);
+    const double g1 = m * (c1 - 2.0 * v2) * gsc, g3 = m * c3 * gsc, kk = fma(m, c3, k35);
+    const float mf = (float)(m * mscale);
+    const float mu3f = (float)(mu3 * mscale * __hiloint2double((1023 + 3 * u.eL) << 20, 0));
+    uint4 *p = a.fpack + j;
+    const size_t n = a.npad;
+    auto fu = [](float f) { return __float_as_uint(f); };
+    auto lw = [](double d) { return (unsigned)__double2loint(d); };
+    auto hw = [](double d) { return (unsigned)__double2hiint(d); };
+    p[0] = make_uint4(fu(hi[0]), fu(hi[1]), fu(hi[2]), fu(mf));
+    p[n] = make_uint4(fu(lo[0]), fu(lo[1]), fu(lo[2]), (unsigned)em);
+    p[2 * n] = make_uint4(x[0].w0, x[0].w1, x[0].w2, x[1].w0);
+    p[3 * n] = make_uint4(x[1].w1, x[1].w2, x[2].w0, x[2].w1);
+    p[4 * n] = make_uint4(x[2].w2, (unsigned)mm, (unsigned)(mm >> 32), fu(mu3f));
+    p[5 * n] = make_uint4((unsigned)w[0].l, (unsigned)w[0].h, (unsigned)w[1].l, (unsigned)w[1].h);
+    p[6 * n] = make_uint4((unsigned)w[2].l, (unsigned)w[2].h, (unsigned)mm3, (unsigned)(mm3 >> 32));
+    p[7 * n] = make_uint4((unsigned)em3, 0u, lw(g1), hw(g1));
+    p[8 * n] = make_uint4(lw(g3), hw(g3), lw(kk), hw(kk));
+    p[9 * n] = make_uint4((unsigned)q[0].l, (unsigned)q[0].h, (unsigned)q[1].l, (unsigned)q[1].h);
+    p[10 * n] = make_uint4((unsigned)q[2].l, (unsigned)q[2].h, lw(qe), hw(qe));
+}
+
 // Per star j (particle p = j + 1): s = x_p - x_0, q = |s|^2, R = 1/sqrt(q + eps^2) (the
 // reference's rsqrt, Limit-sticky9.c:15-19), and the pack entries; global sums
 // A1 = sum m R, B3 = sum m R^3 s, C = sum m R^3 q, P = sum m v.
@@ -132,16 +185,17 @@ __device__ __forceinline__ void prep_body(const PrepArgs &a, int blk, int nblk) 
         a.spos[j] = s[0];
         a.spos[a.npad + j] = s[1];
         a.spos[2 * a.npad + j] = s[2];
+        // the tile origin (the tile's first star)
+        double o[3] = {0, 0, 0};
+        const int jt = (j / a.tj) * a.tj;
+        if ((a.f32 || a.fpack) && jt < a.nstar) {
+            const int pt = jt + 1;
+            o[0] = ld_x(a.x, a.sp, a.sk, pt, 0) - x0;
+            o[1] = ld_x(a.x, a.sp, a.sk, pt, 1) - y0;
+            o[2] = ld_x(a.x, a.sp, a.sk, pt, 2) - z0;
+        }
         if (a.f32) {
-            // position relative to the tile origin (the tile's first star) as an FP32 hi/lo pair
-            double o[3] = {0, 0, 0};
-            const int jt = (j / a.tj) * a.tj;
-            if (real) {
-                const int pt = jt + 1;
-                o[0] = ld_x(a.x, a.sp, a.sk, pt, 0) - x0;
-                o[1] = ld_x(a.x, a.sp, a.sk, pt, 1) - y0;
-                o[2] = ld_x(a.x, a.sp, a.sk, pt, 2) - z0;
-            }
+            // position relative to the tile origin as an FP32 hi/lo pair
             float hi[3], lo[3];
             for (int k = 0; k < 3; ++k) {
                 const double r = real ? s[k] - o[k] : 0.0;
@@ -189,6 +243,26 @@ __device__ __forceinline__ void prep_body(const PrepArgs &a, int blk, int nblk) 
             pk[3 * a.npad + j] = make_double2(vv[2], mu3);
             pk[4 * a.npad + j] = make_double2(c1, c3);
             pk[5 * a.npad + j] = make_double2(k35, qe);
+            if (a.fpack) {
+                // the tile's velocity unit (blocks start at tile boundaries: 256 stars, tiles of 128)
+                const double v2 = vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2];
+                const int we = __reduce_max_sync(0xffffffffu, fix::speed_exp(v2));
+                __shared__ int wev[32];
+                if ((threadIdx.x & 31) == 0) wev[threadIdx.x >> 5] = we;
+                __syncthreads();
+                const int w0 = (threadIdx.x >> 7) * 4;
+                const int ev = max(max(wev[w0], wev[w0 + 1]), max(wev[w0 + 2], wev[w0 + 3]));
+                prep_fix(a, j, real, s, o, vv, v2, ev, mj, mu3, c1, c3, k35, qe, m0);
+                if (j % a.tj == 0 && real) {  // in units of 2^eL
+                    TileOrigin t{};
+                    const double r[3] = {s[0] * a.fu.inv_len, s[1] * a.fu.inv_len, s[2] * a.fu.inv_len};
+                    t.hx = (float)r[0]; t.lx = (float)(r[0] - (double)t.hx);
+                    t.hy = (float)r[1]; t.ly = (float)(r[1] - (double)t.hy);
+                    t.hz = (float)r[2]; t.lz = (float)(r[2] - (double)t.hz);
+                    t.pad0 = __int_as_float(ev);
+                    a.torg[j / a.tj] = t;
+                }
+            }
         }
         if (real) {
             g[G_A1] = mj * R;
@@ -370,6 +444,7 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
             }
             if (b0) atomicOr(a.err, DEVERR_NONFINITE);
             if (a.stage) stage_update(a, 0, acc3);
+            if (a.fix_bad) *a.fix_bad = 0;
             *a.ticket = 0u;
         }
     }
@@ -434,6 +509,7 @@ __device__ __forceinline__ void energy_body(const EnergyArgs &a, int blk, int nb
             a.out[1] = kin;
             a.out[2] = potpn;
             a.out[3] = kin + pot + potpn + pn2;
+            if (a.fix_bad) *a.fix_bad = 0;
             *a.ticket = 0u;
         }
     }

@@ -36,6 +36,9 @@ struct PrepArgs {
     unsigned *ticket;
     float4 *pack2;  // optional (FP32): paired pack [7][npad/2] of the f32x2 sweep
     float4 *ipack;  // optional (FP32): [npad] (v.xyz, qe)
+    uint4 *fpack;   // optional (FP64): the fixed-point sweep's pack [11][npad], its flag and units
+    int *fix_bad;
+    FixUnits fu;
 };
 
 struct FinishArgs {
@@ -54,6 +57,7 @@ struct FinishArgs {
     double *part;
     unsigned *ticket;
     int *err;
+    int *fix_bad;         // optional: cleared for the next evaluation
 };
 
 struct EnergyArgs {
@@ -65,6 +69,7 @@ struct EnergyArgs {
     double eps, eps2, inv_c2;
     double *part, *out;  // out[4] = pot_n, kin_n, pot_pn, total
     unsigned *ticket;
+    int *fix_bad;        // optional: cleared for the next evaluation
 };
 
 cudaError_t launch_prep(const PrepArgs &a, cudaStream_t s);

@@ -31,6 +31,14 @@ template <typename T> struct PackVec;
 template <> struct PackVec<float> { using V = float4; };
 template <> struct PackVec<double> { using V = double2; };
 
+// Units of the fixed-point sweep (pn_fix.cuh): lengths 2^eL; eps60 = eps^2 in them with 60 fraction
+// bits; inv_len = 2^-eL; inv_eps, inv_eps3 = 1 / eps, 1 / eps^3.
+struct FixUnits {
+    int eL;
+    unsigned long long eps60;
+    double inv_len, inv_eps, inv_eps3;
+};
+
 struct PairArgs {
     const void *pack;     // [NG][npad] of PackVec<T>::V
     const TileOrigin *torg;  // FP32 only: per-tile FP64 origin (BH-relative), one per tile of tj
@@ -45,6 +53,13 @@ struct PairArgs {
     int ntiles;           // ceil(nstar / tj)
     int gsplit;           // j-range splits (gridDim.y)
     double eps2;
+    // the fixed-point FP64 sweep (pn_pairfix.cuh): its pack [11][npad], the flag that k_prep raises
+    // for a system outside its range, the state's masses and velocities, and its units
+    const uint4 *fpack;
+    const int *fix_bad;
+    const double *m, *v;
+    long long vsp, vsk;
+    FixUnits fu;
 };
 
 constexpr int PAIR_NT = 128;
