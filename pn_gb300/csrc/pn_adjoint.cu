@@ -900,7 +900,7 @@ static int adj_ensure(pn_ctx *c) {
                     mal((void **)&w->m0bar, 2 * 8) && mal((void **)&w->tickets, 4 * sizeof(unsigned)) &&
                     mal((void **)&w->work, 12 * 3 * ld * 8) && mal(&w->vpack, 6 * np * 16) &&
                     mal((void **)&w->vtorg, (np / 32 + 1) * sizeof(TileOrigin)) &&
-                    mal((void **)&w->vspos, 3 * np * 8) && mal((void **)&w->vpart, (np / 256 + 2) * 8 * 2 * 8) &&
+                    mal((void **)&w->vspos, 3 * np * 8) && mal((void **)&w->vpart, on_blocks(c->npad) * 8 * 2 * 8) &&
                     mal((void **)&w->vglob, 16 * 8);
     if (!ok) {
         free_adjoint(c);

@@ -286,7 +286,7 @@ extern "C" int pn_create(pn_ctx **out, int nmax, const pn_params *p) {
     if (cudaMemset(c->fix_bad, 0, sizeof(int)) != cudaSuccess) return fail("memset");
     if (cudaMemset(c->pack2, 0, 7 * (np / 2) * 16) != cudaSuccess) return fail("memset");
     if (cudaMalloc(&c->torg, (np / 32 + 1) * sizeof(TileOrigin)) != cudaSuccess) return fail("torg");
-    const size_t nblk = np / 256 + 2;
+    const size_t nblk = on_blocks(c->npad);
     if (cudaMalloc(&c->part, nblk * 8 * 2 * sizeof(double)) != cudaSuccess) return fail("part");
     if (cudaMalloc(&c->glob, 16 * sizeof(double)) != cudaSuccess) return fail("glob");
     if (cudaMalloc(&c->eout, 4 * sizeof(double)) != cudaSuccess) return fail("eout");
@@ -390,8 +390,8 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
         ea.spos = c->spos; ea.acc = c->acc; ea.glob = c->glob;
         ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit;
         ea.nacc = pair_nacc(mode); ea.sphi = A_PHI; ea.spsi = A_PSI;
-        ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2;
-        ea.part = c->part + (size_t)(c->npad / 256 + 2) * 8;
+        ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2; ea.inv_eps = 1.0 / c->p.eps;
+        ea.part = c->part + on_blocks(c->npad) * 8;
         ea.out = c->eout; ea.ticket = &c->tickets[2];
         CU(launch_energy_finish(ea, s));
     }
@@ -401,10 +401,10 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     fa.spos = c->spos; fa.acc = c->acc; fa.glob = c->glob;
     fa.nstar = nstar; fa.npad = c->npad; fa.nacc = pair_nacc(mode); fa.gsplit = k.gsplit;
     fa.pn1 = mode_has_force(mode) && c->p.inv_c2 != 0.0;
-    fa.eps = c->p.eps; fa.eps2 = eps2; fa.inv_c2 = c->p.inv_c2; fa.dt = c->p.dt;
+    fa.eps = c->p.eps; fa.eps2 = eps2; fa.inv_c2 = c->p.inv_c2; fa.dt = c->p.dt; fa.inv_eps = 1.0 / c->p.eps;
     fa.a = a_out; fa.asp = asp; fa.ask = ask;
     fa.stage = stage; fa.st = c->st; fa.ld = c->ld; fa.sums_out = sums_out;
-    fa.part = c->part + (size_t)(c->npad / 256 + 2) * 8;
+    fa.part = c->part + on_blocks(c->npad) * 8;
     fa.ticket = &c->tickets[1]; fa.err = c->err; fa.fix_bad = pa.fix_bad;
     CU(launch_finish(fa, s));
     if (timed) CU(cudaEventRecord(c->ev2, s));
@@ -745,8 +745,8 @@ static int eval_energy(pn_ctx *c, const double *x, const double *v, const double
     ea.spos = c->spos; ea.acc = c->acc; ea.glob = c->glob;
     ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit;
     ea.nacc = pair_nacc(MODE_ENERGY); ea.sphi = E_PHI; ea.spsi = E_PSI;
-    ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2;
-    ea.part = c->part + (size_t)(c->npad / 256 + 2) * 8;
+    ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2; ea.inv_eps = 1.0 / c->p.eps;
+    ea.part = c->part + on_blocks(c->npad) * 8;
     ea.out = c->eout; ea.ticket = &c->tickets[2]; ea.fix_bad = pa.fix_bad;
     CU(launch_energy_finish(ea, s));
     return read_energy(c, e);

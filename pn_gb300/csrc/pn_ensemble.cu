@@ -8,7 +8,7 @@
 // set of arrays with row stride S (the total slot count).
 //
 // One force evaluation of the whole ensemble is three launches:
-//   k_prep_ens    every cluster's 256-slot blocks (per-cluster reductions by per-cluster
+//   k_prep_ens    every cluster's blocks of slots (per-cluster reductions by per-cluster
 //                 last-block tickets)
 //   k_pair_ens    ONE persistent launch over the (cluster, i-block, j-range) work items of all
 //                 clusters, biggest first, fetched from a global counter
@@ -66,7 +66,7 @@ struct pn_ens {
     int nc = 0;
     std::vector<int> n, p0, s0, slots, blk0, nblk;
     std::vector<double> eps;
-    int P = 0, S = 0, LD = 0, B = 0;  // particles, star slots, state leading dim, 256-blocks
+    int P = 0, S = 0, LD = 0, B = 0;  // particles, star slots, state leading dim, O(N) blocks
     pn_params p{};
     int ipt = 2, js = 1;
     int x2 = 0;  // mixed precision: the packed FP32x2 sweep (js = 1)
@@ -218,6 +218,7 @@ static int ens_build_tables(pn_ens *e) {
             fa.eps2 = eps2;
             fa.inv_c2 = e->p.inv_c2;
             fa.dt = e->p.dt;
+            fa.inv_eps = 1.0 / eps;
             fa.a = stg == 0 ? e->a_aos + 3 * (size_t)e->p0[c] : nullptr;
             fa.asp = 3;
             fa.ask = 1;
@@ -246,6 +247,7 @@ static int ens_build_tables(pn_ens *e) {
         ea.eps = eps;
         ea.eps2 = eps2;
         ea.inv_c2 = e->p.inv_c2;
+        ea.inv_eps = 1.0 / eps;
         ea.part = e->fpart + (size_t)e->blk0[c] * 8;
         ea.out = e->eout + (size_t)c * 4;
         ea.ticket = &e->tickets[c * 4 + 2];
@@ -344,10 +346,10 @@ extern "C" int pn_ens_create(pn_ens **out, int nclusters, const int *n, const do
         e->blk0.push_back(B);
         const int slots = (int)std::max<long long>(256, rup(n[c] - 1, 256));
         e->slots.push_back(slots);
-        e->nblk.push_back(slots / 256);
+        e->nblk.push_back(slots / ON_NT);
         P += n[c];
         S += slots;
-        B += slots / 256;
+        B += slots / ON_NT;
     }
     e->P = P;
     e->S = S;

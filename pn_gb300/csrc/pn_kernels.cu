@@ -34,53 +34,62 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
     return DD{t, e - (t - s)};
 }
 
-// Block-wide reduction of NV doubles (fixed order: warp butterfly, then warps in order).
-// Result valid in thread 0.  'scratch' holds >= 32*NV doubles.
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double *scratch) {
+// Sums over the block, NQ (8 or 4) values per thread, in a fixed order.  Within a warp the lanes
+// first trade halves of the values (each keeps and adds one half), so that NQ values take NQ - 1
+// additions down to one value per lane and log2(32 / NQ) more across the remaining lanes: 9 FP64
+// additions for 8 values instead of 40, which matters at one FP64 warp instruction per 64 cycles.
+// Then thread q < NQ adds the warps' sums in order; the result is thread q's.  Every thread calls;
+// scratch holds (blockDim.x / 32) * NQ values and is free again on return.
+template <int NQ, typename T, typename Add, typename Shfl>
+__device__ __forceinline__ T block_sum(T (&v)[NQ], T *scratch, Add add, Shfl shfl) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int off = 16;
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
+    for (int h = NQ / 2; h >= 1; h >>= 1, off >>= 1) {
+        const bool up = lane & off;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) scratch[warp * NV + q] = v[q];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double s = 0.0;
-            for (int w = 0; w < nw; ++w) s += scratch[w * NV + q];
-            v[q] = s;
+        for (int q = 0; q < h; ++q) {
+            const T give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+            v[q] = add(keep, shfl(give, off));
         }
     }
+    constexpr int PER = 32 / NQ;  // lanes that hold partial sums of the same value
+#pragma unroll
+    for (int o = PER / 2; o >= 1; o >>= 1) v[0] = add(v[0], shfl(v[0], o));
+    if (lane % PER == 0) scratch[warp * NQ + lane / PER] = v[0];
     __syncthreads();
+    T r = scratch[threadIdx.x % NQ];
+    if (threadIdx.x < NQ)
+        for (int w = 1; w < nw; ++w) r = add(r, scratch[w * NQ + threadIdx.x]);
+    __syncthreads();
+    return r;
 }
-
-template <int NV>
-__device__ __forceinline__ void block_sum_dd(DD (&v)[NV], DD *scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            DD o{__shfl_xor_sync(0xffffffffu, v[q].hi, off), __shfl_xor_sync(0xffffffffu, v[q].lo, off)};
-            v[q] = dd_add(v[q], o);
-        }
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) scratch[warp * NV + q] = v[q];
+template <int NQ>
+__device__ __forceinline__ double block_sum(double (&v)[NQ], double *scratch) {
+    return block_sum<NQ, double>(
+        v, scratch, [](double a, double b) { return a + b; },
+        [](double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); });
+}
+template <int NQ>
+__device__ __forceinline__ DD block_sum(DD (&v)[NQ], DD *scratch) {
+    return block_sum<NQ, DD>(v, scratch, dd_add, [](DD a, int o) {
+        return DD{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
+    });
+}
+// The same over nblk block partials part[b * NQ + q] (thread t adds the blocks t / NQ, t / NQ +
+// blockDim.x / NQ, ... of value t % NQ, then the threads of a value are added in order): the
+// result is thread q's, q < NQ.  scratch holds blockDim.x values.
+template <int NQ, typename T, typename Add, typename Load>
+__device__ __forceinline__ T partials_sum(int nblk, T zero, T *scratch, Add add, Load load) {
+    const int q = threadIdx.x % NQ, first = threadIdx.x / NQ, step = blockDim.x / NQ;
+    T t = zero;
+    for (int b = first; b < nblk; b += step) t = add(t, load(b, q));
+    scratch[threadIdx.x] = t;
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            DD s{0.0, 0.0};
-            for (int w = 0; w < nw; ++w) s = dd_add(s, scratch[w * NV + q]);
-            v[q] = s;
-        }
-    }
-    __syncthreads();
+    const int have = min(step, nblk);
+    if (threadIdx.x < NQ)
+        for (int k = 1; k < have; ++k) t = add(t, scratch[k * NQ + threadIdx.x]);
+    return t;
 }
 
 // Last-CTA election after each CTA published its partial.
@@ -96,6 +105,43 @@ __device__ __forceinline__ bool last_block(unsigned *ticket, int nblk) {
     return am_last;
 }
 
+// ------------------------------------------------------------------ conversions off the FP64 pipe
+// A double rounded to FP32, and as an FP32 pair hi = fl32(x), lo = fl32(x - hi), by integer
+// operations (an FP64 conversion or subtraction costs 64 cycles of the FP64 pipe per warp); exponents
+// that leave FP32's range, infinities and NaN take the FP64 instructions.
+__device__ __forceinline__ bool f32_range(double x) {
+    const int be = (__double2hiint(x) >> 20) & 0x7ff;
+    return be - 943u < 180u;  // 2^-80 <= |x| < 2^100
+}
+__device__ __forceinline__ float f32_bits(long long b) {  // of |x|'s bits plus the rounding bit
+    return __uint_as_float((unsigned)(b >> 29) - (896u << 23));
+}
+__device__ __forceinline__ float to_f32(double x) {
+    if (!f32_range(x)) return (float)x;
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    return copysignf(f32_bits(b + 0x10000000LL), __int_as_float(__double2hiint(x)));
+}
+__device__ __forceinline__ void to_f32_pair(double x, float &hi, float &lo) {
+    if (!f32_range(x)) {
+        hi = (float)x;
+        lo = (float)(x - (double)hi);
+        return;
+    }
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    int low = (int)(b & 0x1fffffff);
+    if (low >= 0x10000000) low -= 0x20000000;  // hi was rounded up
+    const float sg = __int_as_float((__double2hiint(x) & 0x80000000) | 0x3f800000);
+    const int e = (int)(b >> 52) - 1023 - 52;  // the unit of x's last bit
+    hi = sg * f32_bits(b + 0x10000000LL);
+    lo = sg * ((float)low * __int_as_float((e + 127 + 30) << 23)) * 9.31322574615478515625e-10f;  // 2^-30
+}
+// x 2^e
+__device__ __forceinline__ double scale2(double x, int e) {
+    const int be = (__double2hiint(x) >> 20) & 0x7ff;
+    if (be == 0 || be == 0x7ff || be + e <= 0 || be + e >= 0x7ff) return ldexp(x, e);
+    return __hiloint2double(__double2hiint(x) + (e << 20), __double2loint(x));
+}
+
 // ------------------------------------------------------------------ prep
 // The fixed-point sweep's pack of star j (pn_pairfix.cuh): s, its tile's origin o and velocity unit
 // 2^ev, v, m, mu3 and the FP64 coefficients of the W sum.  A padding star has no mass and sits at its tile's origin.
@@ -105,20 +151,21 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     using namespace fix;
     const FixUnits &u = a.fu;
     const int e0 = expo(m0);
-    const double mscale = __hiloint2double((1023 - e0) << 20, 0);
-    constexpr double reach = (double)(1 << POS_BITS);
-    bool in = m0 > 1e-290 && m0 < 1e290 && v2 < 1e180 && fabs(s[0]) * u.inv_len < reach &&
-              fabs(s[1]) * u.inv_len < reach && fabs(s[2]) * u.inv_len < reach;
-    in = in && (m == 0.0 || (m >= m0 * 2.328306436538696e-10 && m <= m0 * 5.764607523034235e17));  // 2^-32, 2^59
+    auto ebits = [](double d) { return (__double2hiint(d) >> 20) & 0x7ff; };  // 0x7ff: not finite
+    bool in = ebits(m0) > 60 && ebits(m0) < 1986 && ebits(v2) < 1023 + 2 * EV_MAX - 10;
+    for (int k = 0; k < 3; ++k) in = in && ebits(s[k]) < 1023 + POS_BITS + u.eL;
+    // m: 0, or 2^-32 .. 2^59 of m0
+    in = in && (__double2hiint(m) >= 0) && (m == 0.0 || (ebits(m) >= 1023 + e0 - 32 && ebits(m) < 1023 + e0 + 59));
     if (real && !in) atomicOr(a.fix_bad, 1);
     if (!in) return;
     float hi[3], lo[3];
     X96 x[3];
     B2 w[3], q[3];
+    const float down = __int_as_float((127 - u.eL) << 23);
     for (int k = 0; k < 3; ++k) {
-        const double r = real ? (s[k] - o[k]) * u.inv_len : 0.0;
-        hi[k] = (float)r;
-        lo[k] = (float)(r - (double)hi[k]);
+        to_f32_pair(real ? s[k] - o[k] : 0.0, hi[k], lo[k]);
+        hi[k] *= down;
+        lo[k] *= down;
         x[k] = to_x96(real ? s[k] : o[k], u.eL);
         w[k] = bal(to_scaled(v[k], W_MANT, 63, 60, ev));
         q[k] = bal(to_scaled(v[k], U_MANT, 62, 62, ev));
@@ -127,10 +174,8 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     const u64 mm = mantissa(m, em), mm3 = mantissa(mu3, em3);
     em = mm ? em - e0 : -8192;
     em3 = mm3 ? em3 - e0 + 3 * u.eL : -8192;
-    const double gsc = __hiloint2double((1023 - 62 - 2 * u.eL) << 20, 0);
-    const double g1 = m * (c1 - 2.0 * v2) * gsc, g3 = m * c3 * gsc, kk = fma(m, c3, k35);
-    const float mf = (float)(m * mscale);
-    const float mu3f = (float)(mu3 * mscale * __hiloint2double((1023 + 3 * u.eL) << 20, 0));
+    const double g1 = scale2(m * fma(-2.0, v2, c1), -62 - 2 * u.eL), g3 = scale2(m * c3, -62 - 2 * u.eL), kk = fma(m, c3, k35);
+    const float mf = to_f32(scale2(m, -e0)), mu3f = to_f32(scale2(mu3, 3 * u.eL - e0));
     uint4 *p = a.fpack + j;
     const size_t n = a.npad;
     auto fu = [](float f) { return __float_as_uint(f); };
@@ -149,154 +194,149 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     p[10 * n] = make_uint4((unsigned)q[2].l, (unsigned)q[2].h, lw(qe), hw(qe));
 }
 
-// Per star j (particle p = j + 1): s = x_p - x_0, q = |s|^2, R = 1/sqrt(q + eps^2) (the
+// Per star j (particle p = j + 1): s = x_p - x_0, q = |s|^2, R = (q + eps^2)^(-1/2) (the
 // reference's rsqrt, Limit-sticky9.c:15-19), and the pack entries; global sums
 // A1 = sum m R, B3 = sum m R^3 s, C = sum m R^3 q, P = sum m v.
+//
+// Bound by the latency of its FP64 instructions (64 cycles each per warp and scheduler, so a block
+// is four warps, one per scheduler): conversions and scalings by powers of two are integer
+// operations, the square root and its inverse one rsqrt, the block's sums 9 additions per warp.
 __device__ __forceinline__ void prep_body(const PrepArgs &a, int blk, int nblk) {
-    __shared__ double red[32 * NGLOB];
-    const int j = blk * blockDim.x + threadIdx.x;
-    const double eps2 = a.eps2;
+    __shared__ double red[ON_NT];
+    const int j = blk * ON_NT + threadIdx.x;
     const double x0 = ld_x(a.x, a.sp, a.sk, 0, 0), y0 = ld_x(a.x, a.sp, a.sk, 0, 1),
                  z0 = ld_x(a.x, a.sp, a.sk, 0, 2);
     const double m0 = a.m[0];
-    double g[NGLOB];
-#pragma unroll
-    for (int q = 0; q < NGLOB; ++q) g[q] = 0.0;
-
-    if (j < a.nfill) {
-        const bool real = j < a.nstar;
-        double s[3] = {0, 0, 0}, vv[3] = {0, 0, 0}, mj = 0, R = 0, q = 0;
-        if (real) {
-            const int p = j + 1;
-            s[0] = ld_x(a.x, a.sp, a.sk, p, 0) - x0;
-            s[1] = ld_x(a.x, a.sp, a.sk, p, 1) - y0;
-            s[2] = ld_x(a.x, a.sp, a.sk, p, 2) - z0;
-            vv[0] = ld_x(a.v, a.sp, a.sk, p, 0);
-            vv[1] = ld_x(a.v, a.sp, a.sk, p, 1);
-            vv[2] = ld_x(a.v, a.sp, a.sk, p, 2);
-            mj = a.m[p];
-            q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
-            R = 1.0 / sqrt(q + eps2);
+    const bool real = j < a.nstar;
+    double s[3] = {0, 0, 0}, vv[3] = {0, 0, 0}, o[3] = {0, 0, 0}, mj = 0, R = 0, q = 0, qe = 0;
+    if (real) {
+        const int p = j + 1;
+        s[0] = ld_x(a.x, a.sp, a.sk, p, 0) - x0;
+        s[1] = ld_x(a.x, a.sp, a.sk, p, 1) - y0;
+        s[2] = ld_x(a.x, a.sp, a.sk, p, 2) - z0;
+        vv[0] = ld_x(a.v, a.sp, a.sk, p, 0);
+        vv[1] = ld_x(a.v, a.sp, a.sk, p, 1);
+        vv[2] = ld_x(a.v, a.sp, a.sk, p, 2);
+        mj = a.m[p];
+        q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+        qe = q + a.eps2;
+        R = rsqrt(qe);
+    }
+    const double R3 = R * R * R;
+    const double mu3 = mj * R3;
+    const double c1 = (1.25 * m0) * R, c3 = (0.25 * m0) * R3, k35 = (3.5 * m0) * mu3;
+    const double v2 = vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2];
+    // the tile origin (the tile's first star)
+    const int jt = (j / a.tj) * a.tj;
+    if ((a.f32 || a.fpack) && jt < a.nstar) {
+        o[0] = ld_x(a.x, a.sp, a.sk, jt + 1, 0) - x0;
+        o[1] = ld_x(a.x, a.sp, a.sk, jt + 1, 1) - y0;
+        o[2] = ld_x(a.x, a.sp, a.sk, jt + 1, 2) - z0;
+    }
+    a.spos[j] = s[0];
+    a.spos[a.npad + j] = s[1];
+    a.spos[2 * a.npad + j] = s[2];
+    if (a.f32) {
+        // position relative to the tile origin as an FP32 hi/lo pair
+        float hi[3], lo[3], v[3];
+        for (int k = 0; k < 3; ++k) {
+            to_f32_pair(real ? s[k] - o[k] : 0.0, hi[k], lo[k]);
+            v[k] = to_f32(vv[k]);
         }
-        const double R3 = R * R * R;
-        const double mu3 = mj * R3;
-        const double c1 = 1.25 * m0 * R, c3 = 0.25 * m0 * R3, k35 = 3.5 * m0 * mu3;
-        const double qe = real ? q + eps2 : 0.0;
-        a.spos[j] = s[0];
-        a.spos[a.npad + j] = s[1];
-        a.spos[2 * a.npad + j] = s[2];
-        // the tile origin (the tile's first star)
-        double o[3] = {0, 0, 0};
-        const int jt = (j / a.tj) * a.tj;
-        if ((a.f32 || a.fpack) && jt < a.nstar) {
-            const int pt = jt + 1;
-            o[0] = ld_x(a.x, a.sp, a.sk, pt, 0) - x0;
-            o[1] = ld_x(a.x, a.sp, a.sk, pt, 1) - y0;
-            o[2] = ld_x(a.x, a.sp, a.sk, pt, 2) - z0;
+        const float qf = to_f32(qe), c3f = to_f32(c3);
+        if (a.pack) {  // the scalar sweep's pack (not needed when only the packed sweep runs)
+            float4 *pk = static_cast<float4 *>(a.pack);
+            pk[j] = make_float4(hi[0], hi[1], hi[2], to_f32(mj));
+            pk[a.npad + j] = make_float4(lo[0], lo[1], lo[2], to_f32(mu3));
+            pk[2 * a.npad + j] = make_float4(v[0], v[1], v[2], qf);
+            pk[3 * a.npad + j] = make_float4(to_f32(c1), c3f, to_f32(k35), 0.f);
         }
-        if (a.f32) {
-            // position relative to the tile origin as an FP32 hi/lo pair
-            float hi[3], lo[3];
-            for (int k = 0; k < 3; ++k) {
-                const double r = real ? s[k] - o[k] : 0.0;
-                hi[k] = (float)r;
-                lo[k] = (float)(r - (double)hi[k]);
+        if (a.pack2) {  // paired layout: star j is lane (j & 1) of pair j / 2; scaled
+            const int lane = j & 1;
+            const size_t prow = (size_t)a.npad / 2;
+            float *p2 = reinterpret_cast<float *>(a.pack2 + j / 2);
+            constexpr double K = X2_K, IK = 1.0 / K, IK3 = 1.0 / (K * K * K);
+            const float vals[7][2] = {{hi[0], hi[1]},
+                                      {hi[2], to_f32(mj * IK3)},
+                                      {lo[0], lo[1]},
+                                      {lo[2], to_f32(mu3 * IK)},
+                                      {to_f32(X2_SQRT3 * vv[0]), to_f32(X2_SQRT3 * vv[1])},
+                                      {to_f32(X2_SQRT3 * vv[2]), to_f32(fma(-2.0, v2, c1))},
+                                      {c3f, to_f32(k35 * IK)}};
+            for (int g = 0; g < 7; ++g) {
+                p2[g * prow * 4 + lane] = vals[g][0];
+                p2[g * prow * 4 + 2 + lane] = vals[g][1];
             }
-            if (a.pack) {  // the scalar sweep's pack (not needed when only the packed sweep runs)
-                float4 *pk = static_cast<float4 *>(a.pack);
-                pk[j] = make_float4(hi[0], hi[1], hi[2], (float)mj);
-                pk[a.npad + j] = make_float4(lo[0], lo[1], lo[2], (float)mu3);
-                pk[2 * a.npad + j] = make_float4((float)vv[0], (float)vv[1], (float)vv[2], (float)qe);
-                pk[3 * a.npad + j] = make_float4((float)c1, (float)c3, (float)k35, 0.f);
-            }
-            if (a.pack2) {  // paired layout: star j is lane (j & 1) of pair j / 2; scaled
-                const int lane = j & 1;
-                const size_t prow = (size_t)a.npad / 2;
-                float *p2 = reinterpret_cast<float *>(a.pack2 + j / 2);
-                const double K = X2_K, v2 = vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2];
-                const float vals[7][2] = {{hi[0], hi[1]},
-                                          {hi[2], (float)(mj / (K * K * K))},
-                                          {lo[0], lo[1]},
-                                          {lo[2], (float)(mu3 / K)},
-                                          {(float)(X2_SQRT3 * vv[0]), (float)(X2_SQRT3 * vv[1])},
-                                          {(float)(X2_SQRT3 * vv[2]), (float)(c1 - 2.0 * v2)},
-                                          {(float)c3, (float)(k35 / K)}};
-                for (int g = 0; g < 7; ++g) {
-                    p2[g * prow * 4 + lane] = vals[g][0];
-                    p2[g * prow * 4 + 2 + lane] = vals[g][1];
-                }
-                a.ipack[j] = make_float4((float)vv[0], (float)vv[1], (float)vv[2], (float)qe);
-            }
-            if (j % a.tj == 0 && real) {
-                TileOrigin o{s[0], s[1], s[2], 0.0};
-                o.hx = (float)s[0]; o.lx = (float)(s[0] - (double)o.hx);
-                o.hy = (float)s[1]; o.ly = (float)(s[1] - (double)o.hy);
-                o.hz = (float)s[2]; o.lz = (float)(s[2] - (double)o.hz);
-                o.pad0 = o.pad1 = 0.f;
-                a.torg[j / a.tj] = o;
-            }
-        } else {
-            double2 *pk = static_cast<double2 *>(a.pack);
-            pk[j] = make_double2(s[0], s[1]);
-            pk[a.npad + j] = make_double2(s[2], mj);
-            pk[2 * a.npad + j] = make_double2(vv[0], vv[1]);
-            pk[3 * a.npad + j] = make_double2(vv[2], mu3);
-            pk[4 * a.npad + j] = make_double2(c1, c3);
-            pk[5 * a.npad + j] = make_double2(k35, qe);
-            if (a.fpack) {
-                // the tile's velocity unit (blocks start at tile boundaries: 256 stars, tiles of 128)
-                const double v2 = vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2];
-                const int we = __reduce_max_sync(0xffffffffu, fix::speed_exp(v2));
-                __shared__ int wev[32];
-                if ((threadIdx.x & 31) == 0) wev[threadIdx.x >> 5] = we;
-                __syncthreads();
-                const int w0 = (threadIdx.x >> 7) * 4;
-                const int ev = max(max(wev[w0], wev[w0 + 1]), max(wev[w0 + 2], wev[w0 + 3]));
-                prep_fix(a, j, real, s, o, vv, v2, ev, mj, mu3, c1, c3, k35, qe, m0);
-                if (j % a.tj == 0 && real) {  // in units of 2^eL
-                    TileOrigin t{};
-                    const double r[3] = {s[0] * a.fu.inv_len, s[1] * a.fu.inv_len, s[2] * a.fu.inv_len};
-                    t.hx = (float)r[0]; t.lx = (float)(r[0] - (double)t.hx);
-                    t.hy = (float)r[1]; t.ly = (float)(r[1] - (double)t.hy);
-                    t.hz = (float)r[2]; t.lz = (float)(r[2] - (double)t.hz);
-                    t.pad0 = __int_as_float(ev);
-                    a.torg[j / a.tj] = t;
-                }
-            }
+            a.ipack[j] = make_float4(v[0], v[1], v[2], qf);
         }
-        if (real) {
-            g[G_A1] = mj * R;
-            g[G_B3X] = mu3 * s[0];
-            g[G_B3Y] = mu3 * s[1];
-            g[G_B3Z] = mu3 * s[2];
-            g[G_C] = mu3 * q;
-            g[G_PX] = mj * vv[0];
-            g[G_PY] = mj * vv[1];
-            g[G_PZ] = mj * vv[2];
+        if (j % a.tj == 0 && real) {
+            TileOrigin t{s[0], s[1], s[2], 0.0};
+            to_f32_pair(s[0], t.hx, t.lx);
+            to_f32_pair(s[1], t.hy, t.ly);
+            to_f32_pair(s[2], t.hz, t.lz);
+            t.pad0 = t.pad1 = 0.f;
+            a.torg[j / a.tj] = t;
+        }
+    } else {
+        double2 *pk = static_cast<double2 *>(a.pack);
+        pk[j] = make_double2(s[0], s[1]);
+        pk[a.npad + j] = make_double2(s[2], mj);
+        pk[2 * a.npad + j] = make_double2(vv[0], vv[1]);
+        pk[3 * a.npad + j] = make_double2(vv[2], mu3);
+        pk[4 * a.npad + j] = make_double2(c1, c3);
+        pk[5 * a.npad + j] = make_double2(k35, qe);
+        if (a.fpack) {
+            // the tile's velocity unit (a block is one tile of 128)
+            static_assert(ON_NT == 128, "one tile per block");
+            __shared__ int wev[4];
+            const int we = __reduce_max_sync(0xffffffffu, fix::speed_exp(v2));
+            if ((threadIdx.x & 31) == 0) wev[threadIdx.x >> 5] = we;
+            __syncthreads();
+            const int ev = max(max(wev[0], wev[1]), max(wev[2], wev[3]));
+            prep_fix(a, j, real, s, o, vv, v2, ev, mj, mu3, c1, c3, k35, qe, m0);
+            if (j % a.tj == 0 && real) {  // in units of 2^eL
+                TileOrigin t{};
+                const float down = __int_as_float((127 - a.fu.eL) << 23);
+                to_f32_pair(s[0], t.hx, t.lx);
+                to_f32_pair(s[1], t.hy, t.ly);
+                to_f32_pair(s[2], t.hz, t.lz);
+                t.hx *= down; t.hy *= down; t.hz *= down;
+                t.lx *= down; t.ly *= down; t.lz *= down;
+                t.pad0 = __int_as_float(ev);
+                a.torg[j / a.tj] = t;
+            }
         }
     }
-    block_sum<NGLOB>(g, red);
-    if (threadIdx.x == 0)
-        for (int q = 0; q < NGLOB; ++q) a.part[(size_t)blk * NGLOB + q] = g[q];
+    // (mj = mu3 = 0 and finite s, q, v for a slot without a star)
+    double g[8] = {mj * R, mu3 * s[0], mu3 * s[1], mu3 * s[2], mu3 * q, mj * vv[0], mj * vv[1], mj * vv[2]};
+    static_assert(NGLOB == 8 && G_A1 == 0 && G_B3X == 1 && G_C == 4 && G_PX == 5, "order of g");
+    const double r = block_sum<8>(g, red);
+    if (threadIdx.x < 8) a.part[(size_t)blk * 8 + threadIdx.x] = r;
     if (last_block(a.ticket, nblk)) {
-        double t[NGLOB];
-        for (int q = 0; q < NGLOB; ++q) t[q] = 0.0;
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-            for (int q = 0; q < NGLOB; ++q) t[q] += __ldcg(&a.part[(size_t)b * NGLOB + q]);
-        block_sum<NGLOB>(t, red);
-        if (threadIdx.x == 0) {
-            for (int q = 0; q < NGLOB; ++q) a.glob[q] = t[q];
-            *a.ticket = 0u;
-        }
+        const double t = partials_sum<8>(nblk, 0.0, red, [](double u, double w) { return u + w; },
+                                         [&](int b, int k) { return __ldcg(&a.part[(size_t)b * 8 + k]); });
+        if (threadIdx.x < 8) a.glob[threadIdx.x] = t;
+        if (threadIdx.x == 0) *a.ticket = 0u;
     }
 }
 
 // ------------------------------------------------------------------ finish
 // Stage updates of the integration step (Limit-sticky9.c:853-891) without FMA contraction,
 // so the state arithmetic is rounded exactly as the reference's.
-__device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const double acc3[3]) {
+// a / 6, correctly rounded, in three operations: with c = RN(1/6), q = RN(a c) and the exact
+// remainder r = a - 6 q, RN(q + r c) is the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990);
+// outside the range where that holds, the division itself.
+__device__ __forceinline__ double sixth(double a) {
+    const int be = (__double2hiint(a) >> 20) & 0x7ff;
+    if (be < 128 || be > 2040) return __ddiv_rn(a, 6.0);
+    constexpr double c = 1.0 / 6.0;
+    const double q = __dmul_rn(a, c);
+    return __fma_rn(__fma_rn(-6.0, q, a), c, q);
+}
+
+__device__ __forceinline__ void stage_update_k(const FinishArgs &a, int p, int k, double acc) {
     const double dt = a.dt;
-    for (int k = 0; k < 3; ++k) {
+    {
         const size_t o = (size_t)k * a.ld + p;
         const double x = a.st.x[o], v = a.st.v[o];
         if (a.stage >= STAGE_RK4_1) {
@@ -304,24 +344,24 @@ __device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const d
             // k1 + 2 k2 + 2 k3 of the position and velocity slopes)
             if (a.stage == STAGE_RK4_1) {
                 a.st.xs[o] = x + 0.5 * dt * v;
-                a.st.vs[o] = v + 0.5 * dt * acc3[k];
+                a.st.vs[o] = v + 0.5 * dt * acc;
                 a.st.hx[o] = v;
-                a.st.hv[o] = acc3[k];
+                a.st.hv[o] = acc;
             } else if (a.stage == STAGE_RK4_4) {
                 const double vprev = a.st.vs[o];
                 a.st.x[o] = x + (dt / 6.0) * (a.st.hx[o] + vprev);
-                a.st.v[o] = v + (dt / 6.0) * (a.st.hv[o] + acc3[k]);
+                a.st.v[o] = v + (dt / 6.0) * (a.st.hv[o] + acc);
             } else {
                 const double vprev = a.st.vs[o];
                 const double f = a.stage == STAGE_RK4_2 ? 0.5 * dt : dt;
                 a.st.xs[o] = x + f * vprev;
-                a.st.vs[o] = v + f * acc3[k];
+                a.st.vs[o] = v + f * acc;
                 a.st.hx[o] += 2.0 * vprev;
-                a.st.hv[o] += 2.0 * acc3[k];
+                a.st.hv[o] += 2.0 * acc;
             }
         } else if (a.stage == 1) {  // :853-860
             const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, v), dt));
-            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc3[k]), dt));
+            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
             a.st.xs[o] = x1;
             a.st.vs[o] = v1;
             a.st.hx[o] = x1;
@@ -329,7 +369,7 @@ __device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const d
         } else if (a.stage == 2) {  // :864-871
             const double vprev = a.st.vs[o];
             const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, vprev), dt));
-            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc3[k]), dt));
+            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
             a.st.xs[o] = x1;
             a.st.vs[o] = v1;
             a.st.hx[o] = __dadd_rn(a.st.hx[o], x1);
@@ -337,42 +377,50 @@ __device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const d
         } else {  // :875-891
             const double vprev = a.st.vs[o];
             const double x3 = __dadd_rn(x, __dmul_rn(vprev, dt));
-            const double v3 = __dadd_rn(v, __dmul_rn(acc3[k], dt));
-            a.st.x[o] = __ddiv_rn(__dadd_rn(__dadd_rn(x, x3), __dmul_rn(2.0, a.st.hx[o])), 6.0);
-            a.st.v[o] = __ddiv_rn(__dadd_rn(__dadd_rn(v, v3), __dmul_rn(2.0, a.st.hv[o])), 6.0);
+            const double v3 = __dadd_rn(v, __dmul_rn(acc, dt));
+            a.st.x[o] = sixth(__dadd_rn(__dadd_rn(x, x3), __dmul_rn(2.0, a.st.hx[o])));
+            a.st.v[o] = sixth(__dadd_rn(__dadd_rn(v, v3), __dmul_rn(2.0, a.st.hv[o])));
         }
     }
 }
+__device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const double acc3[3]) {
+    for (int k = 0; k < 3; ++k) stage_update_k(a, p, k, acc3[k]);
+}
 
+// Bound by its FP64 instructions (about 150 per star, 64 cycles each per warp and scheduler): one
+// warp per scheduler and block, no division per star but the reference's own q, common factors
+// R^3 and m R^3 taken out of the sums.
 __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nblk) {
-    __shared__ double red[32 * 3];
-    const int i = blk * blockDim.x + threadIdx.x;
+    __shared__ double red[ON_NT];
+    const int i = blk * ON_NT + threadIdx.x;
     const double m0 = a.m[0];
-    const double eps = a.eps, eps2 = a.eps2, ic2 = a.inv_c2;
+    const double eps2 = a.eps2, ic2 = a.inv_c2;
     const double *G = a.glob;
-    double bh[3] = {0.0, 0.0, 0.0};
+    double bh[4] = {0.0, 0.0, 0.0, 0.0};
     bool bad = false;
 
     if (i < a.nstar) {
         const int p = i + 1;
         const double s[3] = {a.spos[i], a.spos[a.npad + i], a.spos[2 * a.npad + i]};
         const double q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
-        const double R = 1.0 / sqrt(q + eps2);
+        const double R = rsqrt(q + eps2);
         const double R3 = R * R * R;
         const double mi = a.m[p];
         // the force slots only (a fused-energy sweep has one more, read by the energy kernel)
         const int nk = a.nacc < NACC_MAX ? a.nacc : NACC_MAX;
         double S[NACC_MAX];
-        for (int k = 0; k < nk; ++k) {
-            double t = 0.0;
-            for (int g = 0; g < a.gsplit; ++g) t += a.acc[((size_t)g * a.nacc + k) * a.npad + i];
-            S[k] = t;
-        }
+#pragma unroll
+        for (int k = 0; k < NACC_MAX; ++k) S[k] = k < nk ? a.acc[(size_t)k * a.npad + i] : 0.0;
+        for (int g = 1; g < a.gsplit; ++g)
+#pragma unroll
+            for (int k = 0; k < NACC_MAX; ++k)
+                if (k < nk) S[k] += a.acc[((size_t)g * a.nacc + k) * a.npad + i];
         if (a.sums_out)
             for (int k = 0; k < nk; ++k) a.sums_out[(size_t)k * a.npad + i] = S[k];
         const double Gv[3] = {S[A_GX], S[A_GY], S[A_GZ]};
         double acc3[3];
-        for (int k = 0; k < 3; ++k) acc3[k] = Gv[k] - m0 * R3 * s[k];  // Newton incl. BH column
+        const double mb = m0 * R3;
+        for (int k = 0; k < 3; ++k) acc3[k] = fma(-mb, s[k], Gv[k]);  // Newton incl. BH column
         if (a.pn1) {
             const double v[3] = {ld_x(a.v, a.vsp, a.vsk, p, 0), ld_x(a.v, a.vsp, a.vsk, p, 1),
                                  ld_x(a.v, a.vsp, a.vsk, p, 2)};
@@ -387,36 +435,33 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
             const double Ps = P[0] * s[0] + P[1] * s[1] + P[2] * s[2];
             const double sB3 = s[0] * B3[0] + s[1] * B3[1] + s[2] * B3[2];
             const double sG = s[0] * Gv[0] + s[1] * Gv[1] + s[2] * Gv[2];
+            const double m0R = m0 * R;
             // star i: :215-238 (a_BH), :249-274 (ac direct), :276-382 summed over j (t1..t4, W),
-            // minus the self-pair removal :392-422
-            const double cs = -m0 * R3 * (4.0 * m0 * R - vi2)        // a_BH, s part
-                              + 5.0 * m0 * R3 * mi * R - 4.0 * mi * R3 * vi2   // ac direct
-                              - m0 * R3 * (4.0 * Phi + 1.25 * A1 - 0.25 * C + 0.5 * sB3)  // t1
-                              + 3.5 * m0 * U                             // t3 (s U part)
-                              + 4.0 * R3 * viP                           // t4
-                              + mi * R3 * m0 * (4.0 / eps + 1.25 * R + 0.25 * q * R3)    // -rem
-                              - 3.5 * mi * R3 * m0 * (1.0 / eps - R) - 4.0 * mi * R3 * vi2;
-            const double cv = -4.0 * m0 * R3 * vis + 7.0 * mi * R3 * vis - 3.0 * R3 * Ps
-                              + 7.0 * mi * R3 * vis;
-            const double cg = 4.0 * m0 * R;                              // t2
+            // minus the self-pair removal :392-422.  The s part, over R^3 but for the U term:
+            //   m0 [ -(4 m0 R - v^2) - (4 Phi + 1.25 A1 - 0.25 C + 0.5 s.B3)
+            //        + m_i (9.75 R + 0.5 / eps + 0.25 q R^3) ] - 8 m_i v^2 + 4 v.P
+            const double aa = 4.0 * Phi + 1.25 * A1 + fma(0.5, sB3, -0.25 * C);
+            const double bm = fma(9.75, R, fma(0.25 * q, R3, 0.5 * a.inv_eps));
+            const double br = fma(mi, bm, vi2 - fma(4.0, m0R, aa));
+            const double cs = fma(R3, fma(m0, br, fma(-8.0 * mi, vi2, 4.0 * viP)), (3.5 * m0) * U);
+            const double cv = R3 * fma(vis, fma(14.0, mi, -4.0 * m0), -3.0 * Ps);
+            const double cg = 4.0 * m0R, cb = -3.5 * m0R, cp = -4.0 * R3 * vis;
             for (int k = 0; k < 3; ++k) {
-                const double pn = cs * s[k] + cv * v[k] + cg * Gv[k] - 3.5 * m0 * R * B3[k]
-                                  - 4.0 * R3 * vis * P[k] + W[k];
-                acc3[k] += ic2 * pn;
+                const double pn = fma(cs, s[k], fma(cv, v[k], fma(cg, Gv[k], fma(cb, B3[k], fma(cp, P[k], W[k])))));
+                acc3[k] = fma(ic2, pn, acc3[k]);
             }
             // this star's share of the BH's 1PN acceleration: :58-95 (a1), :101-115 (single),
             // :118-174 summed over j, minus :179-207 (removal, with its 1.25*eps)
-            const double T = -2.0 * sG - (Phi - eps2 * S0);
+            const double im0 = 1.0 / m0;
+            const double T = fma(eps2, S0, -Phi) - 2.0 * sG;
             const double mR3 = mi * R3;
-            const double bs = mR3 * (5.0 * m0 * R - 2.0 * vi2 + 1.5 * vis * vis / q)  // a1
-                              + 4.0 * mR3 * R * mi                                  // single
-                              + mR3 * (4.0 * A1 + 1.25 * Phi + 0.25 * T)           // pair
-                              - (mR3 / m0) * 4.0 * viP
-                              + mR3 * mi * (4.0 * R + 1.25 * eps)                   // -removal
-                              - (mR3 * mi / m0) * 4.0 * vi2;
-            const double bv = 3.0 * mR3 * vis + (mR3 / m0) * 4.0 * Ps + (mR3 * mi / m0) * 7.0 * vis;
-            for (int k = 0; k < 3; ++k)
-                bh[k] = bs * s[k] + bv * v[k] - 3.5 * R * mi * Gv[k] + (mR3 / m0) * 3.0 * vis * P[k];
+            const double bs = fma(5.0, m0R, fma(-2.0, vi2, 1.5 * (vis * vis / q)))          // a1
+                              + fma(4.0, A1, fma(1.25, Phi, 0.25 * T))                      // pair
+                              + mi * fma(8.0, R, 1.25 * a.eps)                              // single, -removal
+                              - (4.0 * im0) * fma(mi, vi2, viP);
+            const double bv = fma(vis, fma(7.0 * mi, im0, 3.0), (4.0 * im0) * Ps);
+            const double bg = -3.5 * R * mi, bp = 3.0 * im0 * vis;
+            for (int k = 0; k < 3; ++k) bh[k] = fma(mR3, fma(bs, s[k], fma(bv, v[k], bp * P[k])), bg * Gv[k]);
         }
         for (int k = 0; k < 3; ++k) {
             if (!isfinite(acc3[k])) bad = true;
@@ -425,25 +470,20 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
         if (a.stage) stage_update(a, p, acc3);
     }
     if (bad) atomicOr(a.err, DEVERR_NONFINITE);
-    block_sum<3>(bh, red);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) a.part[(size_t)blk * 3 + k] = bh[k];
+    const double r = block_sum<4>(bh, red);
+    if (threadIdx.x < 4) a.part[(size_t)blk * 4 + threadIdx.x] = r;
     if (last_block(a.ticket, nblk)) {
-        double t[3] = {0.0, 0.0, 0.0};
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-            for (int k = 0; k < 3; ++k) t[k] += __ldcg(&a.part[(size_t)b * 3 + k]);
-        block_sum<3>(t, red);
-        if (threadIdx.x == 0) {
-            double acc3[3];
-            bool b0 = false;
-            for (int k = 0; k < 3; ++k) {
-                // BH: Newtonian pull of the stars (:36-51, row 0) plus the 1PN sum
-                acc3[k] = G[G_B3X + k] + (a.pn1 ? ic2 * t[k] : 0.0);
-                if (!isfinite(acc3[k])) b0 = true;
-                if (a.a) a.a[(long long)k * a.ask] = acc3[k];
-            }
-            if (b0) atomicOr(a.err, DEVERR_NONFINITE);
-            if (a.stage) stage_update(a, 0, acc3);
+        const double t = partials_sum<4>(nblk, 0.0, red, [](double u, double w) { return u + w; },
+                                         [&](int b, int k) { return __ldcg(&a.part[(size_t)b * 4 + k]); });
+        // BH: Newtonian pull of the stars (:36-51, row 0) plus the 1PN sum; thread k < 3 holds component k
+        const int k = threadIdx.x;
+        if (k < 3) {
+            const double acc = a.pn1 ? fma(ic2, t, G[G_B3X + k]) : G[G_B3X + k];
+            if (!isfinite(acc)) atomicOr(a.err, DEVERR_NONFINITE);
+            if (a.a) a.a[(long long)k * a.ask] = acc;
+            if (a.stage) stage_update_k(a, 0, k, acc);
+        }
+        if (k == 0) {
             if (a.fix_bad) *a.fix_bad = 0;
             *a.ticket = 0u;
         }
@@ -454,9 +494,9 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
 // Per star (Limit-sticky9.c:452-556): kinetic, Newtonian potential row, O(N) 1PN term and the
 // pairwise 1PN energy with its self-pair removal; compensated (double-double) sums.
 __device__ __forceinline__ void energy_body(const EnergyArgs &a, int blk, int nblk) {
-    __shared__ DD red[32 * 4];
-    const int i = blk * blockDim.x + threadIdx.x;
-    const double m0 = a.m[0], eps = a.eps, eps2 = a.eps2;
+    __shared__ DD red[ON_NT];
+    const int i = blk * ON_NT + threadIdx.x;
+    const double m0 = a.m[0], eps2 = a.eps2, ie = a.inv_eps;
     const double v0[3] = {ld_x(a.v, a.sp, a.sk, 0, 0), ld_x(a.v, a.sp, a.sk, 0, 1),
                           ld_x(a.v, a.sp, a.sk, 0, 2)};
     const double A1 = a.glob[G_A1];
@@ -473,38 +513,37 @@ __device__ __forceinline__ void energy_body(const EnergyArgs &a, int blk, int nb
             Psi += a.acc[((size_t)g * a.nacc + a.spsi) * a.npad + i];
         }
         const double q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
-        const double R = 1.0 / sqrt(q + eps2);
+        const double R = rsqrt(q + eps2);
         const double vi2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
         const double v0vi = v0[0] * v[0] + v0[1] * v[1] + v0[2] * v[2];
         const double sv0 = s[0] * v0[0] + s[1] * v0[1] + s[2] * v0[2];
         const double svi = s[0] * v[0] + s[1] * v[1] + s[2] * v[2];
         const double mR = m0 * R;
         e[0].hi = mi * vi2;
-        e[1].hi = (-(mR + Phi) + mi / sqrt(eps2)) * mi;
+        e[1].hi = (-(mR + Phi) + mi * ie) * mi;
         e[2].hi = 0.375 * mi * vi2 * vi2 + 1.5 * mR * mi * vi2 + 0.5 * mR * mR * mi
                   + 0.5 * mR * mi * (3.0 * vi2 - 7.0 * v0vi - sv0 * svi * R * R);
         e[3].hi = 0.25 * mi * (6.0 * vi2 * Phi - Psi) + m0 * mi * R * Phi + 0.5 * m0 * mi * R * A1
-                  - (0.25 * mi * mi / eps * (-vi2) + m0 * mi * mi * (R / eps + 0.5 * R * R));
+                  - mi * mi * (-0.25 * ie * vi2 + m0 * R * (ie + 0.5 * R));
     }
-    block_sum_dd<4>(e, red);
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 4; ++q) {
-            a.part[((size_t)blk * 4 + q) * 2] = e[q].hi;
-            a.part[((size_t)blk * 4 + q) * 2 + 1] = e[q].lo;
-        }
+    const DD r = block_sum<4>(e, red);
+    if (threadIdx.x < 4) {
+        a.part[((size_t)blk * 4 + threadIdx.x) * 2] = r.hi;
+        a.part[((size_t)blk * 4 + threadIdx.x) * 2 + 1] = r.lo;
+    }
     if (last_block(a.ticket, nblk)) {
-        DD t[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-            for (int q = 0; q < 4; ++q)
-                t[q] = dd_add(t[q], DD{__ldcg(&a.part[((size_t)b * 4 + q) * 2]),
-                                       __ldcg(&a.part[((size_t)b * 4 + q) * 2 + 1])});
-        block_sum_dd<4>(t, red);
+        DD t = partials_sum<4>(nblk, DD{0.0, 0.0}, red, dd_add, [&](int b, int q) {
+            return DD{__ldcg(&a.part[((size_t)b * 4 + q) * 2]), __ldcg(&a.part[((size_t)b * 4 + q) * 2 + 1])};
+        });
+        __shared__ double tot[4];
+        if (threadIdx.x < 4) tot[threadIdx.x] = t.hi + t.lo;
+        __syncthreads();
         if (threadIdx.x == 0) {
             const double kin0 = m0 * (v0[0] * v0[0] + v0[1] * v0[1] + v0[2] * v0[2]);
-            const double kin = 0.5 * ((t[0].hi + t[0].lo) + kin0);
-            const double pot = 0.5 * ((t[1].hi + t[1].lo) - m0 * A1);
-            const double potpn = a.inv_c2 * (t[2].hi + t[2].lo);
-            const double pn2 = a.inv_c2 * (t[3].hi + t[3].lo);
+            const double kin = 0.5 * (tot[0] + kin0);
+            const double pot = 0.5 * (tot[1] - m0 * A1);
+            const double potpn = a.inv_c2 * tot[2];
+            const double pn2 = a.inv_c2 * tot[3];
             a.out[0] = pot;
             a.out[1] = kin;
             a.out[2] = potpn;
@@ -517,25 +556,25 @@ __device__ __forceinline__ void energy_body(const EnergyArgs &a, int blk, int nb
 
 // ------------------------------------------------------------------ kernels
 // One system: the block index is the block within the system.
-__global__ void __launch_bounds__(256) k_prep(const PrepArgs a) { prep_body(a, blockIdx.x, gridDim.x); }
-__global__ void __launch_bounds__(256) k_finish(const FinishArgs a) { finish_body(a, blockIdx.x, gridDim.x); }
-__global__ void __launch_bounds__(256) k_energy_finish(const EnergyArgs a) {
+__global__ void __launch_bounds__(ON_NT) k_prep(const PrepArgs a) { prep_body(a, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(ON_NT) k_finish(const FinishArgs a) { finish_body(a, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(ON_NT) k_energy_finish(const EnergyArgs a) {
     energy_body(a, blockIdx.x, gridDim.x);
 }
 
 // An ensemble in one launch: blockmap[b] = (cluster, block within the cluster, blocks of the
 // cluster); each cluster's arguments come from a device table.
-__global__ void __launch_bounds__(256) k_prep_ens(const PrepArgs *tab, const int4 *blockmap) {
+__global__ void __launch_bounds__(ON_NT) k_prep_ens(const PrepArgs *tab, const int4 *blockmap) {
     const int4 bm = blockmap[blockIdx.x];
     const PrepArgs a = tab[bm.x];
     prep_body(a, bm.y, bm.z);
 }
-__global__ void __launch_bounds__(256) k_finish_ens(const FinishArgs *tab, const int4 *blockmap) {
+__global__ void __launch_bounds__(ON_NT) k_finish_ens(const FinishArgs *tab, const int4 *blockmap) {
     const int4 bm = blockmap[blockIdx.x];
     const FinishArgs a = tab[bm.x];
     finish_body(a, bm.y, bm.z);
 }
-__global__ void __launch_bounds__(256) k_energy_ens(const EnergyArgs *tab, const int4 *blockmap) {
+__global__ void __launch_bounds__(ON_NT) k_energy_ens(const EnergyArgs *tab, const int4 *blockmap) {
     const int4 bm = blockmap[blockIdx.x];
     const EnergyArgs a = tab[bm.x];
     energy_body(a, bm.y, bm.z);
@@ -543,33 +582,33 @@ __global__ void __launch_bounds__(256) k_energy_ens(const EnergyArgs *tab, const
 
 // ------------------------------------------------------------------ launchers
 cudaError_t launch_prep_ens(const PrepArgs *tab, const int4 *blockmap, int nblocks, cudaStream_t s) {
-    k_prep_ens<<<nblocks, 256, 0, s>>>(tab, blockmap);
+    k_prep_ens<<<nblocks, ON_NT, 0, s>>>(tab, blockmap);
     return cudaGetLastError();
 }
 cudaError_t launch_finish_ens(const FinishArgs *tab, const int4 *blockmap, int nblocks, cudaStream_t s) {
-    k_finish_ens<<<nblocks, 256, 0, s>>>(tab, blockmap);
+    k_finish_ens<<<nblocks, ON_NT, 0, s>>>(tab, blockmap);
     return cudaGetLastError();
 }
 cudaError_t launch_energy_ens(const EnergyArgs *tab, const int4 *blockmap, int nblocks, cudaStream_t s) {
-    k_energy_ens<<<nblocks, 256, 0, s>>>(tab, blockmap);
+    k_energy_ens<<<nblocks, ON_NT, 0, s>>>(tab, blockmap);
     return cudaGetLastError();
 }
 
 cudaError_t launch_prep(const PrepArgs &a, cudaStream_t s) {
-    const int nb = (a.nfill + 255) / 256;
-    k_prep<<<nb, 256, 0, s>>>(a);
+    const int nb = a.nfill / ON_NT;
+    k_prep<<<nb, ON_NT, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_finish(const FinishArgs &a, cudaStream_t s) {
-    const int nb = a.nstar > 0 ? (a.nstar + 255) / 256 : 1;
-    k_finish<<<nb, 256, 0, s>>>(a);
+    const int nb = a.nstar > 0 ? (a.nstar + ON_NT - 1) / ON_NT : 1;
+    k_finish<<<nb, ON_NT, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_energy_finish(const EnergyArgs &a, cudaStream_t s) {
-    const int nb = a.nstar > 0 ? (a.nstar + 255) / 256 : 1;
-    k_energy_finish<<<nb, 256, 0, s>>>(a);
+    const int nb = a.nstar > 0 ? (a.nstar + ON_NT - 1) / ON_NT : 1;
+    k_energy_finish<<<nb, ON_NT, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -13,6 +13,12 @@ enum RK4Stage : int { STAGE_RK4_1 = 11, STAGE_RK4_2 = 12, STAGE_RK4_3 = 13, STAG
 enum GlobSlot : int { G_A1 = 0, G_B3X, G_B3Y, G_B3Z, G_C, G_PX, G_PY, G_PZ, NGLOB };
 constexpr int NACC_MAX = 9;
 
+// Threads of the O(N) kernels' blocks: one warp per scheduler of an SM (they are bound by the latency
+// and the rate of FP64 instructions, which two warps of a scheduler share).  Partial sums: up to 8
+// doubles per block.
+constexpr int ON_NT = 128;
+inline size_t on_blocks(int npad) { return (size_t)npad / ON_NT + 2; }
+
 // Device state of one system, SoA [3][ld] doubles each (index 0 = BH).
 struct DevState {
     double *x, *v;    // step-start state (the reference's x, v; hx[0], hv[0])
@@ -47,7 +53,7 @@ struct FinishArgs {
     const double *spos, *acc, *glob;
     int nstar, npad, nacc, gsplit;
     int pn1;              // 1PN terms on (pair sweep in MODE_FORCE)
-    double eps, eps2, inv_c2, dt;
+    double eps, eps2, inv_c2, dt, inv_eps;
     double *a;            // output acceleration (may be null), [p*asp + k*ask]
     long long asp, ask;
     int stage;            // 0: none; 1..3: the reference's stages; STAGE_RK4_1..4: classic RK4
@@ -66,7 +72,7 @@ struct EnergyArgs {
     const double *spos, *acc, *glob;
     int nstar, npad, gsplit;
     int nacc, sphi, spsi;  // pair-sum layout: slots per split and the Phi, Psi slots
-    double eps, eps2, inv_c2;
+    double eps, eps2, inv_c2, inv_eps;
     double *part, *out;  // out[4] = pot_n, kin_n, pot_pn, total
     unsigned *ticket;
     int *fix_bad;        // optional: cleared for the next evaluation

@@ -39,7 +39,8 @@ namespace {
 constexpr int kMaxN = PN_NOALLOC_NMAX;           // particles, BH included
 constexpr int kNpad = ((kMaxN - 1 + 255) / 256) * 256;
 constexpr int kMaxSplits = 4;                     // j-range splits of the pair sweep
-constexpr int kBlocks = kNpad / 256 + 2;
+constexpr int kBlocks = kNpad / 256 + 2;  // half the O(N) kernels' blocks; the two halves are one buffer
+static_assert(2 * kBlocks * ON_NT >= kNpad, "partial sums");
 
 // byte offsets of the work buffers inside the array (each 256-byte aligned)
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -186,9 +187,9 @@ extern "C" int pn_force_noalloc(int n, const double *d_x, const double *d_v, con
     fa.spos = spos; fa.acc = acc; fa.glob = glob;
     fa.nstar = nstar; fa.npad = kNpad; fa.nacc = pair_nacc(mode); fa.gsplit = k.gsplit;
     fa.pn1 = mode == MODE_FORCE;
-    fa.eps = eps; fa.eps2 = eps2; fa.inv_c2 = inv_c2; fa.dt = 0.0;
+    fa.eps = eps; fa.inv_eps = 1.0 / eps; fa.eps2 = eps2; fa.inv_c2 = inv_c2; fa.dt = 0.0;
     fa.a = d_a; fa.asp = 3; fa.ask = 1; fa.stage = 0;
-    fa.part = part + (size_t)kBlocks * 8;
+    fa.part = part;  // (k_prep's partial sums are no longer needed)
     fa.ticket = &tickets[1]; fa.err = err;
     if (launch_finish(fa, s) != cudaSuccess) return fail(PN_ERR_CUDA);
     return fail(PN_OK);
