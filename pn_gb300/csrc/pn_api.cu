@@ -97,18 +97,21 @@ bool pn::fix_units(double eps, FixUnits *u) {
     return true;
 }
 
-// Shape of the fixed-point FP64 sweep: lanes per star and j-range splits.
+// Shape of the fixed-point FP64 sweep: lanes per star and j-range splits, from a model of its time in
+// units of one pair of a warp (0.35 us): waves of 3 CTAs per SM; per tile 128 / js pairs, the FP64 totals
+// (3 units) and a unit per halving of the lanes; 8 units around the tiles, and 1 per split for the
+// finishing kernel's sum over them.
 static void choose_fix(PairCfg *k, int nstar, int sms) {
     k->ipt = 1;
     k->tj = 128;
     k->x2 = 1;
     const int ntiles = (nstar + 127) / 128, slots = 3 * sms;
     double best = 1e300;
-    for (int js = 1; js <= 16; js *= 2)
+    for (int js = 1, h = 0; js <= 16; js *= 2, ++h)
         for (int g = 1; g <= 16 && g <= ntiles; ++g) {
-            const int ctas = (nstar * js + 127) / 128 * g;
+            const int ctas = (nstar + 128 / js - 1) / (128 / js) * g;
             const double waves = (ctas + slots - 1) / slots;
-            const double cost = waves * ((double)((ntiles + g - 1) / g) * (128.0 / js + 4.0) + 6.0) + 0.5 * g;
+            const double cost = waves * ((double)((ntiles + g - 1) / g) * (128.0 / js + 3.0 + h) + 8.0) + g;
             if (cost < best) {
                 best = cost;
                 k->js = js;

@@ -1,16 +1,13 @@
 // pn_fix.cuh -- the star-pair terms of the FP64 sweeps in 64-bit fixed point.
 //
-// A GB300 SM issues one FP64 warp instruction every 16 cycles (64 per scheduler; measured) but a
-// 32 x 32 + 64 bit integer multiply-add every second cycle per scheduler, so a product of two
-// 62-bit numbers on the integer pipe costs about a tenth of an FP64 multiply and carries 9 more bits.  The
-// pair terms are therefore formed as fixed-point numbers of 58 to 62 fraction bits; no
-// intermediate has fewer bits than a double.  Host and device compile the same functions (the
-// arithmetic is integer, so a CPU run gives the device's bits for the same seed).
+// A GB300 scheduler issues an FP64 warp instruction every 64 cycles, a 32 x 32 + 64 bit integer
+// multiply-add every 4 (both measured); a product of two 62-bit numbers is three of the latter and carries
+// 9 more bits than a double.  The pair terms are therefore formed as fixed-point numbers of 58 to 62
+// fraction bits.  Host and device compile the same functions (a CPU run checks the device's arithmetic).
 //
 // Units.  Lengths in units of 2^eL, the power of two with 1 <= eps / 2^eL < 2; masses in units of
 // the power of two of the BH's mass; velocities in units of 2^ev, the power of two above the fastest
-// |u| (below) of the two tiles at hand.
-// "S = k" at a variable says that it holds its value times 2^k.
+// |u| (below) of the two tiles at hand.  "S = k" at a variable says that it holds its value times 2^k.
 //
 // One pair (i, j), d = x_j - x_i:
 //   X   BH-relative positions, 96 bits, S = 62: d is exact to 2^-62 eps.
@@ -19,17 +16,20 @@
 //   RHO = |D|^2 + eps^2 2^(-2 ey), S = 60, in (1/4, 1]
 //   r   = 1 - RHO f^2, |r| < 2^-18.8;  Q 2^ey = f (1 + r/2 + 3 r^2/8): the binomial series of
 //         (1 - r)^(-1/2), whose next term is below 2^-58 (2^-60 on average).
-//   n   = d Q, S = 59, the softened unit vector
+//   n   = d Q, S = 60, the softened unit vector
 // and the terms of pn_device.cuh's sums, with w_j = sqrt(3) v_j, u_i = (4 / sqrt(3)) v_i:
-//   G   += (m Q^2) n         Phi += m Q      S0 += m Q^3      U += mu3 Q
-//   W   += [m Q^2 (u.w + (w.n)^2 / 2)] n + ct w,   ct = m Q^2 (u.n - w.n)
+//   G   += (m Q^2) n         S0 += (m Q^2) Q
+//   W   += (m Q^2 F) n + ct w,   F = u.w + (w.n)^2 / 2,  ct = m Q^2 (u.n - w.n)
 //   W64 += [(g1 - g3 qe_i) Q^2 + k] n,  g1 = m (c1 - 2 |v|^2), g3 = m c3, k = g3 + k35
-//          (FP64: its coefficients span the range of R_j^3; c3 rho Q^2 = c3 is in k)
+//          (its coefficient, which spans the range of R_j^3, in FP64; c3 rho Q^2 = c3 is in k)
+//   Phi += m Q,  U += mu3 Q  (FP64; in the energy sweep Phi in integers)
 //   Psi += m Q (7 u.w + (u.n)(w.n))  (four times the energy's)
-// The sums of one j-tile are accumulated as integers relative to the tile's own sum of
-// magnitudes (a first FP32 pass over the tile finds its exponent), so the smallest kept bit is
-// 2^-62 of that sum; the tile sums are added in FP64.  The pair of a star with itself (d = 0: no G,
-// no W) would raise that scale to m / eps^2; it is left out and its Phi, S0, U, Psi added in FP64.
+// The small (cross) parts of the dot products u.w, u.n, w.n are FP32: their rounding, 2^-54 of the
+// velocity unit, is random from pair to pair.  The sums over one j-tile are accumulated as integers
+// relative to the tile's own sums of magnitudes (a first FP32 pass over the tile finds their exponents),
+// so the smallest kept bit is 2^-62 of that sum; the tile sums are added in FP64.  The pair of a star
+// with itself (d = 0: no G, no W) would raise that scale to m / eps^2; it is left out of the integer
+// sums and its S0, and in the energy sweep Phi and Psi, added in FP64.
 #pragma once
 
 #include <cstdint>
@@ -54,6 +54,40 @@ constexpr double W_SCALE = 1.7320508075688772935;  // w / v
 constexpr u64 W_MANT = 0xDDB3D742C265539DULL;      // sqrt(3) 2^63
 constexpr u64 U_MANT = 0x93CD3A2C8198E269ULL;      // 4 / sqrt(3) 2^62
 
+// rounding constants of right shifts
+constexpr i64 half(int s) { return 1LL << (s - 1); }
+
+PNF float fmaf_(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    return ::fmaf(a, b, c);
+#else
+    return __builtin_fmaf(a, b, c);
+#endif
+}
+PNF float as_float(unsigned b) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float f;
+    std::memcpy(&f, &b, 4);
+    return f;
+#endif
+}
+PNF int to_int(float x) {  // rounded
+#ifdef __CUDA_ARCH__
+    return __float2int_rn(x);
+#else
+    return (int)__builtin_rintf(x);
+#endif
+}
+PNF double fma_(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return ::fma(a, b, c);
+#else
+    return __builtin_fma(a, b, c);
+#endif
+}
+
 // value = h 2^32 + l with both limbs signed 32-bit, so that limb products need no sign repair
 struct B2 {
     int h, l;
@@ -68,6 +102,25 @@ PNF i64 limbs(int h, int l) { return (i64)(((u64)(unsigned)h << 32) + (u64)(i64)
 PNF i64 mw(int a, int b, i64 c) { return (i64)a * b + c; }                           // IMAD.WIDE
 PNF u64 muw(unsigned a, unsigned b, u64 c) { return (u64)a * b + c; }                // IMAD.WIDE.U32
 PNF i64 cross(B2 a, B2 b, i64 c) { return mw(a.h, b.l, mw(a.l, b.h, c)); }
+// A factor: value = h 2^32 + l, the high part an integer (and as a float, for the cross products), the
+// low part a float; |h| < 2^31, so the value keeps 55 bits below its scale's top.  A product is
+// h h' 2^64 + (h l' + l h') 2^32: one integer multiply-add for the first part, which may be summed
+// over terms, and two FP32 FMAs for the second, which likewise.
+struct V {
+    int h;
+    float hf, l;
+};
+PNF V vec(B2 b) {
+    V r;
+    r.h = b.h;
+    r.hf = (float)b.h;
+    r.l = (float)b.l;
+    return r;
+}
+// hi + x f, x a sum of cross products and f its unit; |x f| < 2^(31 + B), rounded to 2^B
+template <int B> PNF i64 merge(i64 hi, float x, float f) { return mw(to_int(x * (f * (1.f / (1 << B)))), 1 << B, hi); }
+PNF float crossf(const V &a, const V &b, float c) { return fmaf_(a.hf, b.l, fmaf_(a.l, b.hf, c)); }
+
 PNF u64 mulhi(u64 a, u64 b) {
 #ifdef __CUDA_ARCH__
     return __umul64hi(a, b);
@@ -75,14 +128,14 @@ PNF u64 mulhi(u64 a, u64 b) {
     return (u64)(((unsigned __int128)a * b) >> 64);
 #endif
 }
-// a >> s for 0 <= s (0 from 64 on)
+// a >> s for 0 <= s (0 from 64 on, and for s < 0)
 PNF u64 shr(u64 a, int s) {
 #ifdef __CUDA_ARCH__
     u64 r;
     asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(s));
     return r;
 #else
-    return s > 63 ? 0 : a >> s;
+    return (unsigned)s > 63u ? 0 : a >> s;
 #endif
 }
 
@@ -172,108 +225,138 @@ enum : int { F_NEWTON = 0, F_FORCE = 1, F_ENERGY = 2, F_FORCE_ENERGY = 3 };  // 
 
 struct StarI {  // the accumulating star
     X96 x, y, z;
-    B2 ux, uy, uz;  // u_i, S = 62
-    double qe;      // |s_i|^2 + eps^2
+    V ux, uy, uz;  // u_i in units of its own power of two 2^(ev - d), S = 62
+    int d;         // (per tile)
+    float fd;      // 2^-d
+    double qe;     // |s_i|^2 + eps^2
 };
 struct StarJ {
     X96 x, y, z;
-    u64 m, m3;      // mantissas of m and mu3 = m R^3
-    int em, em3;    // their exponents (in the units above)
-    B2 wx, wy, wz;  // w_j, S = 60
-    double g1, g3, k;  // FP64 coefficients (g1, g3 times 2^(-62 - 2 eL))
+    unsigned mh;        // mantissa of m, S = 64: its high 32 bits as an integer,
+    float mhf, ml;      // and both halves as floats times 2^-34
+    int em;             // its exponent (in the units above)
+    B2 wx, wy, wz;      // w_j, S = 60
+    double m, mu3;      // m and mu3 = m R^3, in the system's units
+    double g1, g3, k;   // the coefficients of W64, in the system's units
 };
-struct Scale {  // the tile's exponents: sum of m Q^2, m Q, m Q^3, mu3 Q is below 2^e
-    int g, p, s, u;
+struct Scale {
+    int g, c;  // the tile's sums: m Q^2 < 2^g (or m Q, energy), |W64's coefficient| < 2^c (the system's units)
+    int q;     // exponent of the system's Q over the units' Q: -eL
+    // left shifts of the velocity terms' factors, from S = 60 relative to 2^g to S = 62 relative to the
+    // tile's own sums: |m Q^2 F| < 2^(g + 2 - lh + 2 ev), |ct| < 2^(g + 2 - lt + ev); 2^(lh - 32), 2^(lt - 32)
+    int lh, lt;
+};
+struct Acc {  // h 2^64 + x 2^32
+    i64 h;
+    float x;
+};
+struct Acci {  // ... all integers
+    i64 h, x;
 };
 struct Sums {
-    i64 gh[3], gx[3];  // G: h 2^64 + x 2^32, S = 121 relative to 2^g
-    i64 wh[3], wx[3];  // W: likewise, S = 121
-    i64 phi, s0, u;    // S = 62, 61, 62 relative to 2^p, 2^s, 2^u
-    i64 ct;            // S = 61 relative to 2^g
-    i64 ph, px;        // Psi: h 2^64 + x 2^32, S = 120 relative to 2^p
-    double w[3];       // W64 (times 2^59)
+    Acci g[3];  // G, S = 122 relative to 2^g
+    Acci c[3];  // W64, S = 122 relative to 2^c
+    Acci w[3];  // W's part along n, S = 122 relative to 2^(g + 2 - lh + 2 ev)
+    Acci t[3];  // W's part along w, S = 122 relative to 2^(g + 2 - lt + 2 ev)
+    i64 s0;     // S0, S = 60 relative to 2^g
+    i64 ct;     // sum of ct, S = 62 relative to 2^(g + 2 - lt + ev)
+    i64 phi;    // energy: Phi, S = 62 relative to 2^g
+    Acc psi;    // energy: Psi, S = 121 relative to 2^(g + 2 ev)
+    double dphi, du;  // force: Phi, U (FP64)
+    double dpsi;      // force and energy: Psi (FP64, times 2^59, relative to 2^(2 ev))
 };
 
 template <int MODE> PNF void clear(Sums &a) {
-    for (int k = 0; k < 3; ++k) a.gh[k] = a.gx[k] = a.wh[k] = a.wx[k] = 0;
-    a.phi = a.s0 = a.u = a.ct = a.ph = a.px = 0;
+    for (int k = 0; k < 3; ++k) {
+        a.g[k].h = a.g[k].x = a.c[k].h = a.c[k].x = a.w[k].h = a.w[k].x = a.t[k].h = a.t[k].x = 0;
+    }
+    a.s0 = a.ct = a.phi = a.psi.h = 0;
+    a.psi.x = 0.f;
+    a.dphi = a.du = a.dpsi = 0.0;
 }
-
-// Moves the cross sums' upper halves into the high sums; at least every 4 pairs (the cross sums
-// of 4 pairs stay below 2^63: see the bounds at pair()).
-template <int MODE> PNF void carry(Sums &a) {
-    if (MODE != F_ENERGY) {
+// Moves the cross sums into the high sums, at least every 8 pairs (see the bounds at pair()).
+PNF void fold(Acc &a) {  // (what is below 2^35 stays in the FP32 sum: 12582912 = 1.5 2^23 rounds to an integer)
+    const float t = fmaf_(a.x, 0x1p-36f, 12582912.f) - 12582912.f;
+    a.h = mw(to_int(t), 16, a.h);
+    a.x = fmaf_(t, -0x1p36f, a.x);
+}
+PNF void fold(Acci &a) {
+    a.h += a.x >> 32;
+    a.x &= 0xffffffffLL;
+}
+template <int MODE> PNF void fold(Sums &a) {
+    if (MODE == F_ENERGY) {
+        fold(a.psi);
+        return;
+    }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            a.gh[k] += a.gx[k] >> 32;
-            a.gx[k] &= 0xffffffffLL;
-            if (MODE != F_NEWTON) {
-                a.wh[k] += a.wx[k] >> 32;
-                a.wx[k] &= 0xffffffffLL;
-            }
+    for (int k = 0; k < 3; ++k) {
+        fold(a.g[k]);
+        if (MODE != F_NEWTON) {
+            fold(a.c[k]);
+            fold(a.w[k]);
+            fold(a.t[k]);
         }
     }
-    if (MODE == F_ENERGY || MODE == F_FORCE_ENERGY) {
-        a.ph += a.px >> 32;
-        a.px &= 0xffffffffLL;
-    }
 }
+
+// The sums after the last fold, S lowered by 60 (the integer ones) or 61
+PNF i64 top(const Acci &a) { return (i64)((u64)a.h << 4) + (a.x >> 28); }
+PNF i64 top(const Acc &a) { return (i64)((u64)a.h << 3) + to_int(a.x * 0x1p-29f); }
+// The shifts of Scale from the exponents of the tile's sums of m Q^2, m Q^2 |F| and |ct|
+// (at most by `most`: beyond that the terms are small beside |v_i|^2 times the tile's sum)
+PNF int lift(int g, int e, int most) { return 2 + (g - e < 0 ? 0 : g - e > most ? most : g - e); }
+constexpr int LIFT_H = 16, LIFT_T = 12;
 
 PNF double scale_down(double x, int e) {  // x 2^-e, x > 0 and normal, result normal
 #ifdef __CUDA_ARCH__
     return __hiloint2double(__double2hiint(x) - (e << 20), __double2loint(x));
 #else
-    u64 b = bits_of(x) - ((u64)e << 52);
+    u64 b = bits_of(x) - ((u64)(i64)e << 52);
     double r;
     std::memcpy(&r, &b, 8);
     return r;
 #endif
 }
-
-// rounding constants of right shifts
-constexpr i64 half(int s) { return 1LL << (s - 1); }
-
-// u.w (S = 58 as h + x / 2^32), and u.n, w.n with S = 61
-struct Dots {
-    i64 vh, vx, un, wn;
-};
-PNF Dots dots(const StarI &I, const StarJ &J, B2 nx, B2 ny, B2 nz) {
-    Dots d;
-    d.vx = cross(I.uz, J.wz, cross(I.uy, J.wy, cross(I.ux, J.wx, 0)));
-    d.vh = mw(I.uz.h, J.wz.h, mw(I.uy.h, J.wy.h, mw(I.ux.h, J.wx.h, 0)));
-    const i64 ux = cross(I.uz, nz, cross(I.uy, ny, cross(I.ux, nx, half(28))));
-    const i64 uh = mw(I.uz.h, nz.h, mw(I.uy.h, ny.h, mw(I.ux.h, nx.h, 0)));
-    const i64 wx = cross(J.wz, nz, cross(J.wy, ny, cross(J.wx, nx, half(26))));
-    const i64 wh = mw(J.wz.h, nz.h, mw(J.wy.h, ny.h, mw(J.wx.h, nx.h, 0)));
-    d.un = (uh << 4) + (ux >> 28);
-    d.wn = (wh << 6) + (wx >> 26);
-    return d;
+PNF double u2d(u64 v) {
+#ifdef __CUDA_ARCH__
+    return __ull2double_rn(v);
+#else
+    return (double)v;
+#endif
 }
-// Psi's term: m Q (7 u.w + (u.n)(w.n)); p = m Q (S = 62), the bracket S = 58 (below 6.1)
-PNF void psi_term(Sums &a, const Dots &d, B2 p) {
-    const B2 un = bal(d.un), wn = bal(d.wn);
-    const B2 z = bal(7 * d.vh + mw(un.h, wn.h, (7 * (d.vx >> 3) + (cross(un, wn, half(32)) >> 3)) >> 29));
-    a.ph = mw(p.h, z.h, a.ph);
-    a.px = cross(p, z, a.px);
+
+PNF void add(Acci &s, B2 a, B2 b) {
+    s.h = mw(a.h, b.h, s.h);
+    s.x = cross(a, b, s.x);
+}
+PNF void add(Acc &s, const V &a, const V &b) {
+    s.h = mw(a.h, b.h, s.h);
+    s.x = crossf(a, b, s.x);
+}
+PNF Acc dot(const V &ax, const V &ay, const V &az, const V &bx, const V &by, const V &bz) {
+    Acc s;
+    s.h = mw(ax.h, bx.h, 0);
+    s.x = fmaf_(ax.hf, bx.l, ax.l * bx.hf);
+    add(s, ay, by);
+    add(s, az, bz);
+    return s;
 }
 
 // One pair.  ybits: the bits of the FP32 seed y (0 < y <= 1 + 2^-20).  eps60: eps^2 in the units
 // above, S = 60 (1 <= eps^2 < 4).
-// Bounds: |D| <= 1 (+ 2^-20), |n| <= 1, |u| < 1 and |w| < 3/4 (the unit 2^ev), the tile's sum of P <= 2^62.
-//   cross sums of G, 4 pairs: sum Ph nl <= 2^30 2^31, Pl nh <= 4 2^31 2^27: 1.5 2^61
-//   cross sums of W, 4 pairs: |H| <= 1.03 2^62 in all, |ct| <= 1.75 2^61 in all, hence
-//     Hh nl <= 1.03 2^61, Hl nh <= 2^60, cth wl <= 0.88 2^61, ctl wh <= 0.75 2^61: 3.2 2^61 < 2^63
-//   cross sums of Psi, 4 pairs: Ph zl <= 2^61, Pl zh <= 4 2^31 6.1 2^26: 1.8 2^61
+// Bounds: |D| <= 1 (+ 2^-18), |n| <= 1, |u| < 1 and |w| < 3/4 (the unit 2^ev), the tile's sums of P, H, t
+// and C below 2^62, so the high sums stay below 2^62.  Integer cross sums of 8 pairs: ah bl with the sum of
+// |ah| <= 2^30, |bl| <= 2^31, and al bh <= 8 2^31 2^28 (t w: 8 2^31 0.75 2^28): below 2^62.6.
 template <int MODE>
 PNF void pair(Sums &a, const StarI &I, const StarJ &J, const Scale &E, unsigned ybits, u64 eps60) {
-    ybits += 8;  // a seed above Q (by 2^-21 .. 2^-20 less its error): Q 2^ey < 2, so Q^2 and Q^3 fit
+    ybits += 8;  // a seed above Q (by 2^-21 .. 2^-20 less its error): Q 2^ey < 2, so Q^2 fits
     const int ey = 127 - (int)(ybits >> 23);
     const unsigned F = (ybits & 0x7fffffu) | 0x800000u;
-    const B2 dx = bal(diff_shift(J.x, I.x, ey)), dy = bal(diff_shift(J.y, I.y, ey)),
-             dz = bal(diff_shift(J.z, I.z, ey));
-    // RHO, S = 60
-    const i64 dt = mw(dz.h, dz.l, mw(dy.h, dy.l, mw(dx.h, dx.l, half(31))));
-    const u64 rho = (u64)(mw(dz.h, dz.h, mw(dy.h, dy.h, mw(dx.h, dx.h, dt >> 31)))) + shr(eps60, 2 * ey);
+    const B2 bx = bal(diff_shift(J.x, I.x, ey)), by = bal(diff_shift(J.y, I.y, ey)), bz = bal(diff_shift(J.z, I.z, ey));
+    // RHO, S = 60 (its cross products in integers: its rounding error would enter every term)
+    const i64 dt = mw(bz.h, bz.l, mw(by.h, by.l, mw(bx.h, bx.l, half(31))));
+    const u64 rho = (u64)(mw(bz.h, bz.h, mw(by.h, by.h, mw(bx.h, bx.h, dt >> 31)))) + shr(eps60, 2 * ey);
     // r = 1 - RHO f^2, S = 58
     const unsigned F8 = F << 8;
     const u64 U = muw((unsigned)(rho >> 32), F8, muw((unsigned)rho, F8, half(32)) >> 32);  // RHO f, S = 59
@@ -283,67 +366,69 @@ PNF void pair(Sums &a, const StarI &I, const StarJ &J, const Scale &E, unsigned 
     const i64 c = mw(6, rsq, r << 5);                       // r/2 + 3 r^2/8, S = 64
     const int F7 = (int)(F << 7);
     const u64 Q = (u64)mw(F7, (int)(c >> 32), (i64)(((u64)F7 << 32) | (muw((unsigned)F7, (unsigned)c, 0) >> 32)));  // S = 62
-    const B2 q = bal((i64)(Q >> 1));  // S = 61
-    const i64 n0 = mw(dx.h, q.h, cross(dx, q, half(32)) >> 32), n1 = mw(dy.h, q.h, cross(dy, q, half(32)) >> 32),
-              n2 = mw(dz.h, q.h, cross(dz, q, half(32)) >> 32);
-    const B2 nx = bal(n0), ny = bal(n1), nz = bal(n2);  // S = 59
+    const B2 bq = bal((i64)Q);
+    // n = d Q, S = 60
+    const B2 mx = bal(mw(bx.h, bq.h, cross(bx, bq, half(32)) >> 32)), my = bal(mw(by.h, bq.h, cross(by, bq, half(32)) >> 32)),
+             mz = bal(mw(bz.h, bq.h, cross(bz, bq, half(32)) >> 32));
     if (MODE == F_ENERGY) {
-        const i64 pq = (i64)shr(mulhi(J.m, Q), E.p - J.em + ey);  // m Q, S = 62
-        a.phi += pq;
-        psi_term(a, dots(I, J, nx, ny, nz), bal(pq));
+        const V q = vec(bq);
+        const u64 mQ = muw(J.mh, (unsigned)q.h, 0) + ((u64)(i64)to_int(fmaf_(J.mhf, q.l, J.ml * q.hf)) << 2);  // S = 62
+        const u64 P = shr(mQ, E.g - J.em + ey);  // m Q relative to 2^g
+        a.phi += (i64)P;
+        const V p = vec(bal((i64)P));
+        const V nx = vec(mx), ny = vec(my), nz = vec(mz), wx = vec(J.wx), wy = vec(J.wy), wz = vec(J.wz);
+        const Acc uw = dot(I.ux, I.uy, I.uz, wx, wy, wz), un = dot(I.ux, I.uy, I.uz, nx, ny, nz), wn = dot(wx, wy, wz, nx, ny, nz);
+        const V b = vec(bal(merge<4>((un.h << 4) >> I.d, un.x, I.fd * 0x1p-28f))), w = vec(bal(merge<5>(wn.h << 6, wn.x, 0x1p-26f)));
+        // 7 u.w + (u.n)(w.n), S = 59 (below 6.1)
+        const V z = vec(bal(merge<5>(((14 * uw.h) >> I.d) + (mw(b.h, w.h, 0) >> 1), fmaf_(14.f * I.fd, uw.x, 0.5f * crossf(b, w, 0.f)), 0x1p-32f)));
+        add(a.psi, p, z);
         return;
     }
-    const u64 Q2 = mulhi(Q, Q) << 2;  // S = 62
-    const B2 p = bal((i64)shr(mulhi(J.m, Q2), E.g - J.em + 2 * ey));  // m Q^2, S = 62 relative to 2^g
-    a.gh[0] = mw(p.h, nx.h, a.gh[0]);
-    a.gh[1] = mw(p.h, ny.h, a.gh[1]);
-    a.gh[2] = mw(p.h, nz.h, a.gh[2]);
-    a.gx[0] = cross(p, nx, a.gx[0]);
-    a.gx[1] = cross(p, ny, a.gx[1]);
-    a.gx[2] = cross(p, nz, a.gx[2]);
+    const unsigned qh = (unsigned)(Q >> 32);
+    const u64 Q2 = muw(qh, qh, muw(qh, (unsigned)Q, 0) >> 31) << 2;  // S = 62
+    const float q2h = (float)(unsigned)(Q2 >> 32), q2l = (float)(unsigned)Q2;
+    const u64 mQ2 = muw(J.mh, (unsigned)(Q2 >> 32), 0) + ((u64)(i64)to_int(fmaf_(J.mhf, q2l, J.ml * q2h)) << 2);  // S = 62
+    const B2 p = bal((i64)shr(mQ2, E.g - J.em + 2 * ey));  // m Q^2, S = 62 relative to 2^g
+    add(a.g[0], p, mx);
+    add(a.g[1], p, my);
+    add(a.g[2], p, mz);
     if (MODE == F_NEWTON) return;
-    const u64 Q3 = mulhi(Q2, Q) << 1;  // S = 61
-    const i64 pq = (i64)shr(mulhi(J.m, Q), E.p - J.em + ey);
-    a.phi += pq;
-    a.s0 += (i64)shr(mulhi(J.m, Q3), E.s - J.em + 3 * ey);
-    a.u += (i64)shr(mulhi(J.m3, Q), E.u - J.em3 + ey);
-    // velocity terms
-    const Dots v = dots(I, J, nx, ny, nz);
-    const B2 wb = bal(v.wn), kb = bal(v.un - v.wn);
-    // F = u.w + (w.n)^2 / 2, S = 60
-    const B2 f = bal((v.vh << 2) + (mw(wb.h, wb.h, 0) << 1) + ((v.vx + mw(wb.h, wb.l, half(30))) >> 30));
-    const B2 H = bal((mw(p.h, f.h, 0) << 4) + (cross(p, f, half(28)) >> 28));   // S = 62
-    const i64 ct = (mw(p.h, kb.h, 0) << 2) + (cross(p, kb, half(30)) >> 30);    // S = 61
+    a.s0 += mw(p.h, bq.h, cross(p, bq, 0) >> 32) >> ey;  // m Q^3 = (m Q^2) Q
+    // velocity terms: the dot products' small parts in FP32, the sums in integers
+    const V nx = vec(mx), ny = vec(my), nz = vec(mz), wx = vec(J.wx), wy = vec(J.wy), wz = vec(J.wz);
+    const Acc uw = dot(I.ux, I.uy, I.uz, wx, wy, wz), un = dot(I.ux, I.uy, I.uz, nx, ny, nz), wn = dot(wx, wy, wz, nx, ny, nz);
+    const i64 b = merge<4>((un.h << 4) >> I.d, un.x, I.fd * 0x1p-28f), w = merge<5>(wn.h << 6, wn.x, 0x1p-26f);  // S = 62
+    const V wv = vec(bal(w));
+    // F = u.w + (w.n)^2 / 2, S = 62
+    const B2 f = bal(merge<4>(mw(wv.h, 2 * wv.h, (uw.h << 4) >> I.d), fmaf_(4.f * wv.hf, wv.l, (16.f * I.fd) * uw.x), 0x1p-32f));
+    const B2 H = bal((i64)((u64)mw(p.h, f.h, 0) << E.lh) + (cross(p, f, 0) >> (32 - E.lh)));
+    const B2 k = bal(b - w);
+    const i64 ct = (i64)((u64)mw(p.h, k.h, 0) << E.lt) + (cross(p, k, 0) >> (32 - E.lt));
     a.ct += ct;
-    const B2 cb = bal(ct);
-    a.wh[0] = mw(H.h, nx.h, mw(cb.h, J.wx.h, a.wh[0]));
-    a.wh[1] = mw(H.h, ny.h, mw(cb.h, J.wy.h, a.wh[1]));
-    a.wh[2] = mw(H.h, nz.h, mw(cb.h, J.wz.h, a.wh[2]));
-    // (with the products of the low limbs: slow stars leave H and ct few high bits)
-    a.wx[0] = cross(H, nx, cross(cb, J.wx, a.wx[0] + (mw(H.l, nx.l, mw(cb.l, J.wx.l, 0)) >> 32)));
-    a.wx[1] = cross(H, ny, cross(cb, J.wy, a.wx[1] + (mw(H.l, ny.l, mw(cb.l, J.wy.l, 0)) >> 32)));
-    a.wx[2] = cross(H, nz, cross(cb, J.wz, a.wx[2] + (mw(H.l, nz.l, mw(cb.l, J.wz.l, 0)) >> 32)));
-    if (MODE == F_FORCE_ENERGY) psi_term(a, v, bal(pq));
-    // FP64 part (g1, g3 carry 2^-62 for Q2's S)
-#ifdef __CUDA_ARCH__
-    const double q2 = scale_down(__ull2double_rn(Q2), 2 * ey);
-    const double co = ::fma(::fma(-I.qe, J.g3, J.g1), q2, J.k);
-    a.w[0] = ::fma(co, __ll2double_rn(n0), a.w[0]);
-    a.w[1] = ::fma(co, __ll2double_rn(n1), a.w[1]);
-    a.w[2] = ::fma(co, __ll2double_rn(n2), a.w[2]);
-#else
-    const double q2 = scale_down((double)Q2, 2 * ey);
-    const double co = __builtin_fma(__builtin_fma(-I.qe, J.g3, J.g1), q2, J.k);
-    a.w[0] = __builtin_fma(co, (double)n0, a.w[0]);
-    a.w[1] = __builtin_fma(co, (double)n1, a.w[1]);
-    a.w[2] = __builtin_fma(co, (double)n2, a.w[2]);
-#endif
+    const B2 t = bal(ct);
+    add(a.w[0], H, mx);
+    add(a.w[1], H, my);
+    add(a.w[2], H, mz);
+    add(a.t[0], t, J.wx);
+    add(a.t[1], t, J.wy);
+    add(a.t[2], t, J.wz);
+    // FP64: Phi, U and the coefficient of W64, which then joins the integers
+    const double qd = scale_down(u2d(Q), 62 + ey - E.q);
+    a.dphi = fma_(J.m, qd, a.dphi);
+    a.du = fma_(J.mu3, qd, a.du);
+    const u64 co = bits_of(fma_(fma_(-I.qe, J.g3, J.g1), qd * qd, J.k));
+    const u64 cm = ((co & 0xfffffffffffffULL) | 0x10000000000000ULL) << 9;  // S = 61 of 1.f
+    const i64 sg = (i64)co >> 63;
+    const B2 C = bal((i64)(((u64)shr(cm, E.c + 1022 - (int)((co >> 52) & 0x7ff)) ^ (u64)sg) - (u64)sg));  // S = 62
+    add(a.c[0], C, mx);
+    add(a.c[1], C, my);
+    add(a.c[2], C, mz);
+    if (MODE == F_FORCE_ENERGY) {
+        const V bv = vec(bal(b));
+        const i64 z = merge<5>(((14 * uw.h) >> I.d) + (mw(bv.h, wv.h, 0) >> 1), fmaf_(14.f * I.fd, uw.x, 0.5f * crossf(bv, wv, 0.f)), 0x1p-32f);  // S = 59
+        a.dpsi = fma_(J.m * qd, (double)z, a.dpsi);
+    }
 }
-
-// h 2^64 + x 2^32 (x carried: 0 <= x < 2^32) divided by 2^(64 - B)
-template <int B> PNF i64 top(i64 h, i64 x) { return (i64)((u64)h << B) + (x >> (32 - B)); }
-// bits kept, and the S of the result
-constexpr int TOP_G = 5, S_G = 62, TOP_W = 4, S_W = 61, TOP_P = 4, S_P = 60;
 
 }  // namespace fix
 }  // namespace pn

@@ -24,7 +24,7 @@ cudaError_t launch_pair_f64(int mode, const PairCfg &c, const PairArgs &a, cudaS
 // The FP64 sweep on the integer pipes (PairCfg::x2 = 1 in FP64; pn_pair_fix.cu): ipt 1, js 1..16,
 // tiles of 128.
 cudaError_t launch_pair_fix(int mode, const PairCfg &c, const PairArgs &a, cudaStream_t s);
-constexpr int FIX_GROUPS = 11;  // 16-byte groups per star of its pack
+constexpr int FIX_GROUPS = 13;  // 16-byte groups per star of its pack
 // Its units for a softening; false where its range does not cover it.
 bool fix_units(double eps, FixUnits *u);
 bool pair_shape_supported(int ipt, int js);

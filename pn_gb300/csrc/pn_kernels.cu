@@ -152,7 +152,8 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     const FixUnits &u = a.fu;
     const int e0 = expo(m0);
     auto ebits = [](double d) { return (__double2hiint(d) >> 20) & 0x7ff; };  // 0x7ff: not finite
-    bool in = ebits(m0) > 60 && ebits(m0) < 1986 && ebits(v2) < 1023 + 2 * EV_MAX - 10;
+    bool in = ebits(m0) > 60 && ebits(m0) < 1986 && ebits(v2) < 1023 + 2 * EV_MAX - 10 &&
+              ebits(v2) < 1023 + 60 + e0 - u.eL;  // (|v|^2 beside the FP32 range of g1f)
     for (int k = 0; k < 3; ++k) in = in && ebits(s[k]) < 1023 + POS_BITS + u.eL;
     // m: 0, or 2^-32 .. 2^59 of m0
     in = in && (__double2hiint(m) >= 0) && (m == 0.0 || (ebits(m) >= 1023 + e0 - 32 && ebits(m) < 1023 + e0 + 59));
@@ -162,36 +163,43 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     X96 x[3];
     B2 w[3], q[3];
     const float down = __int_as_float((127 - u.eL) << 23);
+    const int eu = speed_exp(v2);  // the star's own velocity unit
     for (int k = 0; k < 3; ++k) {
         to_f32_pair(real ? s[k] - o[k] : 0.0, hi[k], lo[k]);
         hi[k] *= down;
         lo[k] *= down;
         x[k] = to_x96(real ? s[k] : o[k], u.eL);
         w[k] = bal(to_scaled(v[k], W_MANT, 63, 60, ev));
-        q[k] = bal(to_scaled(v[k], U_MANT, 62, 62, ev));
+        q[k] = bal(to_scaled(v[k], U_MANT, 62, 62, eu));
     }
-    int em, em3;
-    const u64 mm = mantissa(m, em), mm3 = mantissa(mu3, em3);
+    int em;
+    const u64 mm = mantissa(m, em);
     em = mm ? em - e0 : -8192;
-    em3 = mm3 ? em3 - e0 + 3 * u.eL : -8192;
-    const double g1 = scale2(m * fma(-2.0, v2, c1), -62 - 2 * u.eL), g3 = scale2(m * c3, -62 - 2 * u.eL), kk = fma(m, c3, k35);
-    const float mf = to_f32(scale2(m, -e0)), mu3f = to_f32(scale2(mu3, 3 * u.eL - e0));
+    const double g1 = m * fma(-2.0, v2, c1), g3 = m * c3, kk = fma(m, c3, k35);
+    // FP32 magnitudes in the sweep's units, for the exponents of a tile's sums
+    const float mf = to_f32(scale2(m, -e0)), g1f = fabsf(to_f32(scale2(g1, u.eL - 2 * e0))),
+                g3f = to_f32(scale2(g3, 3 * u.eL - 2 * e0)), kf = to_f32(scale2(kk, 3 * u.eL - 2 * e0));
     uint4 *p = a.fpack + j;
     const size_t n = a.npad;
     auto fu = [](float f) { return __float_as_uint(f); };
     auto lw = [](double d) { return (unsigned)__double2loint(d); };
     auto hw = [](double d) { return (unsigned)__double2hiint(d); };
+    const float down34 = 5.8207660913467407e-11f;  // 2^-34
     p[0] = make_uint4(fu(hi[0]), fu(hi[1]), fu(hi[2]), fu(mf));
     p[n] = make_uint4(fu(lo[0]), fu(lo[1]), fu(lo[2]), (unsigned)em);
     p[2 * n] = make_uint4(x[0].w0, x[0].w1, x[0].w2, x[1].w0);
     p[3 * n] = make_uint4(x[1].w1, x[1].w2, x[2].w0, x[2].w1);
-    p[4 * n] = make_uint4(x[2].w2, (unsigned)mm, (unsigned)(mm >> 32), fu(mu3f));
-    p[5 * n] = make_uint4((unsigned)w[0].l, (unsigned)w[0].h, (unsigned)w[1].l, (unsigned)w[1].h);
-    p[6 * n] = make_uint4((unsigned)w[2].l, (unsigned)w[2].h, (unsigned)mm3, (unsigned)(mm3 >> 32));
-    p[7 * n] = make_uint4((unsigned)em3, 0u, lw(g1), hw(g1));
-    p[8 * n] = make_uint4(lw(g3), hw(g3), lw(kk), hw(kk));
-    p[9 * n] = make_uint4((unsigned)q[0].l, (unsigned)q[0].h, (unsigned)q[1].l, (unsigned)q[1].h);
-    p[10 * n] = make_uint4((unsigned)q[2].l, (unsigned)q[2].h, lw(qe), hw(qe));
+    p[4 * n] = make_uint4(x[2].w2, (unsigned)(mm >> 32), fu((float)(unsigned)(mm >> 32) * down34), fu((float)(unsigned)mm * down34));
+    auto un = [](int i) { return (unsigned)i; };
+    p[5 * n] = make_uint4(un(w[0].h), un(w[0].l), un(w[1].h), un(w[1].l));
+    p[6 * n] = make_uint4(un(w[2].h), un(w[2].l), 0u, 0u);
+    p[7 * n] = make_uint4(0u, fu(g1f), fu(g3f), fu(kf));
+    p[8 * n] = make_uint4(lw(m), hw(m), lw(mu3), hw(mu3));
+    p[9 * n] = make_uint4(lw(g1), hw(g1), lw(g3), hw(g3));
+    // (|w| in the tile's unit, rounded up)
+    p[10 * n] = make_uint4(lw(kk), hw(kk), fu(sqrtf(to_f32(scale2(3.0 * v2, -2 * ev))) * 1.00001f), (unsigned)eu);
+    p[11 * n] = make_uint4(un(q[0].h), un(q[0].l), un(q[1].h), un(q[1].l));
+    p[12 * n] = make_uint4(un(q[2].h), un(q[2].l), lw(qe), hw(qe));
 }
 
 // Per star j (particle p = j + 1): s = x_p - x_0, q = |s|^2, R = (q + eps^2)^(-1/2) (the

@@ -53,7 +53,7 @@ struct PairArgs {
     int ntiles;           // ceil(nstar / tj)
     int gsplit;           // j-range splits (gridDim.y)
     double eps2;
-    // the fixed-point FP64 sweep (pn_pairfix.cuh): its pack [11][npad], the flag that k_prep raises
+    // the fixed-point FP64 sweep (pn_pairfix.cuh): its pack [13][npad], the flag that k_prep raises
     // for a system outside its range, the state's masses and velocities, and its units
     const uint4 *fpack;
     const int *fix_bad;

@@ -8,10 +8,14 @@
 // for the sums themselves, which are added to FP64 totals in shared memory at the tile's end.
 //
 // Why: FP64 issues one warp instruction per 64 cycles and scheduler here and k_pair<double>'s 51 per
-// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 970, of which the
-// integer multiply pipe is busy 79 % and the FP64 pipe (5 FMA, 4 conversions) 62 %.  One force
-// evaluation at N = 65,536: 385 -> 104 ms, at N = 16,384: 24.0 -> 6.55 ms; its error against long
-// sums is a third of the FP64 sweep's (5.6e-16 against 1.6e-15 there, c = 1).
+// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 830, of which the
+// multiply-add pipe is busy 74 % and the FP64 pipe 59 % (6 operations per pair). One force evaluation at
+// N = 65,536: 385 -> 88.5 ms, N = 10,000: 9.3 -> 2.3 ms.  Its error against long double sums is below
+// the FP64 sweep's (medians at N = 2,049: 1.46e-16 against 2.22e-16 at c = 1000, 5.1e-16 against
+// 7.4e-16 at c = 1).  Measured on the way there, at N = 65,536: every product in integers and W64's sum
+// in FP64 (4 conversions and 5 FMA per pair) 104 ms; the dot products' small parts in FP32, Phi and U in
+// FP64 and W64's sum in integers 88.5 ms; the sums' small parts in FP32 too 76 ms, but with twice the FP64
+// sweep's error at c = 1.
 //
 // The integer range covers the systems that k_prep has checked star by star (positions within
 // 2^24 eps, masses zero or 2^-32 .. 2^59 of the BH's, all finite); for any other
@@ -26,9 +30,9 @@ namespace pn {
 constexpr int FIX_TJ = 128;
 
 template <int MODE> struct FixInfo {
-    static constexpr int NG = MODE == MODE_NEWTON ? 5 : MODE == MODE_ENERGY ? 7 : 9;  // streamed 16-byte groups
-    // tile totals: G, Phi, S0, U, W, ct, Psi as the mode has them
-    static constexpr int NT = MODE == MODE_NEWTON ? 3 : MODE == MODE_ENERGY ? 2 : MODE == MODE_FORCE ? 10 : 11;
+    static constexpr int NG = MODE == MODE_NEWTON ? 5 : MODE == MODE_ENERGY ? 8 : 11;  // streamed 16-byte groups
+    // sums over the tiles in shared memory: G; or G, S0, W along n, W64, ct, W along w, Phi, U (and Psi); or Phi, Psi
+    static constexpr int NT = MODE == MODE_NEWTON ? 3 : MODE == MODE_ENERGY ? 2 : MODE == MODE_FORCE ? 16 : 17;
 };
 
 template <int MODE>
@@ -42,6 +46,10 @@ inline size_t fix_smem_bytes() {
     return fast > gen ? fast : gen;
 }
 
+// a velocity component (h, l) of the pack, 2^-s times it
+__device__ __forceinline__ fix::B2 slower(unsigned h, unsigned l, int s) {
+    return fix::bal(fix::limbs((int)h, (int)l) >> s);
+}
 // exponent e with x < 2^e, x >= 0 (x within FP32 range)
 __device__ __forceinline__ int mag_exp(float x) {
     return (int)(__float_as_uint(x * 1.001f) >> 23) - 126;
@@ -73,12 +81,24 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         I.x = {g2.x, g2.y, g2.z};
         I.y = {g2.w, g3.x, g3.y};
         I.z = {g3.z, g3.w, pk[(size_t)4 * a.npad + il].x};
-        const uint4 u1 = pk[(size_t)10 * a.npad + il];
+        const uint4 u1 = pk[(size_t)12 * a.npad + il];
         I.qe = __hiloint2double((int)u1.w, (int)u1.z);
     }
-    // u_i is stored in its own tile's velocity unit 2^ei, w_j in tile t's; a pair of tiles uses the larger
+    // u_i is stored in its own velocity unit 2^eu, w_j in that of its tile; a pair of tiles uses the larger
+    // of theirs
     const int ei = __float_as_int(a.torg[ibase / TJ].pad0);
-    int ev = -100000;
+    int ev = -100000, eu = 0;
+    if constexpr (MODE != MODE_NEWTON) {
+        const uint4 k = pk[(size_t)10 * a.npad + il], u0 = pk[(size_t)11 * a.npad + il], u1 = pk[(size_t)12 * a.npad + il];
+        I.ux = vec(slower(u0.x, u0.y, 0));
+        I.uy = vec(slower(u0.z, u0.w, 0));
+        I.uz = vec(slower(u1.x, u1.y, 0));
+        eu = (int)k.w;
+    }
+    const int e0 = fix::expo(a.m[0]), eL = a.fu.eL;
+    const int eg = e0 - (MODE == MODE_ENERGY ? 1 : 2) * eL;  // exponents of the units of m Q^2 (m Q)
+    const int ec = 2 * e0 - 3 * eL;                          // ... and of W64's coefficient
+    const float qef = FORCE ? (float)(I.qe * pow2(-2 * eL)) : 0.f;
     // the i position in units of 2^eL as an FP32 pair (for the seeds' differences)
     float sh[3], sl[3];
 #pragma unroll
@@ -88,7 +108,6 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         sl[k] = (float)(s - (double)sh[k]);
     }
     Sums A;
-    A.w[0] = A.w[1] = A.w[2] = 0.0;
     if (sub == 0)
 #pragma unroll
         for (int q = 0; q < FixInfo<MODE>::NT; ++q) tot[q * NT + grp] = 0.0;
@@ -123,19 +142,16 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
             const int et = __float_as_int(a.torg[t].pad0), e = max(ei, et);
             if (e != ev) {
                 ev = e;
-                const uint4 u0 = pk[(size_t)9 * a.npad + il], u1 = pk[(size_t)10 * a.npad + il];
-                I.ux = bal(limbs((int)u0.y, (int)u0.x) >> min(e - ei, 63));
-                I.uy = bal(limbs((int)u0.w, (int)u0.z) >> min(e - ei, 63));
-                I.uz = bal(limbs((int)u1.y, (int)u1.x) >> min(e - ei, 63));
+                I.d = min(e - eu, 63);
+                I.fd = __int_as_float((127 - I.d) << 23);
             }
             if (e > et) {  // (the whole CTA) bring the tile's velocities to the larger unit, in place
                 uint4 *q = buf + (size_t)(stage * NG + 5) * TJ + tid;
                 const uint4 g5 = q[0], g6 = q[TJ];
-                const int s = min(e - et, 63);
-                const B2 wx = bal(limbs((int)g5.y, (int)g5.x) >> s), wy = bal(limbs((int)g5.w, (int)g5.z) >> s),
-                         wz = bal(limbs((int)g6.y, (int)g6.x) >> s);
-                q[0] = make_uint4((unsigned)wx.l, (unsigned)wx.h, (unsigned)wy.l, (unsigned)wy.h);
-                q[TJ] = make_uint4((unsigned)wz.l, (unsigned)wz.h, g6.z, g6.w);
+                const int sft = min(e - et, 63);
+                const B2 wx = slower(g5.x, g5.y, sft), wy = slower(g5.z, g5.w, sft), wz = slower(g6.x, g6.y, sft);
+                q[0] = make_uint4((unsigned)wx.h, (unsigned)wx.l, (unsigned)wy.h, (unsigned)wy.l);
+                q[TJ] = make_uint4((unsigned)wz.h, (unsigned)wz.l, g6.z, g6.w);
                 __syncthreads();
             }
         }
@@ -159,110 +175,132 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         // ---- the tile's sums in FP32: their exponents
         Scale E;
         {
-            float mg = 0.f, mp = 0.f, ms = 0.f, mu = 0.f;
+            float mg = 0.f, mc = 0.f, mh = 0.f, mt = 0.f;
+            const float down = FORCE ? exp2f((float)(__float_as_int(a.torg[t].pad0) - ev)) : 0.f;  // w to units of 2^ev
 #pragma unroll 4
             for (int j = sub; j < TJ; j += JS) {
                 const float4 h = reinterpret_cast<const float4 *>(b)[j], l = reinterpret_cast<const float4 *>(b)[TJ + j];
                 const float y = seed(h, l);
-                const float my = j == jself ? 0.f : h.w * y, my2 = my * y;
-                if constexpr (MODE != MODE_ENERGY) mg += my2;
-                if constexpr (MODE != MODE_NEWTON) mp += my;
+                const float my = j == jself ? 0.f : h.w * y;
+                const float my2 = my * y;
+                mg += MODE == MODE_ENERGY ? my : my2;
                 if constexpr (FORCE) {
-                    ms = fmaf(my2, y, ms);
-                    mu = fmaf(j == jself ? 0.f : __uint_as_float(b[4 * TJ + j].w), y, mu);
+                    const float4 g7 = reinterpret_cast<const float4 *>(b)[7 * TJ + j];
+                    mc += j == jself ? 0.f : fmaf(fmaf(g7.z, qef, g7.y), y * y, g7.w);
+                    const float wn = __uint_as_float(b[10 * TJ + j].z) * down;  // |F| <= |u| |w| + |w|^2 / 2, |ct| <= |u| + |w|, |u| <= 2^-d
+                    mh = fmaf(my2 * wn, fmaf(0.5f, wn, I.fd), mh);
+                    mt = fmaf(my2, I.fd + wn, mt);
                 }
             }
 #pragma unroll
             for (int off = JS / 2; off > 0; off >>= 1) {
-                if constexpr (MODE != MODE_ENERGY) mg += __shfl_xor_sync(0xffffffffu, mg, off);
-                if constexpr (MODE != MODE_NEWTON) mp += __shfl_xor_sync(0xffffffffu, mp, off);
+                mg += __shfl_xor_sync(0xffffffffu, mg, off);
                 if constexpr (FORCE) {
-                    ms += __shfl_xor_sync(0xffffffffu, ms, off);
-                    mu += __shfl_xor_sync(0xffffffffu, mu, off);
+                    mc += __shfl_xor_sync(0xffffffffu, mc, off);
+                    mh += __shfl_xor_sync(0xffffffffu, mh, off);
+                    mt += __shfl_xor_sync(0xffffffffu, mt, off);
                 }
             }
             E.g = mag_exp(mg);
-            E.p = mag_exp(mp);
-            E.s = mag_exp(ms);
-            E.u = mag_exp(mu);
+            E.c = mag_exp(mc) + ec;
+            E.q = -eL;
+            E.lh = lift(E.g, mag_exp(mh), LIFT_H);
+            E.lt = lift(E.g, mag_exp(mt), LIFT_T);
         }
         // ---- the sums
         clear<MODE>(A);
-        constexpr int CARRY = TJ / JS < 4 ? TJ / JS : 4;
-        for (int j0 = sub; j0 < TJ; j0 += CARRY * JS) {
-#pragma unroll
-            for (int c = 0; c < CARRY; ++c) {
-                const int j = j0 + c * JS;
+        constexpr int FOLD = TJ / JS < 8 ? TJ / JS : 8;
+        for (int j0 = sub; j0 < TJ; j0 += FOLD * JS) {
+#pragma unroll 4  // (2: 1 % slower; 8: 28 %, the loop leaves the instruction cache)
+            for (int j = j0; j < j0 + FOLD * JS; j += JS) {
                 const float4 h = reinterpret_cast<const float4 *>(b)[j], l = reinterpret_cast<const float4 *>(b)[TJ + j];
                 const uint4 g2 = b[2 * TJ + j], g3 = b[3 * TJ + j], g4 = b[4 * TJ + j];
+                auto uf = [](unsigned u) { return __uint_as_float(u); };
                 StarJ J;
                 J.x = {g2.x, g2.y, g2.z};
                 J.y = {g2.w, g3.x, g3.y};
                 J.z = {g3.z, g3.w, g4.x};
-                J.m = ((u64)g4.z << 32) | g4.y;
+                J.mh = g4.y;
+                J.mhf = uf(g4.z);
+                J.ml = uf(g4.w);
                 J.em = j == jself ? -8192 : __float_as_int(l.w);
                 if constexpr (MODE != MODE_NEWTON) {
                     const uint4 g5 = b[5 * TJ + j], g6 = b[6 * TJ + j];
-                    J.wx = {(int)g5.y, (int)g5.x};
-                    J.wy = {(int)g5.w, (int)g5.z};
-                    J.wz = {(int)g6.y, (int)g6.x};
-                    J.m3 = ((u64)g6.w << 32) | g6.z;
+                    J.wx = {(int)g5.x, (int)g5.y};
+                    J.wy = {(int)g5.z, (int)g5.w};
+                    J.wz = {(int)g6.x, (int)g6.y};
                 }
                 if constexpr (FORCE) {
-                    const uint4 g7 = b[7 * TJ + j], g8 = b[8 * TJ + j];
-                    J.em3 = j == jself ? -8192 : (int)g7.x;
-                    J.g1 = __hiloint2double((int)g7.w, (int)g7.z);
-                    J.g3 = __hiloint2double((int)g8.y, (int)g8.x);
-                    J.k = __hiloint2double((int)g8.w, (int)g8.z);
+                    const double2 g8 = reinterpret_cast<const double2 *>(b)[8 * TJ + j], g9 = reinterpret_cast<const double2 *>(b)[9 * TJ + j];
+                    J.m = g8.x;
+                    J.mu3 = g8.y;
+                    J.g1 = g9.x;
+                    J.g3 = g9.y;
+                    J.k = reinterpret_cast<const double2 *>(b)[10 * TJ + j].x;
                 }
                 fix::pair<MODE>(A, I, J, E, __float_as_uint(seed(h, l)), a.fu.eps60);
             }
-            carry<MODE>(A);
+            fold<MODE>(A);
         }
         // ---- the JS lanes' integer sums share their exponents: added exactly; then the FP64 totals
         i64 v[FixInfo<MODE>::NT];
         int ve[FixInfo<MODE>::NT];  // exponent of the value's unit
-        int nv = 0;
-        auto put = [&](i64 x, int e) {
-            v[nv] = x;
-            ve[nv++] = e;
-        };
-        if constexpr (MODE != MODE_ENERGY)
+        const int gn = E.g + eg;
+        if constexpr (MODE == MODE_ENERGY) {
+            v[0] = A.phi;
+            ve[0] = gn - 62;
+            v[1] = top(A.psi);
+            ve[1] = gn - 60 + 2 * ev - 2;
+        } else {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) put(top<TOP_G>(A.gh[k], A.gx[k]), E.g - S_G);
-        if constexpr (MODE != MODE_NEWTON) put(A.phi, E.p - 62);
-        if constexpr (FORCE) {
-            put(A.s0, E.s - 61);
-            put(A.u, E.u - 62);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) put(top<TOP_W>(A.wh[k], A.wx[k]), E.g - S_W + 2 * ev);
-            put(A.ct, E.g - 61 + ev);
+            for (int k = 0; k < 3; ++k) {
+                v[k] = top(A.g[k]);
+                ve[k] = gn - 62;
+            }
         }
-        if constexpr (PSI) put(top<TOP_P>(A.ph, A.px), E.p - S_P + 2 * ev - 2);
+        if constexpr (FORCE) {
+            v[3] = A.s0;
+            ve[3] = gn - eL - 60;
 #pragma unroll
-        for (int q = 0; q < FixInfo<MODE>::NT; ++q) {
+            for (int k = 0; k < 3; ++k) {
+                v[4 + k] = top(A.w[k]);
+                ve[4 + k] = gn + 2 - E.lh - 62 + 2 * ev;
+                v[11 + k] = top(A.t[k]);
+                ve[11 + k] = gn + 2 - E.lt - 62 + 2 * ev;
+                v[7 + k] = top(A.c[k]);
+                ve[7 + k] = E.c - 62;
+            }
+            v[10] = A.ct;
+            ve[10] = gn + 2 - E.lt - 62 + ev;
+        }
+        constexpr int NI64 = FORCE ? 14 : FixInfo<MODE>::NT;
+#pragma unroll
+        for (int q = 0; q < NI64; ++q) {
             i64 x = v[q];
 #pragma unroll
             for (int off = JS / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
             if (sub == 0) tot[q * NT + grp] = ::fma(__ll2double_rn(x), pow2(ve[q]), tot[q * NT + grp]);
         }
+        if constexpr (FORCE) {
+            const double d[3] = {A.dphi, A.du, A.dpsi};
+#pragma unroll
+            for (int q = 0; q < FixInfo<MODE>::NT - 14; ++q) {
+                double x = d[q];
+#pragma unroll
+                for (int off = JS / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+                double &t = tot[(14 + q) * NT + grp];
+                if (sub == 0) t = q < 2 ? t + x : ::fma(x, pow2(2 * ev - 61), t);
+            }
+        }
         __syncthreads();  // every thread is done with this stage before it is refilled
     }
 
-    if constexpr (FORCE)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int off = JS / 2; off > 0; off >>= 1) A.w[k] += __shfl_xor_sync(0xffffffffu, A.w[k], off);
     if (sub == 0 && valid) {
-        // back to the system's units
-        const int e0 = fix::expo(a.m[0]), eL = a.fu.eL;
-        const double fp = pow2(e0 - eL), fg = pow2(e0 - 2 * eL);
-        // the pair of the star with itself belongs to the range that holds its tile
-        const bool has_self = i / TJ >= t0 && i / TJ < t1;
-        const double mi = has_self ? a.m[i + 1] : 0.0, Qs = a.fu.inv_eps;
         auto T = [&](int q) { return tot[q * NT + grp]; };
         auto out = [&](int slot, double x) { a.out[((size_t)split * NACC + slot) * a.npad + i] = x; };
+        // the pair of the star with itself: in the FP64 sums where they are formed (self at Q = 1 / eps),
+        // left out of the integer sums and added here by the range that holds its tile
+        const double mi = i / TJ >= t0 && i / TJ < t1 ? a.m[i + 1] : 0.0;
         double v[3] = {0.0, 0.0, 0.0}, vi2 = 0.0;
         if constexpr (MODE != MODE_NEWTON) {
 #pragma unroll
@@ -270,27 +308,23 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
             vi2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
         }
         if constexpr (MODE == MODE_NEWTON) {
-            for (int k = 0; k < 3; ++k) out(A_GX + k, fg * T(k));
+            for (int k = 0; k < 3; ++k) out(A_GX + k, T(k));
         } else if constexpr (MODE == MODE_ENERGY) {
-            out(E_PHI, ::fma(mi, Qs, fp * T(0)));
-            out(E_PSI, ::fma(7.0 * vi2, mi * Qs, fp * T(1)));
+            out(E_PHI, ::fma(mi, a.fu.inv_eps, T(0)));
+            out(E_PSI, ::fma(7.0 * vi2, mi * a.fu.inv_eps, T(1)));
         } else {
-            const uint4 g6 = pk[(size_t)6 * a.npad + i], g7 = pk[(size_t)7 * a.npad + i];
-            const u64 m3 = has_self ? ((u64)g6.w << 32) | g6.z : 0;
-            const double mu3 = m3 ? scale_down(__ull2double_rn(m3), 64 - ((int)g7.x + e0 - 3 * eL)) : 0.0;
-            out(A_PHI, ::fma(mi, Qs, fp * T(3)));
-            out(A_S0, ::fma(mi, a.fu.inv_eps3, pow2(e0 - 3 * eL) * T(4)));
-            out(A_U, ::fma(mu3, Qs, pow2(e0 - 4 * eL) * T(5)));
+            out(A_PHI, T(14));
+            out(A_S0, ::fma(mi, a.fu.inv_eps3, T(3)));
+            out(A_U, T(15));
             // the velocity factors of the star itself: -|v_i|^2 G and -3/4 u_i sum ct = -sqrt(3) v_i sum ct
-            const double cs = -fix::W_SCALE * fg * T(9);
+            const double cs = -fix::W_SCALE * T(10);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const double g = fg * T(k);
+                const double g = T(k);
                 out(A_GX + k, g);
-                out(A_WX + k, ::fma(cs, v[k], fg * T(6 + k)) + ::fma(-vi2, g, A.w[k] * (1.0 / 576460752303423488.0)));
+                out(A_WX + k, ::fma(cs, v[k], T(4 + k) + T(11 + k)) + ::fma(-vi2, g, T(7 + k)));
             }
-            if constexpr (MODE == MODE_FORCE_ENERGY)
-                out(A_PSI, ::fma(7.0 * vi2, mi * Qs, fp * T(10)));
+            if constexpr (MODE == MODE_FORCE_ENERGY) out(A_PSI, T(16));
         }
     }
     seq += (uint32_t)(t1 - t0 > 0 ? t1 - t0 : 0);

@@ -15,7 +15,6 @@ typedef long double L;
 struct Star {
     double s[3], v[3], m;
 };
-static double rsq(double x) { return 1.0 / std::sqrt(x); }
 
 static double two(int e) { return std::ldexp(1.0, e); }
 static int mag_exp(float x) { x *= 1.001f; unsigned b; std::memcpy(&b, &x, 4); return (int)(b >> 23) - 126; }
@@ -86,7 +85,8 @@ int main() {
     const int e0 = expo(m0);
     const double eps2 = eps * eps;
     std::vector<StarJ> J(n);
-    std::vector<float> mf(n), m3f(n);
+    std::vector<float> mf(n), g1f(n), g3f(n), kf(n), wn(n);
+    float un = 0;
     StarI I;
     double vi2 = 0;
     for (int j = 0; j < n; ++j) {
@@ -99,75 +99,105 @@ int main() {
         p.wx = bal(to_scaled(b.v[0], W_MANT, 63, 60, ev));
         p.wy = bal(to_scaled(b.v[1], W_MANT, 63, 60, ev));
         p.wz = bal(to_scaled(b.v[2], W_MANT, 63, 60, ev));
-        p.m = mantissa(b.m, p.em);
-        p.em = p.m ? p.em - e0 : -8192;
-        p.m3 = mantissa(mu3, p.em3);
-        p.em3 = p.m3 ? p.em3 - e0 + 3 * eL : -8192;
-        p.g1 = b.m * (c1 - 2.0 * v2) * two(-62 - 2 * eL);
-        p.g3 = b.m * c3 * two(-62 - 2 * eL);
+        const u64 mm = mantissa(b.m, p.em);
+        p.em = mm ? p.em - e0 : -8192;
+        p.mh = (unsigned)(mm >> 32);
+        p.mhf = (float)p.mh * 0x1p-34f;
+        p.ml = (float)(unsigned)mm * 0x1p-34f;
+        p.m = b.m;
+        p.mu3 = mu3;
+        p.g1 = b.m * (c1 - 2.0 * v2);
+        p.g3 = b.m * c3;
         p.k = std::fma(b.m, c3, k35);
         mf[j] = (float)(b.m * two(-e0));
-        m3f[j] = (float)(mu3 * two(3 * eL - e0));
+        g1f[j] = (float)std::fabs(p.g1 * two(eL - 2 * e0));
+        g3f[j] = (float)(p.g3 * two(3 * eL - 2 * e0));
+        kf[j] = (float)(p.k * two(3 * eL - 2 * e0));
+        wn[j] = std::sqrt((float)(3.0 * v2 * two(-2 * ev))) * 1.00001f;
         if (j == i) {
+            un = (float)two(-(ev - speed_exp(v2) < 63 ? ev - speed_exp(v2) : 63));
             I.x = p.x; I.y = p.y; I.z = p.z;
-            I.ux = bal(to_scaled(b.v[0], U_MANT, 62, 62, ev));
-            I.uy = bal(to_scaled(b.v[1], U_MANT, 62, 62, ev));
-            I.uz = bal(to_scaled(b.v[2], U_MANT, 62, 62, ev));
+            const int eu = speed_exp(v2);
+            I.ux = vec(bal(to_scaled(b.v[0], U_MANT, 62, 62, eu)));
+            I.uy = vec(bal(to_scaled(b.v[1], U_MANT, 62, 62, eu)));
+            I.uz = vec(bal(to_scaled(b.v[2], U_MANT, 62, 62, eu)));
+            I.d = ev - eu < 63 ? ev - eu : 63;
+            I.fd = (float)two(-I.d);
             I.qe = q + eps2;
             vi2 = v2;
         }
     }
-    double tot[11] = {0};
+    const float qef = (float)(I.qe * two(-2 * eL));
+    const bool energy = mode == F_ENERGY;
+    double tot[12] = {0};
     Sums A;
-    A.w[0] = A.w[1] = A.w[2] = 0;
+    double phi = 0, us = 0;
     unsigned rnd = 12345;
     for (int t = 0; t < n; t += 128) {
         const int e = t + 128 < n ? t + 128 : n;
         std::vector<unsigned> yb(128);
-        float mg = 0, mp = 0, ms = 0, mu = 0;
+        float mg = 0, mc = 0, mh = 0, mt = 0;
         for (int j = t; j < e; ++j) {
             double rho = eq * eq;
             for (int k = 0; k < 3; ++k) { const double d = (st[j].s[k] - st[i].s[k]) * two(-eL); rho += d * d; }
             rnd = rnd * 1664525u + 1013904223u;  // a seed off by at most err
             const float y = (float)((1.0 / std::sqrt(rho)) * (1.0 + err * (2.0 * (rnd / 4294967296.0) - 1.0)));
             std::memcpy(&yb[j - t], &y, 4);
-            if (j == i) continue;
-            mg += mf[j] * y * y; mp += mf[j] * y; ms += mf[j] * y * y * y; mu += m3f[j] * y;
+            if (j != i) {
+                const float my2 = mf[j] * y * y;
+                mh += my2 * wn[j] * (un + 0.5f * wn[j]);
+                mt += my2 * (un + wn[j]);
+            }
+            if (j != i) mg += energy ? mf[j] * y : mf[j] * y * y;
+            if (j != i) mc += (g3f[j] * qef + g1f[j]) * (y * y) + kf[j];
         }
-        Scale E{mag_exp(mg), mag_exp(mp), mag_exp(ms), mag_exp(mu)};
+        const int lh = lift(mag_exp(mg), mag_exp(mh), LIFT_H), lt = lift(mag_exp(mg), mag_exp(mt), LIFT_T);
+        const Scale E{mag_exp(mg), mag_exp(mc) + 2 * e0 - 3 * eL, -eL, lh, lt};
         clear<F_FORCE_ENERGY>(A);
         for (int j = t; j < e; ++j) {
-            const int em = J[j].em, em3 = J[j].em3;
-            if (j == i) J[j].em = J[j].em3 = -8192;
+            const int em = J[j].em;
+            if (j == i) J[j].em = -8192;
             if (mode == 0) pair<F_NEWTON>(A, I, J[j], E, yb[j - t], eps60);
             else if (mode == 1) pair<F_FORCE>(A, I, J[j], E, yb[j - t], eps60);
             else if (mode == 2) pair<F_ENERGY>(A, I, J[j], E, yb[j - t], eps60);
             else pair<F_FORCE_ENERGY>(A, I, J[j], E, yb[j - t], eps60);
             J[j].em = em;
-            J[j].em3 = em3;
-            if ((j & 3) == 3 || j + 1 == e) carry<F_FORCE_ENERGY>(A);
+            if ((j & 7) == 7 || j + 1 == e) {
+                if (energy) fold<F_ENERGY>(A);
+                else fold<F_FORCE>(A);
+            }
         }
+        const int gn = E.g + e0 - (energy ? 1 : 2) * eL;
         for (int k = 0; k < 3; ++k) {
-            tot[k] += (double)top<TOP_G>(A.gh[k], A.gx[k]) * two(E.g - S_G);
-            tot[6 + k] += (double)top<TOP_W>(A.wh[k], A.wx[k]) * two(E.g - S_W);
+            tot[k] += (double)top(A.g[k]) * two(gn - 62);
+            tot[4 + k] += (double)top(A.w[k]) * two(gn + 2 - lh - 62 + 2 * ev) + (double)top(A.t[k]) * two(gn + 2 - lt - 62 + 2 * ev);
+            tot[7 + k] += (double)top(A.c[k]) * two(E.c - 62);
         }
-        tot[3] += (double)A.phi * two(E.p - 62);
-        tot[4] += (double)A.s0 * two(E.s - 61);
-        tot[5] += (double)A.u * two(E.u - 62);
-        tot[9] += (double)A.ct * two(E.g - 61);
-        tot[10] += (double)top<TOP_P>(A.ph, A.px) * two(E.p - S_P);
+        tot[3] += (double)A.s0 * two(gn - eL - 60);
+        tot[10] += (double)A.ct * two(gn + 2 - lt - 62 + ev);
+        if (energy) {
+            tot[0] += (double)A.phi * two(gn - 62);
+            tot[1] += (double)top(A.psi) * two(gn - 62 + 2 * ev);
+        }
+        tot[11] += A.dpsi * two(2 * ev - 61);
+        phi += A.dphi;
+        us += A.du;
     }
-    const double fp = two(e0 - eL), fg = two(e0 - 2 * eL), fv = fg * two(2 * ev);
-    double f[10];
-    for (int k = 0; k < 3; ++k) {
-        f[k] = fg * tot[k];
-        f[6 + k] = std::fma(-W_SCALE * (fg * two(ev)) * tot[9], st[i].v[k], fv * tot[6 + k]) + std::fma(-vi2, f[k], A.w[k] * two(-59));
+    const double Qs = 1.0 / eps, mi = st[i].m;
+    double f[10] = {0};
+    if (energy) {
+        f[3] = std::fma(mi, Qs, tot[0]);
+        f[9] = std::fma(7.0 * vi2, mi * Qs, tot[1]);
+    } else {
+        for (int k = 0; k < 3; ++k) {
+            f[k] = tot[k];
+            f[6 + k] = std::fma(-W_SCALE * tot[10], st[i].v[k], tot[4 + k]) + std::fma(-vi2, f[k], tot[7 + k]);
+        }
+        f[3] = phi;
+        f[4] = std::fma(mi, (double)(1.0L / ((L)eps * eps * eps)), tot[3]);
+        f[5] = us;
+        f[9] = tot[11];
     }
-    const double Qs = 1.0 / eps, mi = st[i].m, mu3 = mi * rsq(I.qe) * rsq(I.qe) * rsq(I.qe);
-    f[3] = std::fma(mi, Qs, fp * tot[3]);
-    f[4] = std::fma(mi, (double)(1.0L / ((L)eps * eps * eps)), two(e0 - 3 * eL) * tot[4]);
-    f[5] = std::fma(mu3, Qs, two(e0 - 4 * eL) * tot[5]);
-    f[9] = std::fma(7.0 * vi2, mi * Qs, fp * 0.25 * two(2 * ev) * tot[10]);
     Terms<double> d;
     Terms<L> x;
     plain<double>(st, i, eps, m0, d);
