@@ -120,6 +120,32 @@ static void choose_fix(PairCfg *k, int nstar, int sms) {
         }
 }
 
+// Shape of the packed mixed-precision sweep where none was tuned: i per thread and j-range splits, from
+// a model of its time in microseconds: the CTAs of the busiest SM times their work (58 cycles per pair of
+// a warp, 2.07 GHz) over the share of the FMA pipe that as many CTAs of 4 warps keep busy, and 0.6 us
+// per split in the finishing kernel.  Measured against the former rule (2 i per thread from N = 4096,
+// about 32 CTAs per SM, the 2-CTA build): N = 1,001 pair 28.6 -> 12.5 us, 4,096: 75.9 -> 42.5,
+// 12,000: 281 -> 234, 16,384: 424 either way, 65,536: 6.57 -> 6.33 ms, 262,144: 101.2 -> 100.3 ms.
+static void choose_packed(PairCfg *k, int nstar, int sms) {
+    static const double busy[2][4] = {{0.40, 0.70, 0.85, 0.92}, {0.62, 0.88, 1.0, 1.0}};
+    k->js = 1;
+    double best = 1e300;
+    for (int ipt = 1; ipt <= 2; ++ipt) {
+        const int tj = 128 * ipt, ntiles = (nstar + tj - 1) / tj, nib = (nstar + 128 * ipt - 1) / (128 * ipt);
+        for (int g = 1; g <= 32 && g <= ntiles; ++g) {
+            const int n = (nib * g + sms - 1) / sms;
+            const double work = (double)((ntiles + g - 1) / g) * tj * ipt * 58.0 + 5000.0 * ipt;
+            const double cost = n * work / busy[ipt - 1][n < 4 ? n - 1 : 3] / 2070.0 + 0.6 * g;
+            if (cost < best) {
+                best = cost;
+                k->ipt = ipt;
+                k->tj = tj;
+                k->gsplit = g;
+            }
+        }
+    }
+}
+
 // Launch shape of the pair sweep: explicit parameters win; otherwise a heuristic sized for
 // GB300 (152 SMs): enough CTAs for several waves, split along j when there are few i-blocks.
 static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
@@ -161,12 +187,10 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
         if (k.js != 1) k.js = 1;
         const bool occ = k.ipt == 2 && mode_has_force(mode);
         k.x2 = (occ && pv == PN_PAIR_F32X2_OCC3) ? 2 : (occ && pv == PN_PAIR_F32X2_OCC4) ? 3 : 1;
-    } else if (pv == PN_PAIR_AUTO && f32 && !explicit_shape) {
-        // untuned default of the mixed sweep: the packed f32x2 form, 2 i per thread for
-        // N >= 4096 (fastest in the tuner's measurements at N = 2^18: 111 ms vs 125 ms)
-        k.ipt = nstar >= 4096 ? 2 : 1;
-        k.js = 1;
-        k.x2 = 1;
+    } else if (pv == PN_PAIR_AUTO && f32 && !explicit_shape && nstar > 0) {
+        choose_packed(&k, nstar, c->sms);
+        k.x2 = k.ipt == 2 && mode_has_force(mode) ? 2 : 1;
+        return k;
     } else {
         k.x2 = 0;  // scalar sweep: FP64, PN_PAIR_SCALAR, or an explicit shape without the variant
     }
@@ -196,6 +220,7 @@ int pn::ensure_acc(pn_ctx *c, int splits) {
     if (c->acc) cudaFree(c->acc);
     c->acc = nullptr;
     c->acc_splits = 0;
+    c->step_valid = c->timed_valid = false;  // captured steps hold the old buffer
     // room for the widest sweep: the force sweep with the fused energy sum
     size_t bytes = (size_t)splits * pair_nacc(MODE_FORCE_ENERGY) * (size_t)c->npad * sizeof(double);
     if (cudaMalloc(&c->acc, bytes) != cudaSuccess) {
@@ -210,6 +235,7 @@ static void free_ctx(pn_ctx *c) {
     if (!c) return;
     free_adjoint(c);
     if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
+    if (c->timed_exec) cudaGraphExecDestroy(c->timed_exec);
     void *bufs[] = {c->state_buf, c->a_aos, c->in_aos, c->spos, c->pack, c->pack2, c->ipack, c->fpack, c->fix_bad, c->torg, c->acc,
                     c->part, c->glob, c->eout, c->tickets, c->err};
     for (void *b : bufs)
@@ -322,7 +348,7 @@ extern "C" int pn_set_params(pn_ctx *c, const pn_params *p) {
     if (!c || validate_params(p) != PN_OK) return set_err(PN_ERR_INVALID, "pn_set_params");
     c->p = *p;
     c->cfg_set = false;
-    c->step_valid = false;
+    c->step_valid = c->timed_valid = false;
     return PN_OK;
 }
 
@@ -391,7 +417,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
         EnergyArgs ea{};
         ea.v = v; ea.m = m; ea.sp = sp; ea.sk = sk;
         ea.spos = c->spos; ea.acc = c->acc; ea.glob = c->glob;
-        ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit;
+        ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit; ea.accf = 0;
         ea.nacc = pair_nacc(mode); ea.sphi = A_PHI; ea.spsi = A_PSI;
         ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2; ea.inv_eps = 1.0 / c->p.eps;
         ea.part = c->part + on_blocks(c->npad) * 8;
@@ -403,6 +429,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     fa.v = v; fa.m = m; fa.vsp = sp; fa.vsk = sk;
     fa.spos = c->spos; fa.acc = c->acc; fa.glob = c->glob;
     fa.nstar = nstar; fa.npad = c->npad; fa.nacc = pair_nacc(mode); fa.gsplit = k.gsplit;
+    fa.accf = is_f32(c) && k.x2 && !with_energy;
     fa.pn1 = mode_has_force(mode) && c->p.inv_c2 != 0.0;
     fa.eps = c->p.eps; fa.eps2 = eps2; fa.inv_c2 = c->p.inv_c2; fa.dt = c->p.dt; fa.inv_eps = 1.0 / c->p.eps;
     fa.a = a_out; fa.asp = asp; fa.ask = ask;
@@ -458,7 +485,7 @@ extern "C" int pn_set_state(pn_ctx *c, int n, const double *x, const double *v, 
     cudaError_t e4 = cudaStreamSynchronize(c->stream);
     cudaFreeHost(h);
     if (e1 || e2 || e3 || e4) return set_err(PN_ERR_CUDA, "pn_set_state: copy failed");
-    if (n != c->n) { c->cfg_set = false; c->step_valid = false; }
+    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
     c->n = n;
     c->time = 0.0;
     c->have_state = true;
@@ -505,7 +532,7 @@ extern "C" int pn_force_device(pn_ctx *c, int n, const double *d_x, const double
     if (!c || n < 1 || n > c->nmax || !d_x || !d_v || !d_m || !d_a)
         return set_err(PN_ERR_INVALID, "pn_force_device");
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-    if (n != c->n) { c->cfg_set = false; c->step_valid = false; }
+    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
     c->n = n;
     return eval_force(c, d_x, d_v, d_m, 3, 1, d_a, 3, 1, 0, s, false);
 }
@@ -515,38 +542,44 @@ static int step_evaluations(const pn_ctx *c) { return c->p.integrator == PN_INT_
 
 // energy_first: the first evaluation (at the step's starting state) also yields the energies of
 // that state in c->eout.
-static int enqueue_step(pn_ctx *c, cudaStream_t s, bool energy_first = false) {
+// timed: events around the pair sweeps.
+static int enqueue_step(pn_ctx *c, cudaStream_t s, bool energy_first = false, bool timed = false) {
     const long long ld = c->ld;
+    auto slot = [&](int k) { return timed ? k : -1; };
     if (c->p.integrator == PN_INT_RK4) {  // classic RK4: evaluations at y, y2, y3, y4
-        int rc = eval_force(c, c->st.x, c->st.v, c->st.m, 1, ld, nullptr, 3, 1, STAGE_RK4_1, s, false, 0,
+        int rc = eval_force(c, c->st.x, c->st.v, c->st.m, 1, ld, nullptr, 3, 1, STAGE_RK4_1, s, false, slot(0),
                             nullptr, energy_first);
         for (int k = 1; k < 4 && !rc; ++k)
-            rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, STAGE_RK4_1 + k, s, false, k);
+            rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, STAGE_RK4_1 + k, s, false, slot(k));
         return rc;
     }
-    int rc = eval_force(c, c->st.x, c->st.v, c->st.m, 1, ld, nullptr, 3, 1, 1, s, false, 0, nullptr,
+    int rc = eval_force(c, c->st.x, c->st.v, c->st.m, 1, ld, nullptr, 3, 1, 1, s, false, slot(0), nullptr,
                         energy_first);
-    if (!rc) rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, 2, s, false, 1);
-    if (!rc) rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, 3, s, false, 2);
+    if (!rc) rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, 2, s, false, slot(1));
+    if (!rc) rc = eval_force(c, c->st.xs, c->st.vs, c->st.m, 1, ld, nullptr, 3, 1, 3, s, false, slot(2));
     return rc;
 }
 
-static int build_step_graph(pn_ctx *c) {
-    if (c->step_valid) return PN_OK;
-    if (c->step_exec) { cudaGraphExecDestroy(c->step_exec); c->step_exec = nullptr; }
+// The captured step: for pn_steps, and (timed) with events around each pair sweep for pn_bench_steps.
+static int build_step_graph(pn_ctx *c, bool timed = false) {
+    cudaGraphExec_t &exec = timed ? c->timed_exec : c->step_exec;
+    bool &valid = timed ? c->timed_valid : c->step_valid;
+    if (valid) return PN_OK;
+    if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     refresh_cfg(c);
-    int rc = ensure_acc(c, c->cfg_force.gsplit);  // allocate before capture
+    // allocate before capture, for the energy sweep too (a later allocation would make the step stale)
+    int rc = ensure_acc(c, c->cfg_force.gsplit > c->cfg_energy.gsplit ? c->cfg_force.gsplit : c->cfg_energy.gsplit);
     if (rc) return rc;
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = enqueue_step(c, c->stream);
+    rc = enqueue_step(c, c->stream, false, timed);
     cudaError_t ec = cudaStreamEndCapture(c->stream, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (ec != cudaSuccess) return set_err(PN_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ec));
-    cudaError_t ei = cudaGraphInstantiate(&c->step_exec, g, 0);
+    cudaError_t ei = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (ei != cudaSuccess) return set_err(PN_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ei));
-    c->step_valid = true;
+    valid = true;
     return PN_OK;
 }
 
@@ -746,7 +779,7 @@ static int eval_energy(pn_ctx *c, const double *x, const double *v, const double
     EnergyArgs ea{};
     ea.v = v; ea.m = m; ea.sp = sp; ea.sk = sk;
     ea.spos = c->spos; ea.acc = c->acc; ea.glob = c->glob;
-    ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit;
+    ea.nstar = nstar; ea.npad = c->npad; ea.gsplit = k.gsplit; ea.accf = is_f32(c) && k.x2;
     ea.nacc = pair_nacc(MODE_ENERGY); ea.sphi = E_PHI; ea.spsi = E_PSI;
     ea.eps = c->p.eps; ea.eps2 = eps2; ea.inv_c2 = c->p.inv_c2; ea.inv_eps = 1.0 / c->p.eps;
     ea.part = c->part + on_blocks(c->npad) * 8;
@@ -832,7 +865,7 @@ static int drop_upload(pn_ctx *c, const double *x, const double *v, const double
     CU(cudaMemcpyAsync(c->in_aos, g_drop_h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->in_aos + 3 * ld, g_drop_h + 3 * ld, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->in_aos + 6 * ld, g_drop_h + 6 * ld, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    if (n != c->n) { c->cfg_set = false; c->step_valid = false; }
+    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
     c->n = n;
     return PN_OK;
 }
@@ -939,7 +972,7 @@ extern "C" int pn_bench_steps(pn_ctx *c, int nsteps, int flush_l2, double *step_
     if (!c || !c->have_state) return set_err(PN_ERR_STATE, "pn_bench_steps: no state");
     if (nsteps < 0 || (nsteps > 0 && (!step_ms || !pair_ms)))
         return set_err(PN_ERR_INVALID, "pn_bench_steps");
-    int rc = build_step_graph(c);
+    int rc = build_step_graph(c, true);
     if (rc) return rc;
     if (flush_l2 && !c->flush) {
         int l2 = 0;
@@ -954,7 +987,7 @@ extern "C" int pn_bench_steps(pn_ctx *c, int nsteps, int flush_l2, double *step_
     for (int k = 0; k < nsteps; ++k) {
         if (flush_l2) CU(cudaMemsetAsync(c->flush, k & 0xff, c->flush_bytes, c->stream));
         CU(cudaEventRecord(c->ev0, c->stream));
-        CU(cudaGraphLaunch(c->step_exec, c->stream));
+        CU(cudaGraphLaunch(c->timed_exec, c->stream));
         CU(cudaEventRecord(c->ev1, c->stream));
         CU(cudaStreamSynchronize(c->stream));
         c->time += c->p.dt;
@@ -1168,7 +1201,7 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
         if (best_ms) best_ms[which] = best_t;
     }
     c->cfg_set = false;
-    c->step_valid = false;
+    c->step_valid = c->timed_valid = false;
     return PN_OK;
 }
 

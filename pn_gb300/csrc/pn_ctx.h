@@ -40,6 +40,8 @@ struct pn_ctx {
     bool have_state = false;
     cudaGraphExec_t step_exec = nullptr;
     bool step_valid = false;
+    cudaGraphExec_t timed_exec = nullptr;  // the same step with events around its pair sweeps
+    bool timed_valid = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     cudaEvent_t evp[8] = {};      // around the pair launches of a captured step (3, or 4 for RK4)
     void *flush = nullptr;        // L2 flush buffer (benchmarks only)

@@ -91,6 +91,55 @@ __device__ __forceinline__ float two_diff(float a, float b, float &err) {
     return s;
 }
 
+// ------------------------------------------------------------------ conversions off the FP64 pipe
+// A double rounded to FP32, and as an FP32 pair hi = fl32(x), lo = fl32(x - hi), by integer
+// operations (an FP64 conversion or subtraction costs 64 cycles of the FP64 pipe per warp); exponents
+// that leave FP32's range, infinities and NaN take the FP64 instructions.
+__device__ __forceinline__ bool f32_range(double x) {
+    const int be = (__double2hiint(x) >> 20) & 0x7ff;
+    return be - 943u < 180u;  // 2^-80 <= |x| < 2^100
+}
+__device__ __forceinline__ float f32_bits(long long b) {  // of |x|'s bits plus the rounding bit
+    return __uint_as_float((unsigned)(b >> 29) - (896u << 23));
+}
+__device__ __forceinline__ float to_f32(double x) {
+    if (!f32_range(x)) return (float)x;
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    return copysignf(f32_bits(b + 0x10000000LL), __int_as_float(__double2hiint(x)));
+}
+__device__ __forceinline__ void to_f32_pair(double x, float &hi, float &lo) {
+    if (!f32_range(x)) {
+        hi = (float)x;
+        lo = (float)(x - (double)hi);
+        return;
+    }
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    int low = (int)(b & 0x1fffffff);
+    if (low >= 0x10000000) low -= 0x20000000;  // hi was rounded up
+    const float sg = __int_as_float((__double2hiint(x) & 0x80000000) | 0x3f800000);
+    const int e = (int)(b >> 52) - 1023 - 52;  // the unit of x's last bit
+    hi = sg * f32_bits(b + 0x10000000LL);
+    lo = sg * ((float)low * __int_as_float((e + 127 + 30) << 23)) * 9.31322574615478515625e-10f;  // 2^-30
+}
+// x 2^e
+__device__ __forceinline__ double scale2(double x, int e) {
+    const int be = (__double2hiint(x) >> 20) & 0x7ff;
+    if (be == 0 || be == 0x7ff || be + e <= 0 || be + e >= 0x7ff) return ldexp(x, e);
+    return __hiloint2double(__double2hiint(x) + (e << 20), __double2loint(x));
+}
+// An FP32 number as a double.
+__device__ __forceinline__ double to_f64(float x) {
+    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xff;
+    if (e - 1u > 253u) return (double)x;  // zero, denormal, infinite, NaN
+    return __hiloint2double((int)((b & 0x80000000u) | (((b >> 3) & 0x0fffffffu) + 0x38000000u)), (int)(b << 29));
+}
+// (h, l) += the FP32 pair t: the high parts exactly (Knuth's TwoSum), the rest into l.
+__device__ __forceinline__ void pair_add(float &h, float &l, float2 t) {
+    const float s = h + t.x, b = s - h;
+    l += ((h - (s - b)) + (t.x - b)) + t.y;
+    h = s;
+}
+
 // ------------------------------------------------------------------ device error word bits
 enum DevErr : int { DEVERR_TIMEOUT = 1, DEVERR_NONFINITE = 2 };
 

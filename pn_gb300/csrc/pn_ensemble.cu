@@ -213,6 +213,7 @@ static int ens_build_tables(pn_ens *e) {
             fa.npad = e->S;
             fa.nacc = pair_nacc(mode);
             fa.gsplit = g;
+            fa.accf = f32 && e->x2 && e->js == 1;
             fa.pn1 = mode == MODE_FORCE;
             fa.eps = eps;
             fa.eps2 = eps2;
@@ -241,6 +242,7 @@ static int ens_build_tables(pn_ens *e) {
         ea.nstar = nstar;
         ea.npad = e->S;
         ea.gsplit = g;
+        ea.accf = f32 && e->x2 && e->js == 1;
         ea.nacc = pair_nacc(MODE_ENERGY);
         ea.sphi = E_PHI;
         ea.spsi = E_PSI;

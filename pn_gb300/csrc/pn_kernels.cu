@@ -105,43 +105,6 @@ __device__ __forceinline__ bool last_block(unsigned *ticket, int nblk) {
     return am_last;
 }
 
-// ------------------------------------------------------------------ conversions off the FP64 pipe
-// A double rounded to FP32, and as an FP32 pair hi = fl32(x), lo = fl32(x - hi), by integer
-// operations (an FP64 conversion or subtraction costs 64 cycles of the FP64 pipe per warp); exponents
-// that leave FP32's range, infinities and NaN take the FP64 instructions.
-__device__ __forceinline__ bool f32_range(double x) {
-    const int be = (__double2hiint(x) >> 20) & 0x7ff;
-    return be - 943u < 180u;  // 2^-80 <= |x| < 2^100
-}
-__device__ __forceinline__ float f32_bits(long long b) {  // of |x|'s bits plus the rounding bit
-    return __uint_as_float((unsigned)(b >> 29) - (896u << 23));
-}
-__device__ __forceinline__ float to_f32(double x) {
-    if (!f32_range(x)) return (float)x;
-    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-    return copysignf(f32_bits(b + 0x10000000LL), __int_as_float(__double2hiint(x)));
-}
-__device__ __forceinline__ void to_f32_pair(double x, float &hi, float &lo) {
-    if (!f32_range(x)) {
-        hi = (float)x;
-        lo = (float)(x - (double)hi);
-        return;
-    }
-    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-    int low = (int)(b & 0x1fffffff);
-    if (low >= 0x10000000) low -= 0x20000000;  // hi was rounded up
-    const float sg = __int_as_float((__double2hiint(x) & 0x80000000) | 0x3f800000);
-    const int e = (int)(b >> 52) - 1023 - 52;  // the unit of x's last bit
-    hi = sg * f32_bits(b + 0x10000000LL);
-    lo = sg * ((float)low * __int_as_float((e + 127 + 30) << 23)) * 9.31322574615478515625e-10f;  // 2^-30
-}
-// x 2^e
-__device__ __forceinline__ double scale2(double x, int e) {
-    const int be = (__double2hiint(x) >> 20) & 0x7ff;
-    if (be == 0 || be == 0x7ff || be + e <= 0 || be + e >= 0x7ff) return ldexp(x, e);
-    return __hiloint2double(__double2hiint(x) + (e << 20), __double2loint(x));
-}
-
 // ------------------------------------------------------------------ prep
 // The fixed-point sweep's pack of star j (pn_pairfix.cuh): s, its tile's origin o and velocity unit
 // 2^ev, v, m, mu3 and the FP64 coefficients of the W sum.  A padding star has no mass and sits at its tile's origin.
@@ -417,12 +380,28 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
         // the force slots only (a fused-energy sweep has one more, read by the energy kernel)
         const int nk = a.nacc < NACC_MAX ? a.nacc : NACC_MAX;
         double S[NACC_MAX];
+        if (a.accf) {  // FP32 pairs, added in FP32 without loss of their low parts
+            const float2 *p = reinterpret_cast<const float2 *>(a.acc) + i;
+            float h[NACC_MAX], l[NACC_MAX];
 #pragma unroll
-        for (int k = 0; k < NACC_MAX; ++k) S[k] = k < nk ? a.acc[(size_t)k * a.npad + i] : 0.0;
-        for (int g = 1; g < a.gsplit; ++g)
+            for (int k = 0; k < NACC_MAX; ++k) h[k] = l[k] = 0.f;
+#pragma unroll 4
+            for (int g = 0; g < a.gsplit; ++g)
 #pragma unroll
-            for (int k = 0; k < NACC_MAX; ++k)
-                if (k < nk) S[k] += a.acc[((size_t)g * a.nacc + k) * a.npad + i];
+                for (int k = 0; k < NACC_MAX; ++k)
+                    if (k < nk) pair_add(h[k], l[k], p[((size_t)g * a.nacc + k) * a.npad]);
+#pragma unroll
+            for (int k = 0; k < NACC_MAX; ++k) S[k] = to_f64(h[k]) + to_f64(l[k]);
+            S[A_PHI] *= X2_K * X2_K;  // the packed sweep's scale
+        } else {
+#pragma unroll
+            for (int k = 0; k < NACC_MAX; ++k) S[k] = k < nk ? a.acc[(size_t)k * a.npad + i] : 0.0;
+#pragma unroll 2
+            for (int g = 1; g < a.gsplit; ++g)
+#pragma unroll
+                for (int k = 0; k < NACC_MAX; ++k)
+                    if (k < nk) S[k] += a.acc[((size_t)g * a.nacc + k) * a.npad + i];
+        }
         if (a.sums_out)
             for (int k = 0; k < nk; ++k) a.sums_out[(size_t)k * a.npad + i] = S[k];
         const double Gv[3] = {S[A_GX], S[A_GY], S[A_GZ]};
@@ -516,9 +495,20 @@ __device__ __forceinline__ void energy_body(const EnergyArgs &a, int blk, int nb
                              ld_x(a.v, a.sp, a.sk, p, 2)};
         const double mi = a.m[p];
         double Phi = 0.0, Psi = 0.0;
-        for (int g = 0; g < a.gsplit; ++g) {
-            Phi += a.acc[((size_t)g * a.nacc + a.sphi) * a.npad + i];
-            Psi += a.acc[((size_t)g * a.nacc + a.spsi) * a.npad + i];
+        if (a.accf) {
+            const float2 *p = reinterpret_cast<const float2 *>(a.acc) + i;
+            float h[2] = {0.f, 0.f}, l[2] = {0.f, 0.f};
+            for (int g = 0; g < a.gsplit; ++g) {
+                pair_add(h[0], l[0], p[((size_t)g * a.nacc + a.sphi) * a.npad]);
+                pair_add(h[1], l[1], p[((size_t)g * a.nacc + a.spsi) * a.npad]);
+            }
+            Phi = (to_f64(h[0]) + to_f64(l[0])) * (X2_K * X2_K);
+            Psi = to_f64(h[1]) + to_f64(l[1]);
+        } else {
+            for (int g = 0; g < a.gsplit; ++g) {
+                Phi += a.acc[((size_t)g * a.nacc + a.sphi) * a.npad + i];
+                Psi += a.acc[((size_t)g * a.nacc + a.spsi) * a.npad + i];
+            }
         }
         const double q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
         const double R = rsqrt(q + eps2);

@@ -52,6 +52,7 @@ struct FinishArgs {
     long long vsp, vsk;
     const double *spos, *acc, *glob;
     int nstar, npad, nacc, gsplit;
+    int accf;             // acc holds FP32 pairs (hi, lo), float2, instead of doubles (the packed sweep)
     int pn1;              // 1PN terms on (pair sweep in MODE_FORCE)
     double eps, eps2, inv_c2, dt, inv_eps;
     double *a;            // output acceleration (may be null), [p*asp + k*ask]
@@ -71,6 +72,7 @@ struct EnergyArgs {
     long long sp, sk;
     const double *spos, *acc, *glob;
     int nstar, npad, gsplit;
+    int accf;              // as in FinishArgs
     int nacc, sphi, spsi;  // pair-sum layout: slots per split and the Phi, Psi slots
     double eps, eps2, inv_c2, inv_eps;
     double *part, *out;  // out[4] = pot_n, kin_n, pot_pn, total

@@ -175,7 +175,8 @@ constexpr int pair2_min_blocks() {
 
 // One work item of the paired sweep: the i-block at ibase (128 * IPT stars) against j-range
 // `split`.  As pair_block (pn_pair.cuh): TMA double-buffered tiles, bounded waits, per-i Kahan
-// folding of each tile's sums, FP64 partial sums out.  a.pack is the paired pack, a.ipack the
+// folding of each tile's sums; the partial sums go out as FP32 pairs (sum, -compensation), Phi unscaled,
+// with the fused energy as FP64.  a.pack is the paired pack, a.ipack the
 // i-side float4 (v.xyz, qe) array.
 template <int MODE, int IPT>
 __device__ __forceinline__ bool pair2_block(const PairArgs &a, int ibase, int split, uint64_t *bars,
@@ -204,9 +205,9 @@ __device__ __forceinline__ bool pair2_block(const PairArgs &a, int ibase, int sp
         const double sx = valid ? a.spos[i] : 0.0;
         const double sy = valid ? a.spos[a.npad + i] : 0.0;
         const double sz = valid ? a.spos[2 * a.npad + i] : 0.0;
-        shx[k] = (float)sx; slx[k] = (float)(sx - (double)shx[k]);
-        shy[k] = (float)sy; sly[k] = (float)(sy - (double)shy[k]);
-        shz[k] = (float)sz; slz[k] = (float)(sz - (double)shz[k]);
+        to_f32_pair(sx, shx[k], slx[k]);
+        to_f32_pair(sy, shy[k], sly[k]);
+        to_f32_pair(sz, shz[k], slz[k]);
         float vx = 0.f, vy = 0.f, vz = 0.f, qe = 0.f;
         if (MODE != MODE_NEWTON && valid) {
             const float4 g = a.ipack[i];
@@ -325,17 +326,22 @@ __device__ __forceinline__ bool pair2_block(const PairArgs &a, int ibase, int sp
     for (int k = 0; k < IPT; ++k) {
         const int i = ibase + tid + k * NT;
         if (i < a.nstar) {
-            double val[NACC];
-#pragma unroll
-            for (int q = 0; q < NACC; ++q)
-                val[q] = ((double)ksum(q, k) - (double)kcmp(q, k)) * (q == Mode2<MODE>::PHI ? X2_K * X2_K : 1.0);
             if constexpr (MODE == MODE_FORCE_ENERGY) {
+                double val[NACC];
+#pragma unroll
+                for (int q = 0; q < NACC; ++q)
+                    val[q] = ((double)ksum(q, k) - (double)kcmp(q, k)) * (q == Mode2<MODE>::PHI ? X2_K * X2_K : 1.0);
                 float nvi2, u;
                 f2_unpack(I[k].nvi2, nvi2, u);
                 val[A_PSI] = 0.25 * val[A_PSI] - 1.75 * (double)nvi2 * val[A_PHI];
-            }
 #pragma unroll
-            for (int q = 0; q < NACC; ++q) a.out[((size_t)split * NACC + q) * a.npad + i] = val[q];
+                for (int q = 0; q < NACC; ++q) a.out[((size_t)split * NACC + q) * a.npad + i] = val[q];
+            } else {  // as FP32 pairs: an FP64 conversion costs 64 cycles of a warp, 4 per sum here
+                float2 *out = reinterpret_cast<float2 *>(a.out);
+#pragma unroll
+                for (int q = 0; q < NACC; ++q)
+                    out[((size_t)split * NACC + q) * a.npad + i] = make_float2(ksum(q, k), -kcmp(q, k));
+            }
         }
     }
     seq += (uint32_t)(t1 - t0 > 0 ? t1 - t0 : 0);
