@@ -8,6 +8,7 @@
 // An integration step (Limit-sticky9.c:844-893) is three evaluations whose k_finish performs
 // stage 1, 2 and 3 (the last one also the state-averaging combine); it is captured once in a
 // CUDA graph and replayed.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -146,6 +147,19 @@ static void choose_packed(PairCfg *k, int nstar, int sms) {
     }
 }
 
+// Tiles per CTA of the sweep over unordered pairs: about 6 CTAs per resident one (2 per SM), so that the last
+// ones end together, but no more CTAs than are resident while every tile has its own, and 8 tiles at
+// most, where the sums written per CTA are 4 % of the traffic that L2 takes.  Measured, N = 6,000:
+// 1 tile 70 us, 2 tiles 117; 16,384: 1, 2, 4, 8 tiles 387, 365, 410, 416; 32,768: 1.47, 1.40, 1.39, 1.38 ms.
+static void choose_sym(PairCfg *k, int nstar, int sms) {
+    const long long nt = (nstar + 127) / 128, nb = (nt + 3) / 4, units = nb * nt - 2 * nb * (nb - 1);
+    k->ipt = 4;
+    k->js = 1;
+    k->tj = 128;
+    k->x2 = 4;
+    k->gsplit = units <= 2 * sms ? 1 : (int)std::min<long long>(8, std::max<long long>(2, (units + 12 * sms - 1) / (12 * sms)));
+}
+
 // Launch shape of the pair sweep: explicit parameters win; otherwise a heuristic sized for
 // GB300 (152 SMs): enough CTAs for several waves, split along j when there are few i-blocks.
 static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
@@ -171,14 +185,17 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
     const bool x2_ok = f32 && k.js == 1 && k.ipt <= 2;
     const int pv = c->p.pair_variant;
     PairCfg tuned;
+    FixUnits fu;
+    const bool fix = !f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, &fu);
+    // (an FP64 shape tuned for the other of its two sweeps does not apply: 3.5 to 4.5 times slower, or
+    // outside the fixed-point one's range)
     if (!explicit_shape && pv == PN_PAIR_AUTO && nstar > 0 &&
-        tune_lookup(c->p.precision, mode, nstar, &tuned)) {
+        tune_lookup(c->p.precision, mode, nstar, &tuned) && (f32 || (tuned.x2 == 1) == fix)) {
         const int ntiles_t = (nstar + tuned.tj - 1) / tuned.tj;
         if (tuned.gsplit > ntiles_t) tuned.gsplit = ntiles_t;
         return tuned;
     }
-    FixUnits fu;
-    if (!f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, &fu)) {
+    if (fix) {
         choose_fix(&k, nstar, c->sms);
         return k;
     }
@@ -188,6 +205,13 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
         const bool occ = k.ipt == 2 && mode_has_force(mode);
         k.x2 = (occ && pv == PN_PAIR_F32X2_OCC3) ? 2 : (occ && pv == PN_PAIR_F32X2_OCC4) ? 3 : 1;
     } else if (pv == PN_PAIR_AUTO && f32 && !explicit_shape && nstar > 0) {
+        // every pair once from N = 8,000 on (below, its CTAs of 512 stars leave SMs idle): measured against
+        // the packed sweep, N = 4,096 66 against 42 us, 8,192 118 / 132, 12,000 216 / 234, 16,384 365 / 426,
+        // 32,768 1.38 / 1.63 ms, 262,144 84.5 / 101.0 ms
+        if (mode == MODE_FORCE && nstar >= 8000) {
+            choose_sym(&k, nstar, c->sms);
+            return k;
+        }
         choose_packed(&k, nstar, c->sms);
         k.x2 = k.ipt == 2 && mode_has_force(mode) ? 2 : 1;
         return k;
@@ -231,12 +255,31 @@ int pn::ensure_acc(pn_ctx *c, int splits) {
     return PN_OK;
 }
 
+// Room for the partial sums of the sweep over unordered pairs; the packed sweep takes its place where
+// there is none.
+void pn::ensure_sym(pn_ctx *c) {
+    if (!is_f32(c) || c->cfg_force.x2 != 4) return;
+    const size_t need = sym_bytes(c->n - 1, c->cfg_force.gsplit);
+    if (need <= c->sym_have) return;
+    if (c->sym_work) cudaFree(c->sym_work);
+    c->sym_work = nullptr;
+    c->sym_have = 0;
+    c->step_valid = c->timed_valid = false;  // captured steps hold the old buffer
+    if (cudaMalloc(&c->sym_work, need) == cudaSuccess) {
+        c->sym_have = need;
+    } else {
+        cudaGetLastError();
+        c->sym_off = true;
+        c->cfg_force = c->cfg_fused;
+    }
+}
+
 static void free_ctx(pn_ctx *c) {
     if (!c) return;
     free_adjoint(c);
     if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
     if (c->timed_exec) cudaGraphExecDestroy(c->timed_exec);
-    void *bufs[] = {c->state_buf, c->a_aos, c->in_aos, c->spos, c->pack, c->pack2, c->ipack, c->fpack, c->fix_bad, c->torg, c->acc,
+    void *bufs[] = {c->state_buf, c->a_aos, c->in_aos, c->spos, c->pack, c->pack2, c->ipack, c->fpack, c->fix_bad, c->torg, c->acc, c->sym_work,
                     c->part, c->glob, c->eout, c->tickets, c->err};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -357,6 +400,12 @@ void pn::refresh_cfg(pn_ctx *c) {
     const int nstar = c->n - 1;
     c->cfg_force = choose_cfg(c, force_mode(c), nstar);
     c->cfg_energy = choose_cfg(c, MODE_ENERGY, nstar);
+    c->cfg_fused = c->cfg_force;
+    if (is_f32(c) && c->cfg_force.x2 == 4) {
+        choose_packed(&c->cfg_fused, nstar, c->sms);
+        c->cfg_fused.x2 = c->cfg_fused.ipt == 2 ? 2 : 1;
+        if (c->sym_off) c->cfg_force = c->cfg_fused;
+    }
     c->cfg_set = true;
 }
 
@@ -371,8 +420,10 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     const int nstar = n - 1;
     refresh_cfg(c);
     const int mode = with_energy ? (int)MODE_FORCE_ENERGY : force_mode(c);
-    const PairCfg &k = c->cfg_force;
-    int rc = ensure_acc(c, k.gsplit);
+    ensure_sym(c);
+    const PairCfg &k = with_energy ? c->cfg_fused : c->cfg_force;
+    const bool sym = is_f32(c) && k.x2 == 4;
+    int rc = ensure_acc(c, acc_splits(k));
     if (rc) return rc;
     const double eps2 = c->p.eps * c->p.eps;
 
@@ -381,7 +432,10 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     pa.nstar = nstar; pa.npad = c->npad; pa.nfill = (int)round_up(nstar > 0 ? nstar : 1, 256);
     pa.tj = k.tj; pa.f32 = is_f32(c); pa.eps2 = eps2;
     pa.pack = c->pack; pa.torg = c->torg; pa.spos = c->spos;
-    if (pa.f32) {
+    if (sym) {
+        pa.pack = nullptr;
+        pa.spack = static_cast<float4 *>(c->pack);
+    } else if (pa.f32) {
         pa.pack2 = c->pack2;
         pa.ipack = c->ipack;
         if (k.x2) pa.pack = nullptr;  // the packed sweep reads the paired pack only
@@ -407,7 +461,8 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     }
     if (tslot >= 0) CU(cudaEventRecordWithFlags(c->evp[2 * tslot], s, cudaEventRecordExternal));
     if (nstar > 0) {
-        if (is_f32(c)) CU(launch_pair_f32(mode, k, qa, s));
+        if (sym) CU(launch_pair_sym(k, qa, c->sym_work, s));
+        else if (is_f32(c)) CU(launch_pair_f32(mode, k, qa, s));
         else if (k.x2) CU(launch_pair_fix(mode, k, qa, s));
         else CU(launch_pair_f64(mode, k, qa, s));
     }
@@ -428,7 +483,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     FinishArgs fa{};
     fa.v = v; fa.m = m; fa.vsp = sp; fa.vsk = sk;
     fa.spos = c->spos; fa.acc = c->acc; fa.glob = c->glob;
-    fa.nstar = nstar; fa.npad = c->npad; fa.nacc = pair_nacc(mode); fa.gsplit = k.gsplit;
+    fa.nstar = nstar; fa.npad = c->npad; fa.nacc = pair_nacc(mode); fa.gsplit = acc_splits(k);
     fa.accf = is_f32(c) && k.x2 && !with_energy;
     fa.pn1 = mode_has_force(mode) && c->p.inv_c2 != 0.0;
     fa.eps = c->p.eps; fa.eps2 = eps2; fa.inv_c2 = c->p.inv_c2; fa.dt = c->p.dt; fa.inv_eps = 1.0 / c->p.eps;
@@ -439,8 +494,9 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     CU(launch_finish(fa, s));
     if (timed) CU(cudaEventRecord(c->ev2, s));
     c->stats.tile_j = k.tj; c->stats.i_per_thread = k.ipt; c->stats.j_split = k.js;
-    c->stats.grid_split = k.gsplit; c->stats.threads = PAIR_NT;
-    c->stats.pair_variant = k.x2 == 3   ? PN_PAIR_F32X2_OCC4
+    c->stats.grid_split = sym ? sym_panels(nstar, k.gsplit) : k.gsplit; c->stats.threads = PAIR_NT;
+    c->stats.pair_variant = sym         ? PN_PAIR_F32X2_SYM
+                            : k.x2 == 3   ? PN_PAIR_F32X2_OCC4
                             : k.x2 == 2 ? PN_PAIR_F32X2_OCC3
                             : k.x2      ? PN_PAIR_F32X2
                                         : PN_PAIR_SCALAR;
@@ -568,7 +624,8 @@ static int build_step_graph(pn_ctx *c, bool timed = false) {
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     refresh_cfg(c);
     // allocate before capture, for the energy sweep too (a later allocation would make the step stale)
-    int rc = ensure_acc(c, c->cfg_force.gsplit > c->cfg_energy.gsplit ? c->cfg_force.gsplit : c->cfg_energy.gsplit);
+    ensure_sym(c);
+    int rc = ensure_acc(c, std::max({acc_splits(c->cfg_force), c->cfg_energy.gsplit, c->cfg_fused.gsplit}));
     if (rc) return rc;
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -746,8 +803,8 @@ extern "C" int pn_load_checkpoint(pn_ctx *c, const char *path, double *eouttime,
     return PN_OK;
 }
 
-static int eval_energy(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,
-                       long long sk, pn_energy_t *e) {
+static int enqueue_energy(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,
+                          long long sk) {
     const int nstar = c->n - 1;
     refresh_cfg(c);
     const PairCfg &k = c->cfg_energy;
@@ -785,7 +842,13 @@ static int eval_energy(pn_ctx *c, const double *x, const double *v, const double
     ea.part = c->part + on_blocks(c->npad) * 8;
     ea.out = c->eout; ea.ticket = &c->tickets[2]; ea.fix_bad = pa.fix_bad;
     CU(launch_energy_finish(ea, s));
-    return read_energy(c, e);
+    return PN_OK;
+}
+
+static int eval_energy(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,
+                       long long sk, pn_energy_t *e) {
+    const int rc = enqueue_energy(c, x, v, m, sp, sk);
+    return rc ? rc : read_energy(c, e);
 }
 
 extern "C" int pn_energy(pn_ctx *c, pn_energy_t *e) {
@@ -1008,6 +1071,8 @@ extern "C" int pn_bench_steps(pn_ctx *c, int nsteps, int flush_l2, double *step_
 // rsqrt as 1 and every other add/multiply as 1 (the operations written in pn_device.cuh).
 extern "C" double pn_flops_per_pair(int mode, int precision, int pair_variant) {
     const bool f32 = precision == PN_PREC_MIXED;
+    // every pair once: 75 FP32 operations of which 42 FMA, and the MUFU, for two interactions
+    if (f32 && pair_variant == PN_PAIR_F32X2_SYM && mode == MODE_FORCE) return 59.0;
     if (f32 && pair_variant >= PN_PAIR_F32X2 && pair_variant <= PN_PAIR_F32X2_OCC4) {
         // the packed sweep (operands pre-scaled): FORCE 50 FP32 operations of which 24 FMA,
         // NEWTON 22 (7 FMA), ENERGY 32 (12 FMA); FMA = 2 flops, the MUFU rsqrt = 1
@@ -1130,62 +1195,33 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
     if (!c || !c->have_state) return set_err(PN_ERR_STATE, "pn_autotune: no state");
     const int nstar = c->n - 1;
     if (nstar < 1) return PN_OK;
-    int sms = 0;
-    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
+    refresh_cfg(c);
     const bool f32 = is_f32(c);
-    const double eps2 = c->p.eps * c->p.eps;
+    FixUnits fu;
+    const bool fix = !f32 && fix_units(c->p.eps, &fu);
     const int modes[2] = {force_mode(c), MODE_ENERGY};
     for (int which = 0; which < 2; ++which) {
         if (!(sweeps & (1 << which))) continue;
         const int mode = modes[which];
-        std::vector<PairCfg> cands = tune_candidates(f32, mode, nstar, sms);
+        std::vector<PairCfg> cands = tune_candidates(f32, fix, mode, nstar);
         PairCfg best{};
         float best_t = 1e30f;
         for (const PairCfg &k : cands) {
-            int rc = ensure_acc(c, k.gsplit);
-            if (rc) return rc;
-            PrepArgs pa{};
-            pa.x = c->st.x; pa.v = c->st.v; pa.m = c->st.m; pa.sp = 1; pa.sk = c->ld;
-            pa.nstar = nstar; pa.npad = c->npad; pa.nfill = (int)round_up(nstar, 256);
-            pa.tj = k.tj; pa.f32 = f32; pa.eps2 = eps2;
-            pa.pack = c->pack; pa.torg = c->torg; pa.spos = c->spos;
-    if (pa.f32) { pa.pack2 = c->pack2; pa.ipack = c->ipack; }
-            pa.part = c->part; pa.glob = c->glob; pa.ticket = &c->tickets[0];
-            CU(launch_prep(pa, c->stream));
-            PairArgs qa{};
-            qa.pack = c->pack; qa.torg = c->torg; qa.spos = c->spos; qa.pack2 = c->pack2; qa.ipack = c->ipack; qa.out = c->acc; qa.err = c->err;
-            qa.nstar = nstar; qa.npad = c->npad; qa.tj = k.tj; qa.ntiles = (nstar + k.tj - 1) / k.tj;
-            qa.gsplit = k.gsplit; qa.eps2 = eps2;
+            // a whole evaluation (prep, pair sweep, finish), so that the finishing kernel's reads of the
+            // j-range partial sums (72 B per star and split) count against the shapes with many splits
+            (which == 0 ? c->cfg_force : c->cfg_energy) = k;
+            c->cfg_set = true;
             float t = 1e30f;
-            if (which == 0) {
-                // the force sweep: time the whole evaluation (prep, pair sweep, finish), so that
-                // the finishing kernel's reads of the j-range partial sums (72 B per star and
-                // split) count against the shapes with many splits
-                c->cfg_force = k;
-                c->cfg_energy = k;
-                c->cfg_set = true;
-                for (int rep = 0; rep < 3; ++rep) {  // first evaluation warms up; best of two
-                    CU(cudaEventRecord(c->ev0, c->stream));
-                    rc = eval_force(c, c->st.x, c->st.v, c->st.m, 1, c->ld, nullptr, 3, 1, 0, c->stream, false);
-                    if (rc) return rc;
-                    CU(cudaEventRecord(c->ev1, c->stream));
-                    CU(cudaEventSynchronize(c->ev1));
-                    float ms = 0.f;
-                    CU(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-                    if (rep > 0 && ms < t) t = ms;
-                }
-            } else {
-                for (int rep = 0; rep < 2; ++rep) {  // first launch warms up
-                    CU(cudaEventRecord(c->ev0, c->stream));
-                    cudaError_t e = f32 ? launch_pair_f32(mode, k, qa, c->stream)
-                                        : launch_pair_f64(mode, k, qa, c->stream);
-                    if (e != cudaSuccess) return set_err(PN_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
-                    CU(cudaEventRecord(c->ev1, c->stream));
-                    CU(cudaEventSynchronize(c->ev1));
-                    float ms = 0.f;
-                    CU(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-                    if (rep > 0) t = ms;
-                }
+            for (int rep = 0; rep < 3; ++rep) {  // first evaluation warms up; best of two
+                CU(cudaEventRecord(c->ev0, c->stream));
+                int rc = which == 0 ? eval_force(c, c->st.x, c->st.v, c->st.m, 1, c->ld, nullptr, 3, 1, 0, c->stream, false)
+                                    : enqueue_energy(c, c->st.x, c->st.v, c->st.m, 1, c->ld);
+                if (rc) return rc;
+                CU(cudaEventRecord(c->ev1, c->stream));
+                CU(cudaEventSynchronize(c->ev1));
+                float ms = 0.f;
+                CU(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+                if (rep > 0 && ms < t) t = ms;
             }
             if (getenv("PN_TUNE_VERBOSE"))
                 fprintf(stderr, "pn_autotune mode %d: ipt %d js %d tj %d gsplit %d x2 %d: %.3f ms\n", mode,

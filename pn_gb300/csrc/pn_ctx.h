@@ -27,6 +27,9 @@ struct pn_ctx {
     uint4 *fpack = nullptr;       // pack of the fixed-point FP64 sweep [FIX_GROUPS][npad]
     int *fix_bad = nullptr;       // raised by k_prep for a system outside that sweep's range
     pn::TileOrigin *torg = nullptr;
+    void *sym_work = nullptr;     // partial sums of the sweep over unordered pairs (on first use)
+    size_t sym_have = 0;
+    bool sym_off = false;         // there was no memory for them
     double *acc = nullptr;
     int acc_splits = 0;
     double *part = nullptr;  // partial sums (prep / finish / energy share one buffer region each)
@@ -47,7 +50,7 @@ struct pn_ctx {
     void *flush = nullptr;        // L2 flush buffer (benchmarks only)
     size_t flush_bytes = 0;
     pn_stats stats{};
-    pn::PairCfg cfg_force{}, cfg_energy{};
+    pn::PairCfg cfg_force{}, cfg_energy{}, cfg_fused{};  // (fused: force and energy in one sweep)
     bool cfg_set = false;
     AdjointWork *adj = nullptr;  // buffers of the adjoint (created on first use)
     // asynchronous snapshots (created on first use): device copy of x, v, its pinned host image,
@@ -66,6 +69,7 @@ bool is_f32(const pn_ctx *c);
 int force_mode(const pn_ctx *c);
 void refresh_cfg(pn_ctx *c);
 int ensure_acc(pn_ctx *c, int splits);
+void ensure_sym(pn_ctx *c);
 int check_device_err(pn_ctx *c);
 // One force evaluation; see pn_api.cu.  sums_out (optional) receives the per-star pair sums.
 int eval_force(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,

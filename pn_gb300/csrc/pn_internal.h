@@ -14,8 +14,13 @@ struct PairCfg {
     int gsplit = 1;  // j-range splits across CTAs
     int x2 = 0;      // FP32: the packed f32x2 sweep (pn_pair2.cuh; js = 1, ipt 1 or 2);
                      // 2 / 3 = the same sized for 3 / 4 CTAs per SM (ipt 2, force sweeps)
+                     // 4 = the sweep over unordered pairs (pn_pairsym.cuh; MODE_FORCE, tj 128,
+                     // gsplit = tiles per CTA)
                      // FP64: 1 = the fixed-point sweep (pn_pairfix.cuh; ipt 1, tj 128)
 };
+
+// j-range splits that the sweep's partial sums have
+inline int acc_splits(const PairCfg &c) { return c.x2 == 4 ? 1 : c.gsplit; }
 
 // Launches k_pair for the given precision/mode/shape (returns cudaErrorInvalidValue for an
 // unsupported (ipt, js) combination).  Implemented in pn_pair_f32.cu / pn_pair_f64.cu.
@@ -28,6 +33,12 @@ constexpr int FIX_GROUPS = 13;  // 16-byte groups per star of its pack
 // Its units for a softening; false where its range does not cover it.
 bool fix_units(double eps, FixUnits *u);
 bool pair_shape_supported(int ipt, int js);
+// The mixed force sweep over unordered pairs (PairCfg::x2 = 4; pn_pair_sym.cu), whose partial sums take
+// sym_bytes of work, at most SYM_PANEL_BYTES (or one panel of 4 tiles).
+constexpr size_t SYM_PANEL_BYTES = (size_t)512 << 20;
+size_t sym_bytes(int nstar, int chunk);
+int sym_panels(int nstar, int chunk);
+cudaError_t launch_pair_sym(const PairCfg &c, const PairArgs &a, void *work, cudaStream_t s);
 
 // Persistent ensemble sweep (k_pair_ens): (ipt, js) in {(1,1), (2,1), (1,4)}; tjmax = the
 // largest tile size among the clusters; grid <= 0 = one wave of resident CTAs.

@@ -222,6 +222,16 @@ __device__ __forceinline__ void prep_body(const PrepArgs &a, int blk, int nblk) 
             pk[2 * a.npad + j] = make_float4(v[0], v[1], v[2], qf);
             pk[3 * a.npad + j] = make_float4(to_f32(c1), c3f, to_f32(k35), 0.f);
         }
+        if (a.spack) {  // scaled as the paired pack
+            constexpr double K = X2_K, IK = 1.0 / K, IK3 = 1.0 / (K * K * K);
+            float4 *p = a.spack + j;
+            const size_t n = a.npad;
+            p[0] = make_float4(hi[0], hi[1], hi[2], to_f32(mj * IK3));
+            p[n] = make_float4(lo[0], lo[1], lo[2], to_f32(mu3 * IK));
+            p[2 * n] = make_float4(to_f32(X2_SQRT3 * vv[0]), to_f32(X2_SQRT3 * vv[1]), to_f32(X2_SQRT3 * vv[2]),
+                                   to_f32(fma(-2.0, v2, c1)));
+            p[3 * n] = make_float4(c3f, to_f32(k35 * IK), qf, 0.f);
+        }
         if (a.pack2) {  // paired layout: star j is lane (j & 1) of pair j / 2; scaled
             const int lane = j & 1;
             const size_t prow = (size_t)a.npad / 2;

@@ -42,6 +42,7 @@ struct PrepArgs {
     unsigned *ticket;
     float4 *pack2;  // optional (FP32): paired pack [7][npad/2] of the f32x2 sweep
     float4 *ipack;  // optional (FP32): [npad] (v.xyz, qe)
+    float4 *spack;  // optional (FP32): pack of the sweep over unordered pairs [4][npad]
     uint4 *fpack;   // optional (FP64): the fixed-point sweep's pack [13][npad], its flag and units
     int *fix_bad;
     FixUnits fu;

@@ -1,13 +1,12 @@
 // pn_tune.cu -- launch-shape autotuner of the pair sweep.
 //
 // A shape is (i per thread, lanes per i-set, j-tile size, j-range splits).  The tuner times a
-// candidate list on real data (CUDA events; the force sweep as a whole evaluation, so that the
-// cost of reading back many j-range partial sums counts, the energy sweep as its pair launch;
-// one warm-up per shape) and keeps the fastest per key (precision, sweep mode, size class =
+// candidate list on real data (CUDA events; whole evaluations, so that the cost of reading back
+// many j-range partial sums counts; one warm-up per shape) and keeps the fastest per key (precision, sweep mode, size class =
 // floor(log2 N)).
 // Results live in a process-wide table; with PN_TUNE_CACHE=<file> they are also read from and
 // appended to a text file ("prec mode class ipt js tj gsplit x2 ms" per line), so a tuned
-// shape is reused by later runs.  x2 = 1 selects the packed f32x2 sweep (pn_pair2.cuh).
+// shape is reused by later runs.  x2: as PairCfg.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -44,10 +43,13 @@ void load_file_locked() {
     Entry e{};
     while (fscanf(f, "%d %d %d %d %d %d %d %d %lf", &e.prec, &e.mode, &e.cls, &e.cfg.ipt, &e.cfg.js,
                   &e.cfg.tj, &e.cfg.gsplit, &e.cfg.x2, &e.ms) == 9) {
-        if (pair_shape_supported(e.cfg.ipt, e.cfg.js) && e.cfg.gsplit >= 1 && e.cfg.gsplit <= 64 &&
+        const bool fix = e.prec == 0 && e.cfg.x2 == 1 && e.cfg.ipt == 1 && e.cfg.tj == 128 && e.cfg.js == 16;
+        if ((pair_shape_supported(e.cfg.ipt, e.cfg.js) || fix) && e.cfg.gsplit >= 1 && e.cfg.gsplit <= 64 &&
             (e.cfg.tj == 32 || e.cfg.tj == 64 || e.cfg.tj == 128 || e.cfg.tj == 256) &&
-            (e.cfg.x2 == 0 || (e.cfg.x2 == 1 && e.cfg.js == 1 && e.cfg.ipt <= 2 && e.prec == 1) ||
-             ((e.cfg.x2 == 2 || e.cfg.x2 == 3) && e.cfg.js == 1 && e.cfg.ipt == 2 && e.prec == 1)))
+            (e.cfg.x2 == 0 || (e.cfg.x2 == 1 && e.prec == 0 && e.cfg.ipt == 1 && e.cfg.tj == 128) ||
+             (e.cfg.x2 == 1 && e.cfg.js == 1 && e.cfg.ipt <= 2 && e.prec == 1) ||
+             ((e.cfg.x2 == 2 || e.cfg.x2 == 3) && e.cfg.js == 1 && e.cfg.ipt == 2 && e.prec == 1) ||
+             (e.cfg.x2 == 4 && e.cfg.js == 1 && e.cfg.ipt == 4 && e.cfg.tj == 128 && e.prec == 1 && e.mode == MODE_FORCE)))
             g_table.push_back(e);
     }
     fclose(f);
@@ -90,10 +92,35 @@ void tune_clear() {
     g_loaded = true;  // do not re-read the file after an explicit clear
 }
 
-std::vector<PairCfg> tune_candidates(bool f32, int mode, int nstar, int sms) {
+std::vector<PairCfg> tune_candidates(bool f32, bool fix, int mode, int nstar) {
+    std::vector<PairCfg> out;
+    if (fix) {  // FP64: the fixed-point sweep wins at every size
+        PairCfg c;
+        c.ipt = 1;
+        c.tj = 128;
+        c.x2 = 1;
+        const int ntiles = (nstar + 127) / 128;
+        for (c.js = 1; c.js <= 16; c.js *= 2)
+            for (int g : {1, 2, 3, 4, 6, 8, 12, 16}) {
+                if (g > ntiles || (nstar >= 65536 && (c.js > 4 || g > 4))) break;
+                c.gsplit = g;
+                out.push_back(c);
+            }
+        return out;
+    }
+    if (f32 && mode == MODE_FORCE && nstar >= 4096) {  // every pair once
+        PairCfg c;
+        c.ipt = 4;
+        c.tj = 128;
+        c.x2 = 4;
+        for (int g : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16}) {
+            if (nstar >= 65536 && g < 4) continue;
+            c.gsplit = g;
+            out.push_back(c);
+        }
+    }
     // Large systems: only the shapes that can win there (several i per thread, long tiles);
     // small systems: every shape, including lanes splitting j within a warp.
-    std::vector<PairCfg> out;
     const bool big = nstar >= 65536;
     const int shapes_big32[][2] = {{1, 1}, {2, 1}, {4, 1}};
     const int shapes_big64[][2] = {{1, 1}, {1, 2}, {1, 4}};  // FP64: lanes splitting j win
@@ -135,7 +162,6 @@ std::vector<PairCfg> tune_candidates(bool f32, int mode, int nstar, int sms) {
             }
         }
     }
-    (void)sms;
     return out;
 }
 
