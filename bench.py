@@ -588,12 +588,15 @@ def headline(args, rank, world, dist):
     pair_launch_ms = float(pair_ms.mean()) / 3.0
     ctx.close()
 
+    # launches per evaluation: k_prep, the pair sweep (with its reduction, per panel, in the sweep that
+    # forms every pair once), k_finish
+    launches = 2 + 2 * st.grid_split if st.pair_variant == 5 else 3
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64",
             "data": "synthetic (seeded Plummer sphere + BH)",
             "config": workload_config(ns, world),
-            "gpu_launches": 9 * args.steps,
+            "gpu_launches": 3 * launches * args.steps,
             "clocks": clk.summary(int(os.environ.get("LOCAL_RANK", "0")))}
     launch_shape = {"tile_j": st.tile_j, "i_per_thread": st.i_per_thread, "j_split": st.j_split,
                     "grid_split": st.grid_split, "threads": st.threads, "pair_variant": st.pair_variant}
@@ -606,7 +609,8 @@ def headline(args, rank, world, dist):
         achieved = pairs * flops_pair / (pair_launch_ms * 1e-3) / 1e12
         kname = {2: "k_pair2<MODE_FORCE> (packed f32x2)",
                  3: "k_pair2<MODE_FORCE> (packed f32x2, 3 CTAs per SM)",
-                 4: "k_pair2<MODE_FORCE> (packed f32x2, 4 CTAs per SM)"}.get(st.pair_variant, "k_pair<float, MODE_FORCE>")
+                 4: "k_pair2<MODE_FORCE> (packed f32x2, 4 CTAs per SM)",
+                 5: "k_pair2_sym (packed f32x2, every pair once; with k_sym_reduce)"}.get(st.pair_variant, "k_pair<float, MODE_FORCE>")
         line["roofline"] = {"bound": "fp32", "kernel": kname,
                             "achieved": achieved, "peak": peak32, "unit": "TFLOP/s",
                             "frac": achieved / peak32, "traffic": None,
@@ -614,7 +618,7 @@ def headline(args, rank, world, dist):
                             "pair_launch_ms": pair_launch_ms,
                             "peak_source": "measured FP32 FMA throughput of this GPU (pn_probe_fma_peak)",
                             "pair_interactions_per_s": pairs / (pair_launch_ms * 1e-3)}
-        if st.pair_variant in (2, 3, 4):
+        if st.pair_variant in (2, 3, 4, 5):
             # the same FMA work issued as packed two-lane instructions, as the packed sweep does:
             # the ceiling of a sweep made only of fma.rn.f32x2
             peak2 = pn.probe_fma_peak(pn.PROBE_F32X2)
@@ -635,11 +639,13 @@ def headline(args, rank, world, dist):
         # the O(N) kernels (k_prep + k_finish with the fused stage update) per evaluation: the
         # step's time outside the three pair sweeps, against the measured HBM copy bandwidth
         on_ms = max(float(step_ms.mean()) - float(pair_ms.mean()), 0.0) / 3.0
-        gs = st.grid_split
+        sym = st.pair_variant == 5
+        gs = 1 if sym else st.grid_split
         # k_prep reads x, v, m (56 B) and writes spos, the paired pack, the i-side pack (96 B; the
-        # scalar pack's 64 B too when the scalar sweep runs); k_finish reads v, m, spos (56 B) and
+        # scalar pack's 64 B too when the scalar sweep runs; 64 B in all for the sweep that forms every
+        # pair once); k_finish reads v, m, spos (56 B) and
         # the j-range partial sums (9 doubles per split), and reads/writes the stage state (168 B)
-        moved = 56 + (96 if st.pair_variant in (2, 3, 4) else 160) + 56 + 72 * gs + 168
+        moved = 56 + (88 if sym else 96 if st.pair_variant in (2, 3, 4) else 160) + 56 + 72 * gs + 168
         algo = 104 + 144                  # BH-star O(N) terms + one stage update, per star
         peak_hbm = _measured_hbm_gbs()
         line["o_n_kernels"] = {"ms_per_evaluation": on_ms, "bytes_per_star_moved": moved,
@@ -663,7 +669,7 @@ def headline(args, rank, world, dist):
     line["e2e"] = {"value": replica_throughput(world, e2e_steps, inter_step, e2e_s), "unit": UNIT,
                    "h2d_bytes_per_step": 3 * (2 * 24 + 8) * n, "d2h_bytes_per_step": 3 * 24 * n,
                    "path": "drop-in force() x3 per step with host arrays + host stage updates"}
-    line["gpu_launches"] += 9 * e2e_steps
+    line["gpu_launches"] += 3 * launches * e2e_steps
 
     if rank == 0 and not args.quick:
         # ---------------- FP64 path on the same workload (one step) and mixed accuracy

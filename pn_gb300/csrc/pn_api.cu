@@ -148,9 +148,10 @@ static void choose_packed(PairCfg *k, int nstar, int sms) {
 }
 
 // Tiles per CTA of the sweep over unordered pairs: about 6 CTAs per resident one (2 per SM), so that the last
-// ones end together, but no more CTAs than are resident while every tile has its own, and 8 tiles at
-// most, where the sums written per CTA are 4 % of the traffic that L2 takes.  Measured, N = 6,000:
-// 1 tile 70 us, 2 tiles 117; 16,384: 1, 2, 4, 8 tiles 387, 365, 410, 416; 32,768: 1.47, 1.40, 1.39, 1.38 ms.
+// ones end together, at most 8 tiles (a CTA's set-up is then a few percent of its time), and one tile
+// where that takes no more CTAs than are resident.  Measured, N = 6,000: 1 tile 70 us, 2 tiles 117;
+// 16,384: 1, 2, 4, 8 tiles 387, 365, 410, 416; 32,768: 1.47, 1.40, 1.39, 1.38 ms; 262,144: 8 and 16
+// tiles 84.5 and 84.6 ms.
 static void choose_sym(PairCfg *k, int nstar, int sms) {
     const long long nt = (nstar + 127) / 128, nb = (nt + 3) / 4, units = nb * nt - 2 * nb * (nb - 1);
     k->ipt = 4;

@@ -1,8 +1,8 @@
 // pn_pairsym.cuh -- the mixed-precision force sweep over unordered pairs.
 //
 // As k_pair2<MODE_FORCE> (pn_pair2.cuh), but each pair of stars is formed once and serves both: their
-// difference, inverse distance and dot products are shared, so an ordered pair costs 38 packed FP32
-// operations instead of 50 (32 for the pair, 22 per star).
+// difference, inverse distance and dot products are shared, so an ordered pair costs 37.5 packed FP32
+// operations instead of 50 (27 for the pair, 24 per star).
 //
 // A CTA of 128 threads holds 512 rows i in registers, four per thread, two to an f32x2 operand, and
 // runs over a range of 128-star tiles j, from the tiles of its own rows on.  In each 32-star part of a
@@ -11,15 +11,24 @@
 // warps' sums of a tile are added in order and written to slot b (the CTA's row block) of star j.  A
 // tile of the CTA's own rows is swept in both orders and gives row sums only.  Row sums are folded per
 // tile with compensation, as in k_pair2, and written per range of tiles; k_sym_reduce adds a star's slots
-// in order.  No atomics: the sums do not depend on scheduling.
+// in order.  No atomics: the sums do not depend on scheduling.  The slots take 36 bytes per star and row
+// block, so the stars j are swept in panels, as wide as a fixed workspace allows.
 //
 // The operands are k_pair2's scaled ones, but both sides hold w = sqrt(3) v: with a = w_i.w_j, P = w_i.d,
 // S = w_j.d (d = x_j - x_i) star i's bracket has 4 a / 3 + S^2 Q'^2 and its ct the factor 4 P / 3 - S;
 // star j's 4 a / 3 + P^2 Q'^2 and, with d reversed, P - 4 S / 3.  The terms -|v|^2 of the brackets and
 // -w sum ct are applied once per tile.
 //
-// Bound by the FP32 FMA pipe.  Four rows per thread, since the shared-memory pipe carries 8 loads
-// and 10 shuffles per step and would be as busy as the FMA pipe with two (168 against 150 cycles).
+// A sum runs over 128 terms at most before it is folded (rows) or 64 in each half of an operand
+// (stars j).  Against FP64 the median error of the accelerations is 0.93 to 0.99 of k_pair2's at its tiles of
+// 256 (N = 8,100 to 32,767, inv_c2 = 1e-6; 0.75 to 0.85 at 1).
+//
+// Bound by the FP32 FMA pipe (71 % active at N = 16,384) and, with two warps per scheduler, by the latency
+// between its instructions.  Per step of a warp that pipe takes 300 cycles, the shared-memory pipe of
+// the SM 144 (16 wavefronts of loads and 20 shuffles for each of four warps): with half the rows it
+// would be the limit.  Measured at N = 65,536: stars as pairs of equal values in shared memory (twice the
+// loads) 6.09 ms, single values 5.71, two steps unrolled 5.47, four 5.50; three CTAs per SM (168 registers,
+// spills) 5.74; k_pair2 6.31.  N = 262,144: 101.0 -> 84.5 ms; 16,384: 426 -> 365 us.
 #pragma once
 
 #include "pn_pair2.cuh"
