@@ -301,12 +301,25 @@ __global__ void __launch_bounds__(256) k_sym_reduce(const Pair2SymArgs a) {
         h = o.x;
         l = o.y;
     }
-#pragma unroll 4
-    for (int c = max(0, 4 * blk - a.p0) / a.chunk; c < nchunk; ++c)
-        pair_add(h, l, a.rows[((size_t)c * SYM2_NS + q) * a.rstride + i]);
+    const int c0 = max(0, 4 * blk - a.p0) / a.chunk;
+    const float2 *rows = a.rows + (size_t)q * a.rstride + i;
+    const size_t rs = (size_t)SYM2_NS * a.rstride, cs = (size_t)SYM2_NS * a.cstride;
+    for (int c = c0; c < nchunk; c += 16) {  // (16 loads in flight; adding zeros changes nothing)
+        float2 t[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) t[u] = c + u < nchunk ? rows[(c + u) * rs] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) pair_add(h, l, t[u]);
+    }
     if (j >= 0) {
-#pragma unroll 8
-        for (int b = 0; b < blk; ++b) pair_add(h, l, make_float2(a.cols[((size_t)b * SYM2_NS + q) * a.cstride + j], 0.f));
+        const float *cols = a.cols + (size_t)q * a.cstride + j;
+        for (int b = 0; b < blk; b += 16) {
+            float t[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) t[u] = b + u < blk ? cols[(b + u) * cs] : 0.f;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) pair_add(h, l, make_float2(t[u], 0.f));
+        }
     }
     *out = make_float2(h, l);
 }
