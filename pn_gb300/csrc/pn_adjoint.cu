@@ -30,6 +30,7 @@
 
 #include "pn_ctx.h"
 #include "pn_finish_vjp_gen.cuh"
+#include "pn_pair2.cuh"
 
 using namespace pn;
 
@@ -171,6 +172,37 @@ struct PairVjpArgs {
     double eps2;
 };
 
+// Two FP32 values in one register pair, as a number: the same sums for two rows at once with packed
+// instructions (pn_pair2.cuh).
+struct F2v {
+    f2 v;
+    F2v() = default;
+    __device__ __forceinline__ explicit F2v(float c) : v(f2_bcast(c)) {}
+    __device__ __forceinline__ F2v(float lo, float hi) : v(f2_pack(lo, hi)) {}
+};
+__device__ __forceinline__ F2v raw2(f2 v) {
+    F2v r;
+    r.v = v;
+    return r;
+}
+__device__ __forceinline__ F2v operator+(F2v a, F2v b) { return raw2(add2(a.v, b.v)); }
+__device__ __forceinline__ F2v operator-(F2v a, F2v b) { return raw2(sub2(a.v, b.v)); }
+__device__ __forceinline__ F2v operator*(F2v a, F2v b) { return raw2(mul2(a.v, b.v)); }
+__device__ __forceinline__ F2v operator-(F2v a) { return raw2(a.v ^ 0x8000000080000000ull); }
+__device__ __forceinline__ void operator+=(F2v &a, F2v b) { a = a + b; }
+template <> __device__ __forceinline__ F2v pn_fma<F2v>(F2v a, F2v b, F2v c) { return raw2(fma2(a.v, b.v, c.v)); }
+template <> __device__ __forceinline__ F2v pn_rsqrt<F2v>(F2v x) { return raw2(rsqrt2(x.v, 1.f)); }
+
+// Zeroes the value of a self pair; bit r of self: row r.
+template <typename T> __device__ __forceinline__ void skip_self(T &Q, int self) {
+    if (self) Q = T(0);
+}
+__device__ __forceinline__ void skip_self(F2v &Q, int self) {
+    float lo, hi;
+    f2_unpack(Q.v, lo, hi);
+    Q = F2v(self & 1 ? 0.f : lo, self & 2 ? 0.f : hi);
+}
+
 template <typename T> struct VjpState {
     T ex, ey, ez, lx, ly, lz;  // position (FP32: hi/lo relative to the tile origin)
     T vx, vy, vz, m, mu3, c3, k35, qe;
@@ -219,11 +251,11 @@ template <typename T> struct VjpTerms {
 
 template <typename T>
 __device__ __forceinline__ VjpTerms<T> vjp_terms(const VjpState<T> &P, const VjpState<T> &Qj, T dx, T dy, T dz,
-                                                 T eps2, bool self) {
+                                                 T eps2, int self) {
     VjpTerms<T> r;
     const T rhoe = pn_fma(dz, dz, pn_fma(dy, dy, pn_fma(dx, dx, eps2)));
     T Q = pn_rsqrt<T>(rhoe);
-    if (self) Q = T(0);
+    skip_self(Q, self);
     const T Q2 = Q * Q, Q3 = Q2 * Q;
     const T vdp = pn_fma(P.vz, dz, pn_fma(P.vy, dy, P.vx * dx));     // v_p . d
     const T vdq = pn_fma(Qj.vz, dz, pn_fma(Qj.vy, dy, Qj.vx * dx));  // v_q . d
@@ -516,11 +548,28 @@ __global__ void __launch_bounds__(VJP_NT) k_pair_vjp(const PairVjpArgs a) {
 // skipped (its mu3 term is added per row, as in the ordered sweep).
 constexpr int SYM_T = 128;
 
-// Rows per lane: FP32 lanes hold two rows p against the same q (the q data read from shared
-// memory and the 17 shuffles of q's sums then serve two pairs), FP64 lanes one (register-bound).
+// Rows per lane: FP32 lanes hold two rows p against the same q, one in each half of packed operands
+// (one instruction then serves two pairs, which leaves issue slots for the loads of q's data and
+// the shuffles of its sums), FP64 lanes one (register-bound).  Bound by the FP32 FMA pipe (188 cycles
+// of the 268 that an unordered pair of a warp takes) and instruction latency.  Measured at
+// N = 16,384: two rows as scalars, 6 CTAs per SM 953 us; packed, 4 CTAs (212 registers) 917, two
+// steps unrolled 894; packed, 6 CTAs (spills) 1,033.
 template <typename T> __host__ __device__ constexpr int sym_rows() { return sizeof(T) == 4 ? 2 : 1; }
+template <typename T> struct SymLane { using E = T; };
+template <> struct SymLane<float> { using E = F2v; };
+
+__device__ __forceinline__ void vjp_pack(VjpState<F2v> &s, const VjpState<float> &a, const VjpState<float> &b) {
+    s.ex = F2v(a.ex, b.ex); s.ey = F2v(a.ey, b.ey); s.ez = F2v(a.ez, b.ez);
+    s.lx = F2v(a.lx, b.lx); s.ly = F2v(a.ly, b.ly); s.lz = F2v(a.lz, b.lz);
+    s.vx = F2v(a.vx, b.vx); s.vy = F2v(a.vy, b.vy); s.vz = F2v(a.vz, b.vz);
+    s.m = F2v(a.m, b.m); s.mu3 = F2v(a.mu3, b.mu3); s.c3 = F2v(a.c3, b.c3); s.k35 = F2v(a.k35, b.k35);
+    s.qe = F2v(a.qe, b.qe); s.nvi2 = F2v(a.nvi2, b.nvi2); s.c1v = F2v(a.c1v, b.c1v);
+    s.Gx = F2v(a.Gx, b.Gx); s.Gy = F2v(a.Gy, b.Gy); s.Gz = F2v(a.Gz, b.Gz);
+    s.Phi = F2v(a.Phi, b.Phi); s.S0 = F2v(a.S0, b.S0); s.U = F2v(a.U, b.U);
+    s.Wx = F2v(a.Wx, b.Wx); s.Wy = F2v(a.Wy, b.Wy); s.Wz = F2v(a.Wz, b.Wz); s.cW = F2v(a.cW, b.cW);
+}
 template <typename T> __host__ __device__ constexpr int sym_threads() { return SYM_T / sym_rows<T>(); }
-template <typename T> __host__ __device__ constexpr int sym_min_blocks() { return sizeof(T) == 4 ? 6 : 2; }
+template <typename T> __host__ __device__ constexpr int sym_min_blocks() { return sizeof(T) == 4 ? 4 : 2; }
 
 template <typename T>
 constexpr size_t sym_smem_bytes() {
@@ -535,6 +584,7 @@ __global__ void __launch_bounds__(sym_threads<T>(), (sym_min_blocks<T>()))
     constexpr int NGF = VjpPack<T>::NGF, NGA = VjpPack<T>::NGA;
     constexpr int R = sym_rows<T>(), NTH = sym_threads<T>(), NW = NTH / 32;
     constexpr bool F32 = sizeof(T) == 4;
+    using E = typename SymLane<T>::E;
     extern __shared__ __align__(128) unsigned char smem[];
     V *qd = reinterpret_cast<V *>(smem);                                          // [NGF + NGA][SYM_T]
     T *qp = reinterpret_cast<T *>(smem + (size_t)(NGF + NGA) * SYM_T * sizeof(V));  // [NW][NY][SYM_T]
@@ -556,57 +606,66 @@ __global__ void __launch_bounds__(sym_threads<T>(), (sym_min_blocks<T>()))
         for (int g = 0; g < NGA; ++g) qd[(NGF + g) * SYM_T + e] = pa[(size_t)g * a.npad + q0 + e];
     }
     // lane's rows: local star 32 (R warp + r) + lane of tile I
-    VjpState<T> P[R];
-    T y[R][NY];
+    VjpState<E> P;
+    if constexpr (F32) {  // p relative to tile J's origin, as an FP32 hi/lo pair
+        VjpState<float> row[2];
+        const TileOrigin o = a.torg[J];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int p = I * SYM_T + 32 * (R * warp + r) + lane;
-        vjp_load<T>(P[r], pf, pa, a.npad, p);
-        if constexpr (F32) {  // p relative to tile J's origin, as an FP32 hi/lo pair
-            const TileOrigin o = a.torg[J];
+        for (int r = 0; r < 2; ++r) {
+            const int p = I * SYM_T + 32 * (2 * warp + r) + lane;
+            vjp_load<float>(row[r], pf, pa, a.npad, p);
             const double rx = a.spos[p] - o.x, ry = a.spos[a.npad + p] - o.y, rz = a.spos[2 * a.npad + p] - o.z;
-            P[r].ex = (float)rx; P[r].ey = (float)ry; P[r].ez = (float)rz;
-            P[r].lx = (float)(rx - (double)P[r].ex);
-            P[r].ly = (float)(ry - (double)P[r].ey);
-            P[r].lz = (float)(rz - (double)P[r].ez);
+            to_f32_pair(rx, row[r].ex, row[r].lx);
+            to_f32_pair(ry, row[r].ey, row[r].ly);
+            to_f32_pair(rz, row[r].ez, row[r].lz);
         }
-#pragma unroll
-        for (int c = 0; c < NY; ++c) y[r][c] = T(0);
+        vjp_pack(P, row[0], row[1]);
+    } else {
+        vjp_load<T>(P, pf, pa, a.npad, I * SYM_T + 32 * warp + lane);
     }
+    E y[NY], z[NY];
+#pragma unroll
+    for (int c = 0; c < NY; ++c) y[c] = E(0);
     __syncthreads();
-    const T eps2 = (T)a.eps2;
+    const E eps2 = E(a.eps2);
     const V *qa = qd + NGF * SYM_T;
     const int from = (lane + 1) & 31;
-    T z[NY];
     for (int k = 0; k < SYM_T / 32; ++k) {
 #pragma unroll
-        for (int c = 0; c < NY; ++c) z[c] = T(0);
-#pragma unroll 1
+        for (int c = 0; c < NY; ++c) z[c] = E(0);
+        const int self = !diag ? 0 : k == R * warp ? 1 : k == R * warp + R - 1 ? 2 : 0;
+#pragma unroll 2
         for (int st = 0; st < 32; ++st) {
             const int qi = k * 32 + ((lane + st) & 31);
-            VjpState<T> Qj;
-            vjp_load<T>(Qj, qd, qa, SYM_T, qi);
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                T dx, dy, dz;
-                if constexpr (F32) {
-                    dx = (Qj.ex - P[r].ex) + (Qj.lx - P[r].lx);
-                    dy = (Qj.ey - P[r].ey) + (Qj.ly - P[r].ly);
-                    dz = (Qj.ez - P[r].ez) + (Qj.lz - P[r].lz);
-                } else {
-                    dx = Qj.ex - P[r].ex;
-                    dy = Qj.ey - P[r].ey;
-                    dz = Qj.ez - P[r].ez;
-                }
-                const VjpTerms<T> t = vjp_terms<T>(P[r], Qj, dx, dy, dz, eps2, diag && k == R * warp + r && st == 0);
-                vjp_acc_p<T>(y[r], t, Qj, dx, dy, dz);
-                vjp_acc_q<T>(z, t, P[r], dx, dy, dz);
+            VjpState<E> Qj;
+            E dx, dy, dz;
+            if constexpr (F32) {
+                VjpState<float> q;
+                vjp_load<float>(q, qd, qa, SYM_T, qi);
+                vjp_pack(Qj, q, q);
+                dx = (Qj.ex - P.ex) + (Qj.lx - P.lx);
+                dy = (Qj.ey - P.ey) + (Qj.ly - P.ly);
+                dz = (Qj.ez - P.ez) + (Qj.lz - P.lz);
+            } else {
+                vjp_load<T>(Qj, qd, qa, SYM_T, qi);
+                dx = Qj.ex - P.ex;
+                dy = Qj.ey - P.ey;
+                dz = Qj.ez - P.ez;
             }
+            const VjpTerms<E> t = vjp_terms<E>(P, Qj, dx, dy, dz, eps2, st == 0 ? self : 0);
+            vjp_acc_p<E>(y, t, Qj, dx, dy, dz);
+            vjp_acc_q<E>(z, t, P, dx, dy, dz);
 #pragma unroll
-            for (int c = 0; c < NY; ++c) z[c] = __shfl_sync(0xffffffffu, z[c], from);
+            for (int c = 0; c < NY; ++c) {
+                if constexpr (F32) z[c].v = __shfl_sync(0xffffffffu, z[c].v, from);
+                else z[c] = __shfl_sync(0xffffffffu, z[c], from);
+            }
         }
 #pragma unroll
-        for (int c = 0; c < NY; ++c) qp[(warp * NY + c) * SYM_T + k * 32 + lane] = z[c];
+        for (int c = 0; c < NY; ++c) {
+            if constexpr (F32) qp[(warp * NY + c) * SYM_T + k * 32 + lane] = f2_sum(z[c].v);
+            else qp[(warp * NY + c) * SYM_T + k * 32 + lane] = z[c];
+        }
     }
     __syncthreads();
     // rows q of tile J: the warps' sums added in a fixed order; one thread per star q
@@ -623,6 +682,12 @@ __global__ void __launch_bounds__(sym_threads<T>(), (sym_min_blocks<T>()))
         }
     }
     if (diag) __syncthreads();  // uniform over the CTA
+    T row[R][NY];
+#pragma unroll
+    for (int c = 0; c < NY; ++c) {
+        if constexpr (F32) f2_unpack(y[c].v, row[0][c], row[1][c]);
+        else row[0][c] = y[c];
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int pl = 32 * (R * warp + r) + lane;
@@ -630,9 +695,9 @@ __global__ void __launch_bounds__(sym_threads<T>(), (sym_min_blocks<T>()))
 #pragma unroll
         for (int c = 0; c < NY; ++c) {
             if (diag)  // every pair of the tile was visited in both orders: half of each
-                part[((size_t)I * NY + c) * a.npad + p] = T(0.5) * (y[r][c] + qp[c * SYM_T + pl]);
+                part[((size_t)I * NY + c) * a.npad + p] = T(0.5) * (row[r][c] + qp[c * SYM_T + pl]);
             else
-                part[((size_t)J * NY + c) * a.npad + p] = y[r][c];  // row p, its pairs with tile J
+                part[((size_t)J * NY + c) * a.npad + p] = row[r][c];  // row p, its pairs with tile J
         }
     }
 }

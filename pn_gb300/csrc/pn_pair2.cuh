@@ -68,18 +68,18 @@ __device__ __forceinline__ void lds2(const void *p, f2 &a, f2 &b) {
 }
 // K times the inverse square root of both lanes: MUFU rsqrt each, refined by one Newton-Raphson
 // step y' = y (1.5 - 0.5 x y^2) whose two constants are scaled by K (exact in FP32).
-__device__ __forceinline__ f2 rsqrt2k(f2 x) {
+__device__ __forceinline__ f2 rsqrt2(f2 x, float K) {
     float a, b;
     f2_unpack(x, a, b);
     float ya, yb;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
     const f2 y = f2_pack(ya, yb);
-    constexpr float K = (float)X2_K;
     const f2 nxh = mul2(x, f2_bcast(-0.5f * K));
     const f2 r = fma2(nxh, mul2(y, y), f2_bcast(1.5f * K));
     return mul2(y, r);
 }
+__device__ __forceinline__ f2 rsqrt2k(f2 x) { return rsqrt2(x, (float)X2_K); }
 __device__ __forceinline__ float f2_sum(f2 v) {
     float a, b;
     f2_unpack(v, a, b);
