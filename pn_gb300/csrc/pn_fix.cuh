@@ -19,9 +19,9 @@
 //   n   = d Q, S = 60, the softened unit vector
 // and the terms of pn_device.cuh's sums, with w_j = sqrt(3) v_j, u_i = (4 / sqrt(3)) v_i:
 //   G   += (m Q^2) n         S0 += (m Q^2) Q
-//   W   += (m Q^2 F) n + ct w,   F = u.w + (w.n)^2 / 2,  ct = m Q^2 (u.n - w.n)
-//   W64 += [(g1 - g3 qe_i) Q^2 + k] n,  g1 = m (c1 - 2 |v|^2), g3 = m c3, k = g3 + k35
-//          (its coefficient, which spans the range of R_j^3, in FP64; c3 rho Q^2 = c3 is in k)
+//   W   += (H + C) n + ct w,   H = m Q^2 F,  F = u.w + (w.n)^2 / 2,  ct = m Q^2 (u.n - w.n),
+//          C = (g1 - g3 qe_i) Q^2 + k,  g1 = m (c1 - 2 |v|^2), g3 = m c3, k = g3 + k35
+//          (C, which spans the range of R_j^3, is formed in FP64; c3 rho Q^2 = c3 is in k)
 //   Phi += m Q,  U += mu3 Q  (FP64; in the energy sweep Phi in integers)
 //   Psi += m Q (7 u.w + (u.n)(w.n))  (four times the energy's)
 // The small (cross) parts of the dot products u.w, u.n, w.n are FP32: their rounding, 2^-54 of the
@@ -237,10 +237,12 @@ struct StarJ {
     int em;             // its exponent (in the units above)
     B2 wx, wy, wz;      // w_j, S = 60
     double m, mu3;      // m and mu3 = m R^3, in the system's units
-    double g1, g3, k;   // the coefficients of W64, in the system's units
+    double g1, g3, k;   // the coefficients of C, in the system's units
 };
 struct Scale {
-    int g, c;  // the tile's sums: m Q^2 < 2^g (or m Q, energy), |W64's coefficient| < 2^c (the system's units)
+    int g;     // the tile's sums: m Q^2 < 2^g (or m Q, energy)
+    int c;     // ... |C + H| < 2^c (the system's units): c one above the larger of C's and H's exponents
+    int rh;    // right shift of H from its own exponent to 2^c
     int q;     // exponent of the system's Q over the units' Q: -eL
     // left shifts of the velocity terms' factors, from S = 60 relative to 2^g to S = 62 relative to the
     // tile's own sums: |m Q^2 F| < 2^(g + 2 - lh + 2 ev), |ct| < 2^(g + 2 - lt + ev); 2^(lh - 32), 2^(lt - 32)
@@ -255,8 +257,7 @@ struct Acci {  // ... all integers
 };
 struct Sums {
     Acci g[3];  // G, S = 122 relative to 2^g
-    Acci c[3];  // W64, S = 122 relative to 2^c
-    Acci w[3];  // W's part along n, S = 122 relative to 2^(g + 2 - lh + 2 ev)
+    Acci c[3];  // W's part along n, S = 122 relative to 2^c
     Acci t[3];  // W's part along w, S = 122 relative to 2^(g + 2 - lt + 2 ev)
     i64 s0;     // S0, S = 60 relative to 2^g
     i64 ct;     // sum of ct, S = 62 relative to 2^(g + 2 - lt + ev)
@@ -268,7 +269,7 @@ struct Sums {
 
 template <int MODE> PNF void clear(Sums &a) {
     for (int k = 0; k < 3; ++k) {
-        a.g[k].h = a.g[k].x = a.c[k].h = a.c[k].x = a.w[k].h = a.w[k].x = a.t[k].h = a.t[k].x = 0;
+        a.g[k].h = a.g[k].x = a.c[k].h = a.c[k].x = a.t[k].h = a.t[k].x = 0;
     }
     a.s0 = a.ct = a.phi = a.psi.h = 0;
     a.psi.x = 0.f;
@@ -294,7 +295,6 @@ template <int MODE> PNF void fold(Sums &a) {
         fold(a.g[k]);
         if (MODE != F_NEWTON) {
             fold(a.c[k]);
-            fold(a.w[k]);
             fold(a.t[k]);
         }
     }
@@ -307,6 +307,11 @@ PNF i64 top(const Acc &a) { return (i64)((u64)a.h << 3) + to_int(a.x * 0x1p-29f)
 // (at most by `most`: beyond that the terms are small beside |v_i|^2 times the tile's sum)
 PNF int lift(int g, int e, int most) { return 2 + (g - e < 0 ? 0 : g - e > most ? most : g - e); }
 constexpr int LIFT_H = 16, LIFT_T = 12;
+// Scale::c and rh from C's exponent and H's own (in the system's units)
+PNF void join(Scale &E, int ec, int eh) {
+    E.c = (ec > eh ? ec : eh) + 1;
+    E.rh = E.c - eh < 63 ? E.c - eh : 63;
+}
 
 PNF double scale_down(double x, int e) {  // x 2^-e, x > 0 and normal, result normal
 #ifdef __CUDA_ARCH__
@@ -401,25 +406,22 @@ PNF void pair(Sums &a, const StarI &I, const StarJ &J, const Scale &E, unsigned 
     const V wv = vec(bal(w));
     // F = u.w + (w.n)^2 / 2, S = 62
     const B2 f = bal(merge<4>(mw(wv.h, 2 * wv.h, (uw.h << 4) >> I.d), fmaf_(4.f * wv.hf, wv.l, (16.f * I.fd) * uw.x), 0x1p-32f));
-    const B2 H = bal((i64)((u64)mw(p.h, f.h, 0) << E.lh) + (cross(p, f, 0) >> (32 - E.lh)));
+    const i64 H = ((i64)((u64)mw(p.h, f.h, 0) << E.lh) + (cross(p, f, 0) >> (32 - E.lh))) >> E.rh;
     const B2 k = bal(b - w);
     const i64 ct = (i64)((u64)mw(p.h, k.h, 0) << E.lt) + (cross(p, k, 0) >> (32 - E.lt));
     a.ct += ct;
     const B2 t = bal(ct);
-    add(a.w[0], H, mx);
-    add(a.w[1], H, my);
-    add(a.w[2], H, mz);
     add(a.t[0], t, J.wx);
     add(a.t[1], t, J.wy);
     add(a.t[2], t, J.wz);
-    // FP64: Phi, U and the coefficient of W64, which then joins the integers
+    // FP64: Phi, U and C, which then joins the integers
     const double qd = scale_down(u2d(Q), 62 + ey - E.q);
     a.dphi = fma_(J.m, qd, a.dphi);
     a.du = fma_(J.mu3, qd, a.du);
     const u64 co = bits_of(fma_(fma_(-I.qe, J.g3, J.g1), qd * qd, J.k));
     const u64 cm = ((co & 0xfffffffffffffULL) | 0x10000000000000ULL) << 9;  // S = 61 of 1.f
     const i64 sg = (i64)co >> 63;
-    const B2 C = bal((i64)(((u64)shr(cm, E.c + 1022 - (int)((co >> 52) & 0x7ff)) ^ (u64)sg) - (u64)sg));  // S = 62
+    const B2 C = bal((i64)(((u64)shr(cm, E.c + 1022 - (int)((co >> 52) & 0x7ff)) ^ (u64)sg) - (u64)sg) + H);  // S = 62
     add(a.c[0], C, mx);
     add(a.c[1], C, my);
     add(a.c[2], C, mz);

@@ -8,14 +8,14 @@
 // for the sums themselves, which are added to FP64 totals in shared memory at the tile's end.
 //
 // Why: FP64 issues one warp instruction per 64 cycles and scheduler here and k_pair<double>'s 51 per
-// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 830, of which the
-// multiply-add pipe is busy 74 % and the FP64 pipe 59 % (6 operations per pair). One force evaluation at
-// N = 65,536: 385 -> 88.5 ms, N = 10,000: 9.3 -> 2.3 ms.  Its error against long double sums is below
-// the FP64 sweep's (medians at N = 2,049: 1.46e-16 against 2.22e-16 at c = 1000, 5.1e-16 against
-// 7.4e-16 at c = 1).  Measured on the way there, at N = 65,536: every product in integers and W64's sum
+// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 725 and is bound by the
+// multiply-add pipe, beside the FP64 pipe's 6 operations per pair. One force evaluation at
+// N = 65,536: 385 -> 77.3 ms, N = 10,000: 9.3 -> 2.0 ms.  Its error against long double sums is below
+// the FP64 sweep's (medians at N = 2,049: 1.46e-16 against 2.22e-16 at c = 1000, 5.2e-16 against
+// 7.4e-16 at c = 1).  Measured on the way there, at N = 65,536: every product in integers and C's sum
 // in FP64 (4 conversions and 5 FMA per pair) 104 ms; the dot products' small parts in FP32, Phi and U in
-// FP64 and W64's sum in integers 88.5 ms; the sums' small parts in FP32 too 76 ms, but with twice the FP64
-// sweep's error at c = 1.
+// FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms; the sums' small parts in FP32
+// too (before that) 76 against 88 ms, but with twice the FP64 sweep's error at c = 1.
 //
 // The integer range covers the systems that k_prep has checked star by star (positions within
 // 2^24 eps, masses zero or 2^-32 .. 2^59 of the BH's, all finite); for any other
@@ -31,8 +31,8 @@ constexpr int FIX_TJ = 128;
 
 template <int MODE> struct FixInfo {
     static constexpr int NG = MODE == MODE_NEWTON ? 5 : MODE == MODE_ENERGY ? 8 : 11;  // streamed 16-byte groups
-    // sums over the tiles in shared memory: G; or G, S0, W along n, W64, ct, W along w, Phi, U (and Psi); or Phi, Psi
-    static constexpr int NT = MODE == MODE_NEWTON ? 3 : MODE == MODE_ENERGY ? 2 : MODE == MODE_FORCE ? 16 : 17;
+    // sums over the tiles in shared memory: G; or G, S0, W along n, ct, W along w, Phi, U (and Psi); or Phi, Psi
+    static constexpr int NT = MODE == MODE_NEWTON ? 3 : MODE == MODE_ENERGY ? 2 : MODE == MODE_FORCE ? 13 : 14;
 };
 
 template <int MODE>
@@ -97,7 +97,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
     }
     const int e0 = fix::expo(a.m[0]), eL = a.fu.eL;
     const int eg = e0 - (MODE == MODE_ENERGY ? 1 : 2) * eL;  // exponents of the units of m Q^2 (m Q)
-    const int ec = 2 * e0 - 3 * eL;                          // ... and of W64's coefficient
+    const int ec = 2 * e0 - 3 * eL;                          // ... and of C
     const float qef = FORCE ? (float)(I.qe * pow2(-2 * eL)) : 0.f;
     // the i position in units of 2^eL as an FP32 pair (for the seeds' differences)
     float sh[3], sl[3];
@@ -202,10 +202,10 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                 }
             }
             E.g = mag_exp(mg);
-            E.c = mag_exp(mc) + ec;
             E.q = -eL;
             E.lh = lift(E.g, mag_exp(mh), LIFT_H);
             E.lt = lift(E.g, mag_exp(mt), LIFT_T);
+            join(E, mag_exp(mc) + ec, E.g + eg + 2 - E.lh + 2 * ev);
         }
         // ---- the sums
         clear<MODE>(A);
@@ -263,17 +263,15 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
             ve[3] = gn - eL - 60;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                v[4 + k] = top(A.w[k]);
-                ve[4 + k] = gn + 2 - E.lh - 62 + 2 * ev;
-                v[11 + k] = top(A.t[k]);
-                ve[11 + k] = gn + 2 - E.lt - 62 + 2 * ev;
-                v[7 + k] = top(A.c[k]);
-                ve[7 + k] = E.c - 62;
+                v[4 + k] = top(A.c[k]);
+                ve[4 + k] = E.c - 62;
+                v[8 + k] = top(A.t[k]);
+                ve[8 + k] = gn + 2 - E.lt - 62 + 2 * ev;
             }
-            v[10] = A.ct;
-            ve[10] = gn + 2 - E.lt - 62 + ev;
+            v[7] = A.ct;
+            ve[7] = gn + 2 - E.lt - 62 + ev;
         }
-        constexpr int NI64 = FORCE ? 14 : FixInfo<MODE>::NT;
+        constexpr int NI64 = FORCE ? 11 : FixInfo<MODE>::NT;
 #pragma unroll
         for (int q = 0; q < NI64; ++q) {
             i64 x = v[q];
@@ -284,11 +282,11 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         if constexpr (FORCE) {
             const double d[3] = {A.dphi, A.du, A.dpsi};
 #pragma unroll
-            for (int q = 0; q < FixInfo<MODE>::NT - 14; ++q) {
+            for (int q = 0; q < FixInfo<MODE>::NT - NI64; ++q) {
                 double x = d[q];
 #pragma unroll
                 for (int off = JS / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-                double &t = tot[(14 + q) * NT + grp];
+                double &t = tot[(NI64 + q) * NT + grp];
                 if (sub == 0) t = q < 2 ? t + x : ::fma(x, pow2(2 * ev - 61), t);
             }
         }
@@ -313,18 +311,18 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
             out(E_PHI, ::fma(mi, a.fu.inv_eps, T(0)));
             out(E_PSI, ::fma(7.0 * vi2, mi * a.fu.inv_eps, T(1)));
         } else {
-            out(A_PHI, T(14));
+            out(A_PHI, T(11));
             out(A_S0, ::fma(mi, a.fu.inv_eps3, T(3)));
-            out(A_U, T(15));
+            out(A_U, T(12));
             // the velocity factors of the star itself: -|v_i|^2 G and -3/4 u_i sum ct = -sqrt(3) v_i sum ct
-            const double cs = -fix::W_SCALE * T(10);
+            const double cs = -fix::W_SCALE * T(7);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const double g = T(k);
                 out(A_GX + k, g);
-                out(A_WX + k, ::fma(cs, v[k], T(4 + k) + T(11 + k)) + ::fma(-vi2, g, T(7 + k)));
+                out(A_WX + k, ::fma(cs, v[k], T(8 + k)) + ::fma(-vi2, g, T(4 + k)));
             }
-            if constexpr (MODE == MODE_FORCE_ENERGY) out(A_PSI, T(16));
+            if constexpr (MODE == MODE_FORCE_ENERGY) out(A_PSI, T(13));
         }
     }
     seq += (uint32_t)(t1 - t0 > 0 ? t1 - t0 : 0);

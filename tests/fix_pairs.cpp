@@ -152,7 +152,8 @@ int main() {
             if (j != i) mc += (g3f[j] * qef + g1f[j]) * (y * y) + kf[j];
         }
         const int lh = lift(mag_exp(mg), mag_exp(mh), LIFT_H), lt = lift(mag_exp(mg), mag_exp(mt), LIFT_T);
-        const Scale E{mag_exp(mg), mag_exp(mc) + 2 * e0 - 3 * eL, -eL, lh, lt};
+        Scale E{mag_exp(mg), 0, 0, -eL, lh, lt};
+        join(E, mag_exp(mc) + 2 * e0 - 3 * eL, E.g + e0 - 2 * eL + 2 - lh + 2 * ev);
         clear<F_FORCE_ENERGY>(A);
         for (int j = t; j < e; ++j) {
             const int em = J[j].em;
@@ -170,7 +171,7 @@ int main() {
         const int gn = E.g + e0 - (energy ? 1 : 2) * eL;
         for (int k = 0; k < 3; ++k) {
             tot[k] += (double)top(A.g[k]) * two(gn - 62);
-            tot[4 + k] += (double)top(A.w[k]) * two(gn + 2 - lh - 62 + 2 * ev) + (double)top(A.t[k]) * two(gn + 2 - lt - 62 + 2 * ev);
+            tot[4 + k] += (double)top(A.t[k]) * two(gn + 2 - lt - 62 + 2 * ev);
             tot[7 + k] += (double)top(A.c[k]) * two(E.c - 62);
         }
         tot[3] += (double)A.s0 * two(gn - eL - 60);
