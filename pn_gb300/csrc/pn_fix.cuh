@@ -117,8 +117,6 @@ PNF V vec(B2 b) {
     r.l = (float)b.l;
     return r;
 }
-// hi + x f, x a sum of cross products and f its unit; |x f| < 2^(31 + B), rounded to 2^B
-template <int B> PNF i64 merge(i64 hi, float x, float f) { return mw(to_int(x * (f * (1.f / (1 << B)))), 1 << B, hi); }
 PNF float crossf(const V &a, const V &b, float c) { return fmaf_(a.hf, b.l, fmaf_(a.l, b.hf, c)); }
 
 PNF u64 mulhi(u64 a, u64 b) {
@@ -139,6 +137,61 @@ PNF u64 shr(u64 a, int s) {
 #endif
 }
 
+// Sums of a product and a 32-bit part as carry additions of their halves: as the addend of a multiply-add the
+// part would have to be moved and extended into a register pair, by moves on the pipe that bounds the
+// sweep (N = 65,536: 77.3 -> 71.3 ms).
+// a + (c >> 32)
+PNF i64 plus_hi(i64 a, i64 c) {
+#ifdef __CUDA_ARCH__
+    const int ch = (int)(c >> 32);
+    unsigned lo, hi;
+    asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
+        : "=r"(lo), "=r"(hi) : "r"((unsigned)a), "r"((unsigned)((u64)a >> 32)), "r"(ch), "r"(ch >> 31));
+    return (i64)(((u64)hi << 32) | lo);
+#else
+    return a + (c >> 32);
+#endif
+}
+// hi 2^32 + a + (c >> 32), unsigned
+PNF u64 plus_hi(u64 a, u64 c, unsigned h) {
+#ifdef __CUDA_ARCH__
+    unsigned lo, hi;
+    asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
+        : "=r"(lo), "=r"(hi) : "r"((unsigned)a), "r"((unsigned)(a >> 32)), "r"((unsigned)(c >> 32)), "r"(h));
+    return ((u64)hi << 32) | lo;
+#else
+    return a + (((u64)h << 32) | (c >> 32));
+#endif
+}
+
+// a + t
+PNF i64 plus_small(i64 a, unsigned t) {
+#ifdef __CUDA_ARCH__
+    unsigned lo, hi;
+    asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, 0;"
+        : "=r"(lo), "=r"(hi) : "r"((unsigned)a), "r"((unsigned)((u64)a >> 32)), "r"(t));
+    return (i64)(((u64)hi << 32) | lo);
+#else
+    return a + t;
+#endif
+}
+// a + t 2^B
+template <int B> PNF i64 plus_low(i64 a, int t) {
+#ifdef __CUDA_ARCH__
+    unsigned lo, hi;
+    asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
+        : "=r"(lo), "=r"(hi)
+        : "r"((unsigned)a), "r"((unsigned)((u64)a >> 32)), "r"((unsigned)t << B), "r"(t >> (32 - B)));
+    return (i64)(((u64)hi << 32) | lo);
+#else
+    return a + (i64)((u64)(i64)t << B);
+#endif
+}
+
+// hi + x f, x a sum of cross products and f its unit; |x f| < 2^(31 + B), rounded to 2^B
+template <int B> PNF i64 merge(i64 hi, float x, float f) {
+    return plus_low<B>(hi, to_int(x * (f * (1.f / (1 << B)))));
+}
 struct X96 {
     unsigned w0, w1, w2;
 };
@@ -364,17 +417,17 @@ PNF void pair(Sums &a, const StarI &I, const StarJ &J, const Scale &E, unsigned 
     const u64 rho = (u64)(mw(bz.h, bz.h, mw(by.h, by.h, mw(bx.h, bx.h, dt >> 31)))) + shr(eps60, 2 * ey);
     // r = 1 - RHO f^2, S = 58
     const unsigned F8 = F << 8;
-    const u64 U = muw((unsigned)(rho >> 32), F8, muw((unsigned)rho, F8, half(32)) >> 32);  // RHO f, S = 59
-    const i64 r = (i64)((1ULL << 58) - muw((unsigned)(U >> 32), F8, muw((unsigned)U, F8, half(32)) >> 32));
+    const u64 U = plus_hi(muw((unsigned)(rho >> 32), F8, 0), muw((unsigned)rho, F8, half(32)), 0u);  // RHO f, S = 59
+    const i64 r = (i64)((1ULL << 58) - plus_hi(muw((unsigned)(U >> 32), F8, 0), muw((unsigned)U, F8, half(32)), 0u));
     const int rs = (int)(r >> 12);                          // S = 46 (below 2^28)
     const int rsq = (int)(mw(rs, rs, 0) >> 32);             // r^2, S = 60
-    const i64 c = mw(6, rsq, r << 5);                       // r/2 + 3 r^2/8, S = 64
+    const i64 c = plus_small(r << 5, 6u * (unsigned)rsq);  // r/2 + 3 r^2/8, S = 64
     const int F7 = (int)(F << 7);
-    const u64 Q = (u64)mw(F7, (int)(c >> 32), (i64)(((u64)F7 << 32) | (muw((unsigned)F7, (unsigned)c, 0) >> 32)));  // S = 62
+    const u64 Q = plus_hi((u64)mw(F7, (int)(c >> 32), 0), muw((unsigned)F7, (unsigned)c, 0), (unsigned)F7);  // S = 62
     const B2 bq = bal((i64)Q);
     // n = d Q, S = 60
-    const B2 mx = bal(mw(bx.h, bq.h, cross(bx, bq, half(32)) >> 32)), my = bal(mw(by.h, bq.h, cross(by, bq, half(32)) >> 32)),
-             mz = bal(mw(bz.h, bq.h, cross(bz, bq, half(32)) >> 32));
+    const B2 mx = bal(plus_hi(mw(bx.h, bq.h, 0), cross(bx, bq, half(32)))), my = bal(plus_hi(mw(by.h, bq.h, 0), cross(by, bq, half(32)))),
+             mz = bal(plus_hi(mw(bz.h, bq.h, 0), cross(bz, bq, half(32))));
     if (MODE == F_ENERGY) {
         const V q = vec(bq);
         const u64 mQ = muw(J.mh, (unsigned)q.h, 0) + ((u64)(i64)to_int(fmaf_(J.mhf, q.l, J.ml * q.hf)) << 2);  // S = 62
@@ -398,7 +451,7 @@ PNF void pair(Sums &a, const StarI &I, const StarJ &J, const Scale &E, unsigned 
     add(a.g[1], p, my);
     add(a.g[2], p, mz);
     if (MODE == F_NEWTON) return;
-    a.s0 += mw(p.h, bq.h, cross(p, bq, 0) >> 32) >> ey;  // m Q^3 = (m Q^2) Q
+    a.s0 += plus_hi(mw(p.h, bq.h, 0), cross(p, bq, 0)) >> ey;  // m Q^3 = (m Q^2) Q
     // velocity terms: the dot products' small parts in FP32, the sums in integers
     const V nx = vec(mx), ny = vec(my), nz = vec(mz), wx = vec(J.wx), wy = vec(J.wy), wz = vec(J.wz);
     const Acc uw = dot(I.ux, I.uy, I.uz, wx, wy, wz), un = dot(I.ux, I.uy, I.uz, nx, ny, nz), wn = dot(wx, wy, wz, nx, ny, nz);
