@@ -920,15 +920,14 @@ static pn_ctx *drop_ctx(double eps) {
     return g_drop;
 }
 
-// Copies x, v, m (host AoS) to the device AoS staging buffers of the implicit context.
+// Copies x, v, m (host AoS) to the device AoS staging buffer of the implicit context, one after the
+// other: x at 0, v at 3 n, m at 6 n (one copy; three made a force of 1,000 stars take 104.5 us instead of 97.6).
 static int drop_upload(pn_ctx *c, const double *x, const double *v, const double *m, int n) {
-    const size_t ld = (size_t)c->ld;
-    std::memcpy(g_drop_h, x, 3 * (size_t)n * sizeof(double));
-    std::memcpy(g_drop_h + 3 * ld, v, 3 * (size_t)n * sizeof(double));
-    std::memcpy(g_drop_h + 6 * ld, m, (size_t)n * sizeof(double));
-    CU(cudaMemcpyAsync(c->in_aos, g_drop_h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->in_aos + 3 * ld, g_drop_h + 3 * ld, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->in_aos + 6 * ld, g_drop_h + 6 * ld, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    const size_t w = (size_t)n;
+    std::memcpy(g_drop_h, x, 3 * w * sizeof(double));
+    std::memcpy(g_drop_h + 3 * w, v, 3 * w * sizeof(double));
+    std::memcpy(g_drop_h + 6 * w, m, w * sizeof(double));
+    CU(cudaMemcpyAsync(c->in_aos, g_drop_h, 7 * w * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
     c->n = n;
     return PN_OK;
@@ -943,19 +942,19 @@ extern "C" void force(double (*x)[3], double (*v)[3], double *m, double eps, dou
     }
     pn_ctx *c = drop_ctx(eps);
     if (!c) return;
-    const size_t ld = (size_t)c->ld;
+    const size_t w = (size_t)n;
     if (drop_upload(c, &x[0][0], &v[0][0], m, n)) drop_fatal("force");
-    int rc = eval_force(c, c->in_aos, c->in_aos + 3 * ld, c->in_aos + 6 * ld, 3, 1, c->a_aos, 3, 1, 0,
+    int rc = eval_force(c, c->in_aos, c->in_aos + 3 * w, c->in_aos + 6 * w, 3, 1, c->a_aos, 3, 1, 0,
                         c->stream, false);
     if (rc) drop_fatal("force");
-    if (cudaMemcpyAsync(g_drop_h, c->a_aos, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
+    if (cudaMemcpyAsync(g_drop_h, c->a_aos, 3 * w * sizeof(double), cudaMemcpyDeviceToHost,
                         c->stream) != cudaSuccess) {
         set_err(PN_ERR_CUDA, "force: copy back");
         drop_fatal("force");
     }
     rc = check_device_err(c);  // sets the last error (PN_OK or PN_ERR_NONFINITE)
     if (rc == PN_ERR_CUDA || rc == PN_ERR_TIMEOUT) drop_fatal("force");
-    std::memcpy(&a[0][0], g_drop_h, 3 * (size_t)n * sizeof(double));
+    std::memcpy(&a[0][0], g_drop_h, 3 * w * sizeof(double));
 }
 
 static int drop_energy(double x[][3], double v[][3], double m[], int n, double eps, pn_energy_t *e) {
@@ -963,9 +962,9 @@ static int drop_energy(double x[][3], double v[][3], double m[], int n, double e
         return set_err(PN_ERR_INVALID, "energy: n=%d", n);
     pn_ctx *c = drop_ctx(eps);
     if (!c) return g_last_error;
-    const size_t ld = (size_t)c->ld;
+    const size_t w = (size_t)n;
     if (drop_upload(c, &x[0][0], &v[0][0], m, n)) drop_fatal("energy");
-    int rc = eval_energy(c, c->in_aos, c->in_aos + 3 * ld, c->in_aos + 6 * ld, 3, 1, e);
+    int rc = eval_energy(c, c->in_aos, c->in_aos + 3 * w, c->in_aos + 6 * w, 3, 1, e);
     if (rc == PN_ERR_CUDA || rc == PN_ERR_TIMEOUT) drop_fatal("energy");
     return rc;
 }
