@@ -70,6 +70,12 @@ struct pn_ens {
     pn_params p{};
     int ipt = 2, js = 1;
     int x2 = 0;  // mixed precision: the packed FP32x2 sweep (js = 1)
+    bool sym = false;       // ... forming every pair once (the force sweep, pn_pairsym.cuh)
+    int sms = 0;
+    void *sym_work = nullptr;  // its partial sums
+    Pair2SymArgs *t_sym = nullptr;  // [nc]
+    int4 *sym_items = nullptr;
+    int nsym = 0;
     ClassShape cls[32];
     cudaStream_t stream = nullptr;
     double *state = nullptr;
@@ -85,7 +91,7 @@ struct pn_ens {
     int *err = nullptr;
     int4 *blockmap = nullptr, *items = nullptr;
     int nitems = 0;
-    PrepArgs *t_prep = nullptr;    // [2][nc]: evaluation at (x, v) / at (xs, vs)
+    PrepArgs *t_prep = nullptr;    // [3][nc]: force evaluation at (x, v) / at (xs, vs); energy at (x, v)
     FinishArgs *t_fin = nullptr;   // [4][nc]: stage 0 (a out), 1, 2, 3
     EnergyArgs *t_en = nullptr;    // [nc]
     PairArgs *t_pair = nullptr;    // [2][nc]: force / energy sweep
@@ -104,7 +110,7 @@ static void ens_free(pn_ens *e) {
     if (e->step_exec) cudaGraphExecDestroy(e->step_exec);
     void *bufs[] = {e->state, e->a_aos, e->spos, e->acc, e->ppart, e->fpart, e->glob, e->eout,
                     e->pack, e->pack2, e->ipack, e->torg, e->tickets, e->counter, e->err, e->blockmap, e->items,
-                    e->t_prep, e->t_fin, e->t_en, e->t_pair};
+                    e->t_prep, e->t_fin, e->t_en, e->t_pair, e->sym_work, e->t_sym, e->sym_items};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (e->e0) cudaEventDestroy(e->e0);
@@ -125,6 +131,63 @@ static int cluster_gsplit(const pn_ens *e, int c) {
     return g;
 }
 
+// Tables and work items of the sweep over unordered pairs; false (and the packed sweep) where its
+// partial sums would take more than SYM_ENS_BYTES or there is no memory for them.  Tiles per item as for
+// one system (pn_api.cu, choose_sym), over the work of all clusters.
+constexpr size_t SYM_ENS_BYTES = (size_t)2 << 30;
+static bool ens_build_sym(pn_ens *e) {
+    long long units = 0;
+    for (int c = 0; c < e->nc; ++c) {
+        const long long nt = (e->n[c] + 126) / 128, nb = (nt + 3) / 4;
+        units += nb * nt - 2 * nb * (nb - 1);
+    }
+    const int chunk = (int)std::min<long long>(8, std::max<long long>(1, (units + 12 * e->sms - 1) / (12 * e->sms)));
+    size_t bytes = 0;
+    for (int c = 0; c < e->nc; ++c) bytes += sym_ens_bytes(e->n[c] - 1, chunk);
+    if (bytes > SYM_ENS_BYTES) return false;
+    for (void **p : {&e->sym_work, (void **)&e->t_sym, (void **)&e->sym_items}) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+    }
+    std::vector<Pair2SymArgs> tab(e->nc);
+    std::vector<int4> items;
+    if (cudaMalloc(&e->sym_work, std::max<size_t>(1, bytes)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    char *work = static_cast<char *>(e->sym_work);
+    for (int c = 0; c < e->nc; ++c) {
+        const int nstar = e->n[c] - 1;
+        const size_t so = (size_t)e->s0[c];
+        Pair2SymArgs &a = tab[c];
+        a = Pair2SymArgs{};
+        sym_ens_args(&a, nstar, chunk, work);
+        work += sym_ens_bytes(nstar, chunk);
+        a.pack = static_cast<const float4 *>(e->pack) + so;
+        a.torg = e->torg + so / 32;
+        a.spos = e->spos + so;
+        a.out = reinterpret_cast<float2 *>(e->acc + so);
+        a.err = e->err;
+        a.npad = e->S;
+        a.eps2 = e->eps[c] * e->eps[c];
+        for (int b = 0; 4 * b < a.p1; ++b)
+            for (int y = 4 * b / chunk; y * chunk < a.p1; ++y) items.push_back(make_int4(c, b, y, 0));
+    }
+    auto tiles = [&](const int4 &w) {
+        return std::min(tab[w.x].p1, (w.z + 1) * chunk) - std::max(4 * w.y, w.z * chunk);
+    };
+    std::stable_sort(items.begin(), items.end(), [&](const int4 &a, const int4 &b) { return tiles(a) > tiles(b); });
+    e->nsym = (int)items.size();
+    const size_t ib = std::max<size_t>(1, items.size()) * sizeof(int4), tb = tab.size() * sizeof(Pair2SymArgs);
+    if (cudaMalloc(&e->t_sym, tb) != cudaSuccess || cudaMalloc(&e->sym_items, ib) != cudaSuccess ||
+        cudaMemcpy(e->t_sym, tab.data(), tb, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(e->sym_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 // Rebuilds the argument tables and the work-item list from the current shapes.
 static int ens_build_tables(pn_ens *e) {
     const bool f32 = ens_f32(e);
@@ -138,7 +201,8 @@ static int ens_build_tables(pn_ens *e) {
         ECU(cudaMalloc(&e->acc, (size_t)gmax * NACC_MAX * e->S * sizeof(double)));
         e->acc_splits = gmax;
     }
-    std::vector<PrepArgs> tp(2 * nc);
+    if (e->sym) e->sym = ens_build_sym(e);
+    std::vector<PrepArgs> tp(3 * nc);
     std::vector<FinishArgs> tf(4 * nc);
     std::vector<EnergyArgs> te(nc);
     std::vector<PairArgs> tq(2 * nc);
@@ -154,11 +218,11 @@ static int ens_build_tables(pn_ens *e) {
         DevState sc = e->st;  // pointers offset to this cluster's first particle
         sc.x += e->p0[c]; sc.v += e->p0[c]; sc.xs += e->p0[c]; sc.vs += e->p0[c];
         sc.hx += e->p0[c]; sc.hv += e->p0[c]; sc.m += e->p0[c];
-        for (int ev = 0; ev < 2; ++ev) {
+        for (int ev = 0; ev < 3; ++ev) {
             PrepArgs &pa = tp[ev * nc + c];
             pa = PrepArgs{};
-            pa.x = ev ? sc.xs : sc.x;
-            pa.v = ev ? sc.vs : sc.v;
+            pa.x = ev == 1 ? sc.xs : sc.x;
+            pa.v = ev == 1 ? sc.vs : sc.v;
             pa.m = sc.m;
             pa.sp = 1;
             pa.sk = ld;
@@ -169,7 +233,11 @@ static int ens_build_tables(pn_ens *e) {
             pa.f32 = f32;
             pa.eps2 = eps2;
             pa.pack = static_cast<char *>(e->pack) + so * 16;
-            if (e->pack2) {  // slot offsets are multiples of 256, so so / 2 is a whole pair row
+            if (e->sym && ev < 2) {
+                pa.tj = 128;
+                pa.pack = nullptr;
+                pa.spack = static_cast<float4 *>(e->pack) + so;
+            } else if (e->pack2) {  // slot offsets are multiples of 256, so so / 2 is a whole pair row
                 pa.pack2 = e->pack2 + so / 2;
                 pa.ipack = e->ipack + so;
             }
@@ -212,7 +280,7 @@ static int ens_build_tables(pn_ens *e) {
             fa.nstar = nstar;
             fa.npad = e->S;
             fa.nacc = pair_nacc(mode);
-            fa.gsplit = g;
+            fa.gsplit = e->sym ? 1 : g;
             fa.accf = f32 && e->x2 && e->js == 1;
             fa.pn1 = mode == MODE_FORCE;
             fa.eps = eps;
@@ -289,6 +357,10 @@ static int ens_tjmax(const pn_ens *e) {
 
 static int ens_pair_launch(pn_ens *e, int mode, const PairArgs *tab, cudaStream_t s) {
     ECU(cudaMemsetAsync(e->counter, 0, sizeof(unsigned), s));
+    if (e->sym && mode == MODE_FORCE) {
+        ECU(launch_pair_sym_ens(e->t_sym, e->sym_items, e->nsym, e->blockmap, e->B, e->sms, e->counter, s));
+        return PN_OK;
+    }
     cudaError_t r;
     if (ens_f32(e) && e->x2 && e->js == 1 && e->pack2)
         r = launch_pair2_ens_f32(mode, e->ipt, ens_tjmax(e), 0, tab, e->items, e->nitems, e->counter, s);
@@ -358,6 +430,13 @@ extern "C" int pn_ens_create(pn_ens **out, int nclusters, const int *n, const do
     e->B = B;
     e->LD = (int)rup(P, 256);
     if (ens_f32(e)) { e->ipt = 2; e->js = 1; e->x2 = 1; } else { e->ipt = 1; e->js = 4; }
+    e->sym = ens_f32(e) && ens_mode(e) == MODE_FORCE;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || e->sms < 1) {
+        ens_free(e);
+        return fail(PN_ERR_CUDA, "SM count");
+    }
     for (int k = 0; k < 32; ++k) {
         e->cls[k].tj = ens_f32(e) ? (k >= 12 ? 256 : 128) : 128;
         e->cls[k].tiles_per_item = 32;
@@ -390,7 +469,7 @@ extern "C" int pn_ens_create(pn_ens **out, int nclusters, const int *n, const do
     if (cudaMalloc(&e->counter, sizeof(unsigned))) return bad("counter");
     if (cudaMalloc(&e->err, sizeof(int))) return bad("err");
     if (cudaMalloc(&e->blockmap, (size_t)B * sizeof(int4))) return bad("blockmap");
-    if (cudaMalloc(&e->t_prep, 2 * (size_t)nclusters * sizeof(PrepArgs))) return bad("tables");
+    if (cudaMalloc(&e->t_prep, 3 * (size_t)nclusters * sizeof(PrepArgs))) return bad("tables");
     if (cudaMalloc(&e->t_fin, 4 * (size_t)nclusters * sizeof(FinishArgs))) return bad("tables");
     if (cudaMalloc(&e->t_en, (size_t)nclusters * sizeof(EnergyArgs))) return bad("tables");
     if (cudaMalloc(&e->t_pair, 2 * (size_t)nclusters * sizeof(PairArgs))) return bad("tables");
@@ -521,7 +600,7 @@ extern "C" int pn_ens_bench_steps(pn_ens *e, int nsteps, double *step_ms) {
 
 extern "C" int pn_ens_energy(pn_ens *e, double *out) {
     if (!e || !e->have_state || !out) return fail(PN_ERR_STATE, "pn_ens_energy");
-    ECU(launch_prep_ens(e->t_prep, e->blockmap, e->B, e->stream));
+    ECU(launch_prep_ens(e->t_prep + 2 * (size_t)e->nc, e->blockmap, e->B, e->stream));
     int rc = ens_pair_launch(e, MODE_ENERGY, e->t_pair + e->nc, e->stream);
     if (rc) return rc;
     ECU(launch_energy_ens(e->t_en, e->blockmap, e->B, e->stream));
@@ -534,11 +613,13 @@ extern "C" int pn_ens_last_error(void) { return g_ens_err; }
 
 extern "C" int pn_ens_set_shape(pn_ens *e, int ipt, int js, int size_class_, int tile_j, int tiles_per_item) {
     if (!e) return fail(PN_ERR_INVALID, "pn_ens_set_shape");
+    bool chosen = false;
     if (ipt > 0 || js > 0) {
         if (!ens_shape_supported(ipt, js)) return fail(PN_ERR_INVALID, "shape");
         e->ipt = ipt;
         e->js = js;
         e->x2 = 0;  // an explicit shape selects the scalar sweep
+        chosen = true;
     }
     if (size_class_ >= 0) {
         if (size_class_ > 31 || (tile_j != 32 && tile_j != 64 && tile_j != 128 && tile_j != 256) ||
@@ -546,7 +627,9 @@ extern "C" int pn_ens_set_shape(pn_ens *e, int ipt, int js, int size_class_, int
             return fail(PN_ERR_INVALID, "class shape");
         e->cls[size_class_].tj = tile_j;
         e->cls[size_class_].tiles_per_item = tiles_per_item;
+        chosen = true;
     }
+    if (chosen) e->sym = false;  // (it has no such shapes)
     return ens_build_tables(e);
 }
 
@@ -574,6 +657,7 @@ extern "C" int pn_ens_autotune(pn_ens *e) {
         ECU(cudaEventElapsedTime(ms, e->e0, e->e1));
         return PN_OK;
     };
+    e->sym = false;  // (tried at the end)
     // per class: the other classes keep their shape; only this class's items are timed by
     // restricting the item list to it
     for (int k : classes) {
@@ -632,8 +716,20 @@ extern "C" int pn_ens_autotune(pn_ens *e) {
     e->ipt = bi;
     e->js = bj;
     e->x2 = bx;
+    e->sym = f32 && mode == MODE_FORCE && bx && bj == 1;
     int rc = ens_build_tables(e);
     if (rc) return rc;
+    if (e->sym) {
+        float ms = 0.f, ms2 = 0.f;
+        rc = time_sweep(&ms);
+        if (!rc) rc = time_sweep(&ms2);
+        if (rc) return rc;
+        if (std::min(ms, ms2) >= best_ms) {
+            e->sym = false;
+            rc = ens_build_tables(e);
+            if (rc) return rc;
+        }
+    }
     return ens_check(e);
 }
 

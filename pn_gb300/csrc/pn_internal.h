@@ -38,6 +38,28 @@ bool pair_shape_supported(int ipt, int js);
 constexpr size_t SYM_PANEL_BYTES = (size_t)512 << 20;
 size_t sym_bytes(int nstar, int chunk);
 int sym_panels(int nstar, int chunk);
+// (its argument block: pn_pairsym.cuh)
+constexpr int SYM2_ROWS = 512, SYM2_TJ = 128, SYM2_NG = 4, SYM2_NS = 9;
+
+struct Pair2SymArgs {
+    const float4 *pack;      // [SYM2_NG][npad]: (x y z m) (lx ly lz mu3) (wx wy wz c1) (c3 k35 qe 0), scaled (k_prep)
+    const TileOrigin *torg;  // per tile of 128
+    const double *spos;
+    float2 *rows;            // [chunks][9][rstride] row sums (sum, -compensation) of each range of tiles
+    float *cols;             // [blocks][9][cstride] sums of the panel's star j from row block b
+    float2 *out;             // [9][npad]
+    int *err;
+    int nstar, npad, chunk;  // tiles per range
+    int p0, p1;              // tiles of this panel (multiples of 4, or the last tile)
+    int rstride, cstride;
+    double eps2;
+};
+// Its ensemble form: one panel per cluster (tab[c]), items (cluster, row block, range of chunk tiles, 0);
+// blockmap, nblocks: the O(N) kernels' blocks of 128 stars.  sym_ens_bytes: a cluster's partial sums.
+size_t sym_ens_bytes(int nstar, int chunk);
+void sym_ens_args(Pair2SymArgs *a, int nstar, int chunk, void *work);
+cudaError_t launch_pair_sym_ens(const Pair2SymArgs *tab, const int4 *items, int nitems, const int4 *blockmap,
+                                int nblocks, int sms, unsigned *counter, cudaStream_t s);
 cudaError_t launch_pair_sym(const PairCfg &c, const PairArgs &a, void *work, cudaStream_t s);
 
 // Persistent ensemble sweep (k_pair_ens): (ipt, js) in {(1,1), (2,1), (1,4)}; tjmax = the

@@ -38,6 +38,30 @@ int sym_panels(int nstar, int chunk) {
     return n;
 }
 
+size_t sym_ens_bytes(int nstar, int chunk) { return panel_bytes(0, (nstar + SYM2_TJ - 1) / SYM2_TJ, chunk); }
+
+void sym_ens_args(Pair2SymArgs *a, int nstar, int chunk, void *work) {
+    a->nstar = nstar;
+    a->chunk = chunk;
+    a->p0 = 0;
+    a->p1 = (nstar + SYM2_TJ - 1) / SYM2_TJ;
+    a->rstride = a->cstride = a->p1 * SYM2_TJ;
+    a->rows = static_cast<float2 *>(work);
+    a->cols = reinterpret_cast<float *>(a->rows + (size_t)((a->p1 + chunk - 1) / chunk) * SYM2_NS * a->rstride);
+}
+
+cudaError_t launch_pair_sym_ens(const Pair2SymArgs *tab, const int4 *items, int nitems, const int4 *blockmap,
+                                int nblocks, int sms, unsigned *counter, cudaStream_t s) {
+    if (nitems <= 0) return cudaSuccess;
+    const size_t smem = sym2_smem_bytes();
+    cudaError_t e = cudaFuncSetAttribute(k_pair2_sym_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_pair2_sym_ens<<<2 * sms, PAIR_NT, smem, s>>>(tab, items, nitems, counter);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_sym_reduce_ens<<<dim3(nblocks, SYM2_NS), 128, 0, s>>>(tab, blockmap);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pair_sym(const PairCfg &c, const PairArgs &q, void *work, cudaStream_t s) {
     if (q.nstar <= 0) return cudaSuccess;
     if (c.tj != SYM2_TJ || c.gsplit < 1 || !work) return cudaErrorInvalidValue;

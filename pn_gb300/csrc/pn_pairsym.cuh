@@ -35,22 +35,6 @@
 
 namespace pn {
 
-constexpr int SYM2_ROWS = 512, SYM2_TJ = 128, SYM2_NG = 4, SYM2_NS = 9;
-
-struct Pair2SymArgs {
-    const float4 *pack;      // [SYM2_NG][npad]: (x y z m) (lx ly lz mu3) (wx wy wz c1) (c3 k35 qe 0), scaled (k_prep)
-    const TileOrigin *torg;  // per tile of 128
-    const double *spos;
-    float2 *rows;            // [chunks][9][rstride] row sums (sum, -compensation) of each range of tiles
-    float *cols;             // [blocks][9][cstride] sums of the panel's star j from row block b
-    float2 *out;             // [9][npad]
-    int *err;
-    int nstar, npad, chunk;  // tiles per range
-    int p0, p1;              // tiles of this panel (multiples of 4, or the last tile)
-    int rstride, cstride;
-    double eps2;
-};
-
 inline size_t sym2_smem_bytes() {
     return 128 + (size_t)2 * SYM2_NS * 4 * PAIR_NT * 4 + (size_t)4 * 10 * SYM2_TJ * 4 + (size_t)2 * SYM2_NG * SYM2_TJ * 16;
 }
@@ -142,22 +126,17 @@ __device__ __forceinline__ void sym2_tile(f2 (&y)[2][10], float *zs, const Row2 
     }
 }
 
-__global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) {
+// One work item: row block blk against range y of the panel's tiles.  seq: the tiles that this CTA has
+// consumed before (pair_block).  Returns false when a bounded wait gave up.
+__device__ __forceinline__ bool sym2_block(const Pair2SymArgs &a, int blk, int y, unsigned char *smem, uint32_t &seq) {
     constexpr int NT = PAIR_NT, TJ = SYM2_TJ, NS = SYM2_NS;
-    extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
     float *kahan = reinterpret_cast<float *>(smem + 128);          // [2][9][4][128]
     float *zs = kahan + 2 * NS * 4 * NT;                           // [4][10][128]
     float4 *buf = reinterpret_cast<float4 *>(zs + 4 * 10 * TJ);    // [2][8][128]
-    const int tid = threadIdx.x, blk = blockIdx.x;
-    const int tc = a.p0 + (int)blockIdx.y * a.chunk, t0 = max(4 * blk, tc), t1 = min(a.p1, tc + a.chunk);
-    if (t0 >= t1) return;
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
+    const int tid = threadIdx.x;
+    const int tc = a.p0 + y * a.chunk, t0 = max(4 * blk, tc), t1 = min(a.p1, tc + a.chunk);
+    if (t0 >= t1) return true;
     const f2 eps2 = f2_bcast((float)a.eps2);
     float sh[3][4], sl[3][4];
     Row2 I[2];
@@ -194,10 +173,11 @@ __global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) 
         for (int g = 0; g < SYM2_NG; ++g)
             bulk_g2s(buf + (size_t)(stage * SYM2_NG + g) * TJ, a.pack + (size_t)g * a.npad + (size_t)t * TJ, gbytes, &bars[stage]);
     };
-    if (tid == 0) issue(t0, 0);
+    if (tid == 0) issue(t0, (int)(seq & 1u));
     for (int t = t0; t < t1; ++t) {
-        const int it = t - t0, stage = it & 1;
-        const uint32_t phase = (uint32_t)(it >> 1) & 1u;
+        const uint32_t it = seq + (uint32_t)(t - t0);
+        const int stage = (int)(it & 1u);
+        const uint32_t phase = (it >> 1) & 1u;
         const bool next = t + 1 < t1;
         if (tid == 0 && next) issue(t + 1, stage ^ 1);
         const bool ok = mbar_wait_bounded(&bars[stage], phase);
@@ -205,9 +185,9 @@ __global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) 
             if (tid == 0) {
                 atomicOr(a.err, DEVERR_TIMEOUT);
                 mbar_wait_bounded(&bars[stage], phase);
-                if (next) mbar_wait_bounded(&bars[stage ^ 1], (uint32_t)((it + 1) >> 1) & 1u);
+                if (next) mbar_wait_bounded(&bars[stage ^ 1], ((it + 1) >> 1) & 1u);
             }
-            return;
+            return false;
         }
         {
             const TileOrigin &o = a.torg[t];
@@ -283,15 +263,52 @@ __global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) 
         if (i < a.nstar)
 #pragma unroll
             for (int q = 0; q < NS; ++q)
-                a.rows[((size_t)blockIdx.y * NS + q) * a.rstride + i] = make_float2(ksum(q, r), -kcmp(q, r));
+                a.rows[((size_t)y * NS + q) * a.rstride + i] = make_float2(ksum(q, r), -kcmp(q, r));
+    }
+    seq += (uint32_t)(t1 - t0);
+    return true;
+}
+
+__device__ __forceinline__ void sym2_init(unsigned char *smem) {
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
+    if (threadIdx.x == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    sym2_init(smem);
+    uint32_t seq = 0;
+    sym2_block(a, blockIdx.x, blockIdx.y, smem, seq);
+}
+
+// Ensemble form, as k_pair2_ens: items (cluster, row block, range, 0), one panel per cluster.
+__global__ void __launch_bounds__(PAIR_NT, 2)
+    k_pair2_sym_ens(const Pair2SymArgs *tab, const int4 *items, int nitems, unsigned *counter) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int cur;
+    sym2_init(smem);
+    uint32_t seq = 0;
+    for (;;) {
+        if (threadIdx.x == 0) cur = (int)atomicAdd(counter, 1u);
+        __syncthreads();
+        const int w = cur;
+        __syncthreads();  // everyone has read cur before thread 0 fetches the next item
+        if (w >= nitems) break;
+        const int4 it = items[w];
+        const Pair2SymArgs a = tab[it.x];
+        if (!sym2_block(a, it.y, it.z, smem, seq)) break;
     }
 }
 
 // Adds a star's slots of a panel in order: the row sums of its block's ranges, then the column sums from
 // the row blocks before its own (a star of an earlier panel only has row sums there, on top of its
 // sums so far).  One thread per (star, sum).
-__global__ void __launch_bounds__(256) k_sym_reduce(const Pair2SymArgs a) {
-    const int i = blockIdx.x * 256 + threadIdx.x, q = blockIdx.y;
+__device__ __forceinline__ void sym_reduce_star(const Pair2SymArgs &a, int i, int q) {
     if (i >= min(a.nstar, a.p1 * SYM2_TJ)) return;
     const int blk = i / SYM2_ROWS, nchunk = (a.p1 - a.p0 + a.chunk - 1) / a.chunk, j = i - a.p0 * SYM2_TJ;
     float2 *out = a.out + (size_t)q * a.npad + i;
@@ -322,6 +339,14 @@ __global__ void __launch_bounds__(256) k_sym_reduce(const Pair2SymArgs a) {
         }
     }
     *out = make_float2(h, l);
+}
+__global__ void __launch_bounds__(256) k_sym_reduce(const Pair2SymArgs a) {
+    sym_reduce_star(a, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(128) k_sym_reduce_ens(const Pair2SymArgs *tab, const int4 *blockmap) {
+    const int4 bm = blockmap[blockIdx.x];
+    const Pair2SymArgs a = tab[bm.x];
+    sym_reduce_star(a, bm.y * 128 + threadIdx.x, blockIdx.y);
 }
 
 }  // namespace pn

@@ -128,3 +128,30 @@ def test_tuned_shapes(pn, precision):
     else:
         assert np.abs(a - b).max() <= 1e-12 * np.abs(a).max()
     assert np.abs(e - f).max() <= (1e-6 if precision else 1e-12) * np.abs(e).max()
+
+
+class _System:
+    def __init__(self, n):
+        self.x, self.v, self.m = system(n)
+
+
+@pytest.mark.parametrize("ic2", [1e-6, 1.0])
+def test_ensemble_every_pair_once(pn, ic2):
+    """Clusters at the edges of tiles and row blocks in one launch, also after their energies and with the
+    shape given (which selects the ordered sweep)."""
+    sizes = [1, 2, 3, 128, 129, 130, 512, 513, 514, 641, 1026, 2049, 4100]
+    systems = [_System(n) for n in sizes]
+    with pn.Ensemble(systems, [EPS] * len(sizes), precision=1, inv_c2=ic2, dt=1e-3) as e:
+        a = e.force()
+        en = e.energy()
+        again = e.force()
+        e.set_shape(2, 1)
+        ordered = e.force()
+        en2 = e.energy()
+    for s, f, g, h in zip(systems, a, again, ordered):
+        assert np.array_equal(f, g)
+        ref = force(pn, s.x, s.v, s.m, ic2, 0)
+        if len(s.x) > 1:
+            close(f, ref, len(s.x))
+            close(h, ref, len(s.x))
+    assert np.abs(en - en2).max() <= 1e-6 * np.abs(en).max()
