@@ -19,9 +19,12 @@
 // star j's 4 a / 3 + P^2 Q'^2 and, with d reversed, P - 4 S / 3.  The terms -|v|^2 of the brackets and
 // -w sum ct are applied once per tile.
 //
-// A sum runs over 128 terms at most before it is folded (rows) or 64 in each half of an operand
-// (stars j).  Against FP64 the median error of the accelerations is 0.93 to 0.99 of k_pair2's at its tiles of
-// 256 (N = 8,100 to 32,767, inv_c2 = 1e-6; 0.75 to 0.85 at 1).
+// Row sums run over SPAN terms before they are folded, star j's over 64 in each half of an operand.
+// SPAN is what k_pair2's tiles give: 128 for one system of 8,000 stars or more (256-star tiles),
+// 64 for an ensemble, whose clusters may be small (128-star tiles; folding twice per tile costs 1 % there, and 4 %
+// at N = 262,144).  Against FP64 the median error of the accelerations is 0.93 to 0.99 of k_pair2's for
+// one system (N = 8,100 to 32,767, inv_c2 = 1e-6; 0.75 to 0.85 at 1); for ensembles of 128 to 4,000 stars
+// the error of the whole vector is 0.95 of k_pair2's in the mean (with 128 terms it was 1.15 of it).
 //
 // Bound by the FP32 FMA pipe (71 % active at N = 16,384) and, with two warps per scheduler, by the latency
 // between its instructions.  Per step of a warp that pipe takes 300 cycles, the shared-memory pipe of
@@ -102,11 +105,11 @@ __device__ __forceinline__ void sym2_load(Star2 &J, const float4 *b, int q) {
     J.c3 = f2_bcast(g3.x); J.k35 = f2_bcast(g3.y); J.qe = f2_bcast(g3.z);
 }
 
-template <bool BOTH>
-__device__ __forceinline__ void sym2_tile(f2 (&y)[2][10], float *zs, const Row2 (&I)[2], const float4 *b, f2 eps2) {
+template <bool BOTH, int SPAN>
+__device__ __forceinline__ void sym2_span(f2 (&y)[2][10], float *zs, const Row2 (&I)[2], const float4 *b, f2 eps2, int k0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int from = (lane + 1) & 31;
-    for (int k = 0; k < SYM2_TJ; k += 32) {
+    for (int k = k0; k < k0 + SPAN; k += 32) {
         f2 z[10];
 #pragma unroll
         for (int c = 0; c < 10; ++c) z[c] = 0ull;
@@ -128,6 +131,7 @@ __device__ __forceinline__ void sym2_tile(f2 (&y)[2][10], float *zs, const Row2 
 
 // One work item: row block blk against range y of the panel's tiles.  seq: the tiles that this CTA has
 // consumed before (pair_block).  Returns false when a bounded wait gave up.
+template <int SPAN>
 __device__ __forceinline__ bool sym2_block(const Pair2SymArgs &a, int blk, int y, unsigned char *smem, uint32_t &seq) {
     constexpr int NT = PAIR_NT, TJ = SYM2_TJ, NS = SYM2_NS;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
@@ -208,35 +212,38 @@ __device__ __forceinline__ bool sym2_block(const Pair2SymArgs &a, int blk, int y
             }
         }
         const float4 *b = buf + (size_t)stage * SYM2_NG * TJ;
-        f2 y[2][10];
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int c = 0; c < 10; ++c) y[p][c] = 0ull;
         const bool both = t >= 4 * blk + 4;  // (the whole CTA)
-        if (both)
-            sym2_tile<true>(y, zs, I, b, eps2);
-        else
-            sym2_tile<false>(y, zs, I, b, eps2);
-        // rows: -w sum ct and -|v|^2 G of the tile into W, then the running sums
+#pragma unroll 1
+        for (int k = 0; k < TJ; k += SPAN) {
+            f2 y[2][10];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const f2 third = f2_bcast((float)(-1.0 / 3.0));
-            const f2 nv2 = mul2(third, fma2(I[p].wz, I[p].wz, fma2(I[p].wy, I[p].wy, mul2(I[p].wx, I[p].wx))));
-            const f2 nct = sub2(0ull, y[p][9]);
-            y[p][6] = fma2(nct, I[p].wx, fma2(nv2, y[p][0], y[p][6]));
-            y[p][7] = fma2(nct, I[p].wy, fma2(nv2, y[p][1], y[p][7]));
-            y[p][8] = fma2(nct, I[p].wz, fma2(nv2, y[p][2], y[p][8]));
+            for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int q = 0; q < NS; ++q) {
-                float ts[2];
-                f2_unpack(y[p][q], ts[0], ts[1]);
+                for (int c = 0; c < 10; ++c) y[p][c] = 0ull;
+            if (both)
+                sym2_span<true, SPAN>(y, zs, I, b, eps2, k);
+            else
+                sym2_span<false, SPAN>(y, zs, I, b, eps2, k);
+            // rows: -w sum ct and -|v|^2 G into W, then the running sums
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float sum = ksum(q, 2 * p + e), comp = kcmp(q, 2 * p + e);
-                    kahan_add(sum, comp, ts[e]);
-                    ksum(q, 2 * p + e) = sum;
-                    kcmp(q, 2 * p + e) = comp;
+            for (int p = 0; p < 2; ++p) {
+                const f2 third = f2_bcast((float)(-1.0 / 3.0));
+                const f2 nv2 = mul2(third, fma2(I[p].wz, I[p].wz, fma2(I[p].wy, I[p].wy, mul2(I[p].wx, I[p].wx))));
+                const f2 nct = sub2(0ull, y[p][9]);
+                y[p][6] = fma2(nct, I[p].wx, fma2(nv2, y[p][0], y[p][6]));
+                y[p][7] = fma2(nct, I[p].wy, fma2(nv2, y[p][1], y[p][7]));
+                y[p][8] = fma2(nct, I[p].wz, fma2(nv2, y[p][2], y[p][8]));
+#pragma unroll
+                for (int q = 0; q < NS; ++q) {
+                    float ts[2];
+                    f2_unpack(y[p][q], ts[0], ts[1]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float sum = ksum(q, 2 * p + e), comp = kcmp(q, 2 * p + e);
+                        kahan_add(sum, comp, ts[e]);
+                        ksum(q, 2 * p + e) = sum;
+                        kcmp(q, 2 * p + e) = comp;
+                    }
                 }
             }
         }
@@ -283,7 +290,7 @@ __global__ void __launch_bounds__(PAIR_NT, 2) k_pair2_sym(const Pair2SymArgs a) 
     extern __shared__ __align__(128) unsigned char smem[];
     sym2_init(smem);
     uint32_t seq = 0;
-    sym2_block(a, blockIdx.x, blockIdx.y, smem, seq);
+    sym2_block<128>(a, blockIdx.x, blockIdx.y, smem, seq);
 }
 
 // Ensemble form, as k_pair2_ens: items (cluster, row block, range, 0), one panel per cluster.
@@ -301,7 +308,7 @@ __global__ void __launch_bounds__(PAIR_NT, 2)
         if (w >= nitems) break;
         const int4 it = items[w];
         const Pair2SymArgs a = tab[it.x];
-        if (!sym2_block(a, it.y, it.z, smem, seq)) break;
+        if (!sym2_block<64>(a, it.y, it.z, smem, seq)) break;
     }
 }
 
