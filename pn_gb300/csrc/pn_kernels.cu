@@ -315,62 +315,117 @@ __device__ __forceinline__ double sixth(double a) {
     return __fma_rn(__fma_rn(-6.0, q, a), c, q);
 }
 
-__device__ __forceinline__ void stage_update_k(const FinishArgs &a, int p, int k, double acc) {
+// What a stage reads of particle p's component k, loaded ahead of the arithmetic (the stores of one
+// component would hold back the loads of the next).
+struct StageIn {
+    double x, v, vs, hx, hv;
+};
+__device__ __forceinline__ StageIn stage_load(const FinishArgs &a, int p, int k) {
+    const size_t o = (size_t)k * a.ld + p;
+    StageIn r{a.st.x[o], a.st.v[o], 0.0, 0.0, 0.0};
+    if (a.stage != 1 && a.stage != STAGE_RK4_1) {
+        r.vs = a.st.vs[o];
+        r.hx = a.st.hx[o];
+        r.hv = a.st.hv[o];
+    }
+    return r;
+}
+__device__ __forceinline__ void stage_update_k(const FinishArgs &a, int p, int k, double acc, const StageIn &in) {
     const double dt = a.dt;
-    {
-        const size_t o = (size_t)k * a.ld + p;
-        const double x = a.st.x[o], v = a.st.v[o];
-        if (a.stage >= STAGE_RK4_1) {
-            // classic fourth-order Runge-Kutta (optional integrator; hx, hv accumulate
-            // k1 + 2 k2 + 2 k3 of the position and velocity slopes)
-            if (a.stage == STAGE_RK4_1) {
-                a.st.xs[o] = x + 0.5 * dt * v;
-                a.st.vs[o] = v + 0.5 * dt * acc;
-                a.st.hx[o] = v;
-                a.st.hv[o] = acc;
-            } else if (a.stage == STAGE_RK4_4) {
-                const double vprev = a.st.vs[o];
-                a.st.x[o] = x + (dt / 6.0) * (a.st.hx[o] + vprev);
-                a.st.v[o] = v + (dt / 6.0) * (a.st.hv[o] + acc);
-            } else {
-                const double vprev = a.st.vs[o];
-                const double f = a.stage == STAGE_RK4_2 ? 0.5 * dt : dt;
-                a.st.xs[o] = x + f * vprev;
-                a.st.vs[o] = v + f * acc;
-                a.st.hx[o] += 2.0 * vprev;
-                a.st.hv[o] += 2.0 * acc;
-            }
-        } else if (a.stage == 1) {  // :853-860
-            const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, v), dt));
-            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
-            a.st.xs[o] = x1;
-            a.st.vs[o] = v1;
-            a.st.hx[o] = x1;
-            a.st.hv[o] = v1;
-        } else if (a.stage == 2) {  // :864-871
-            const double vprev = a.st.vs[o];
-            const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, vprev), dt));
-            const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
-            a.st.xs[o] = x1;
-            a.st.vs[o] = v1;
-            a.st.hx[o] = __dadd_rn(a.st.hx[o], x1);
-            a.st.hv[o] = __dadd_rn(a.st.hv[o], v1);
-        } else {  // :875-891
-            const double vprev = a.st.vs[o];
-            const double x3 = __dadd_rn(x, __dmul_rn(vprev, dt));
-            const double v3 = __dadd_rn(v, __dmul_rn(acc, dt));
-            a.st.x[o] = sixth(__dadd_rn(__dadd_rn(x, x3), __dmul_rn(2.0, a.st.hx[o])));
-            a.st.v[o] = sixth(__dadd_rn(__dadd_rn(v, v3), __dmul_rn(2.0, a.st.hv[o])));
+    const size_t o = (size_t)k * a.ld + p;
+    const double x = in.x, v = in.v, vprev = in.vs;
+    if (a.stage >= STAGE_RK4_1) {
+        // classic fourth-order Runge-Kutta (optional integrator; hx, hv accumulate
+        // k1 + 2 k2 + 2 k3 of the position and velocity slopes)
+        if (a.stage == STAGE_RK4_1) {
+            a.st.xs[o] = x + 0.5 * dt * v;
+            a.st.vs[o] = v + 0.5 * dt * acc;
+            a.st.hx[o] = v;
+            a.st.hv[o] = acc;
+        } else if (a.stage == STAGE_RK4_4) {
+            a.st.x[o] = x + (dt / 6.0) * (in.hx + vprev);
+            a.st.v[o] = v + (dt / 6.0) * (in.hv + acc);
+        } else {
+            const double f = a.stage == STAGE_RK4_2 ? 0.5 * dt : dt;
+            a.st.xs[o] = x + f * vprev;
+            a.st.vs[o] = v + f * acc;
+            a.st.hx[o] = in.hx + 2.0 * vprev;
+            a.st.hv[o] = in.hv + 2.0 * acc;
         }
+    } else if (a.stage == 1) {  // :853-860
+        const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, v), dt));
+        const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
+        a.st.xs[o] = x1;
+        a.st.vs[o] = v1;
+        a.st.hx[o] = x1;
+        a.st.hv[o] = v1;
+    } else if (a.stage == 2) {  // :864-871
+        const double x1 = __dadd_rn(x, __dmul_rn(__dmul_rn(0.5, vprev), dt));
+        const double v1 = __dadd_rn(v, __dmul_rn(__dmul_rn(0.5, acc), dt));
+        a.st.xs[o] = x1;
+        a.st.vs[o] = v1;
+        a.st.hx[o] = __dadd_rn(in.hx, x1);
+        a.st.hv[o] = __dadd_rn(in.hv, v1);
+    } else {  // :875-891
+        const double x3 = __dadd_rn(x, __dmul_rn(vprev, dt));
+        const double v3 = __dadd_rn(v, __dmul_rn(acc, dt));
+        a.st.x[o] = sixth(__dadd_rn(__dadd_rn(x, x3), __dmul_rn(2.0, in.hx)));
+        a.st.v[o] = sixth(__dadd_rn(__dadd_rn(v, v3), __dmul_rn(2.0, in.hv)));
     }
 }
-__device__ __forceinline__ void stage_update(const FinishArgs &a, int p, const double acc3[3]) {
-    for (int k = 0; k < 3; ++k) stage_update_k(a, p, k, acc3[k]);
+
+// Star i's first NK pair sums over the j-range splits, in order, the loads of several splits in flight
+// at once (one split after the other, they were half of the kernel's time with 8 splits: N = 1,000 mixed
+// 25.6 -> 19.8 us with a cold cache).
+template <int NK>
+__device__ __forceinline__ void split_sums(const FinishArgs &a, int i, double (&S)[NACC_MAX]) {
+#pragma unroll
+    for (int k = NK; k < NACC_MAX; ++k) S[k] = 0.0;
+    if (a.accf) {  // FP32 pairs, added in FP32 without loss of their low parts
+        constexpr int U = 4;
+        const float2 *p = reinterpret_cast<const float2 *>(a.acc) + i;
+        float h[NK], l[NK];
+#pragma unroll
+        for (int k = 0; k < NK; ++k) h[k] = l[k] = 0.f;
+        for (int g = 0; g < a.gsplit; g += U) {
+            float2 t[U][NK];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < NK; ++k)
+                    t[u][k] = g + u < a.gsplit ? p[((size_t)(g + u) * a.nacc + k) * a.npad] : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < NK; ++k) pair_add(h[k], l[k], t[u][k]);
+        }
+#pragma unroll
+        for (int k = 0; k < NK; ++k) S[k] = to_f64(h[k]) + to_f64(l[k]);
+        S[A_PHI] *= X2_K * X2_K;  // the packed sweep's scale
+    } else {
+        constexpr int U = 3;
+        const double *p = a.acc + i;
+#pragma unroll
+        for (int k = 0; k < NK; ++k) S[k] = p[(size_t)k * a.npad];
+        for (int g = 1; g < a.gsplit; g += U) {
+            double t[U][NK];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < NK; ++k) t[u][k] = g + u < a.gsplit ? p[((size_t)(g + u) * a.nacc + k) * a.npad] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (g + u < a.gsplit)
+#pragma unroll
+                    for (int k = 0; k < NK; ++k) S[k] += t[u][k];
+        }
+    }
 }
 
 // Bound by its FP64 instructions (about 150 per star, 64 cycles each per warp and scheduler): one
 // warp per scheduler and block, no division per star but the reference's own q, common factors
-// R^3 and m R^3 taken out of the sums.
+// R^3 and m R^3 taken out of the sums.  Whatever it reads is loaded first: the latency of a load is
+// that of ten of them.
 __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nblk) {
     __shared__ double red[ON_NT];
     const int i = blk * ON_NT + threadIdx.x;
@@ -383,47 +438,38 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
     if (i < a.nstar) {
         const int p = i + 1;
         const double s[3] = {a.spos[i], a.spos[a.npad + i], a.spos[2 * a.npad + i]};
+        const double mi = a.m[p];
+        double v[3] = {0.0, 0.0, 0.0}, glob[NGLOB] = {0.0};
+        StageIn in[3] = {};
+        if (a.pn1) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = ld_x(a.v, a.vsp, a.vsk, p, k);
+#pragma unroll
+            for (int k = 0; k < NGLOB; ++k) glob[k] = G[k];
+        }
+        if (a.stage)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) in[k] = stage_load(a, p, k);
         const double q = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
         const double R = rsqrt(q + eps2);
         const double R3 = R * R * R;
-        const double mi = a.m[p];
         // the force slots only (a fused-energy sweep has one more, read by the energy kernel)
         const int nk = a.nacc < NACC_MAX ? a.nacc : NACC_MAX;
         double S[NACC_MAX];
-        if (a.accf) {  // FP32 pairs, added in FP32 without loss of their low parts
-            const float2 *p = reinterpret_cast<const float2 *>(a.acc) + i;
-            float h[NACC_MAX], l[NACC_MAX];
-#pragma unroll
-            for (int k = 0; k < NACC_MAX; ++k) h[k] = l[k] = 0.f;
-#pragma unroll 4
-            for (int g = 0; g < a.gsplit; ++g)
-#pragma unroll
-                for (int k = 0; k < NACC_MAX; ++k)
-                    if (k < nk) pair_add(h[k], l[k], p[((size_t)g * a.nacc + k) * a.npad]);
-#pragma unroll
-            for (int k = 0; k < NACC_MAX; ++k) S[k] = to_f64(h[k]) + to_f64(l[k]);
-            S[A_PHI] *= X2_K * X2_K;  // the packed sweep's scale
-        } else {
-#pragma unroll
-            for (int k = 0; k < NACC_MAX; ++k) S[k] = k < nk ? a.acc[(size_t)k * a.npad + i] : 0.0;
-#pragma unroll 2
-            for (int g = 1; g < a.gsplit; ++g)
-#pragma unroll
-                for (int k = 0; k < NACC_MAX; ++k)
-                    if (k < nk) S[k] += a.acc[((size_t)g * a.nacc + k) * a.npad + i];
-        }
+        if (nk == NACC_MAX) split_sums<NACC_MAX>(a, i, S);
+        else split_sums<3>(a, i, S);
         if (a.sums_out)
-            for (int k = 0; k < nk; ++k) a.sums_out[(size_t)k * a.npad + i] = S[k];
+#pragma unroll
+            for (int k = 0; k < NACC_MAX; ++k)
+                if (k < nk) a.sums_out[(size_t)k * a.npad + i] = S[k];
         const double Gv[3] = {S[A_GX], S[A_GY], S[A_GZ]};
         double acc3[3];
         const double mb = m0 * R3;
         for (int k = 0; k < 3; ++k) acc3[k] = fma(-mb, s[k], Gv[k]);  // Newton incl. BH column
         if (a.pn1) {
-            const double v[3] = {ld_x(a.v, a.vsp, a.vsk, p, 0), ld_x(a.v, a.vsp, a.vsk, p, 1),
-                                 ld_x(a.v, a.vsp, a.vsk, p, 2)};
-            const double P[3] = {G[G_PX], G[G_PY], G[G_PZ]};
-            const double B3[3] = {G[G_B3X], G[G_B3Y], G[G_B3Z]};
-            const double A1 = G[G_A1], C = G[G_C];
+            const double P[3] = {glob[G_PX], glob[G_PY], glob[G_PZ]};
+            const double B3[3] = {glob[G_B3X], glob[G_B3Y], glob[G_B3Z]};
+            const double A1 = glob[G_A1], C = glob[G_C];
             const double Phi = S[A_PHI], S0 = S[A_S0], U = S[A_U];
             const double W[3] = {S[A_WX], S[A_WY], S[A_WZ]};
             const double vi2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
@@ -464,21 +510,25 @@ __device__ __forceinline__ void finish_body(const FinishArgs &a, int blk, int nb
             if (!isfinite(acc3[k])) bad = true;
             if (a.a) a.a[(long long)p * a.asp + (long long)k * a.ask] = acc3[k];
         }
-        if (a.stage) stage_update(a, p, acc3);
+        if (a.stage)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) stage_update_k(a, p, k, acc3[k], in[k]);
     }
     if (bad) atomicOr(a.err, DEVERR_NONFINITE);
     const double r = block_sum<4>(bh, red);
     if (threadIdx.x < 4) a.part[(size_t)blk * 4 + threadIdx.x] = r;
     if (last_block(a.ticket, nblk)) {
+        const int k = threadIdx.x;
+        StageIn in{};
+        if (a.stage && k < 3) in = stage_load(a, 0, k);
         const double t = partials_sum<4>(nblk, 0.0, red, [](double u, double w) { return u + w; },
                                          [&](int b, int k) { return __ldcg(&a.part[(size_t)b * 4 + k]); });
         // BH: Newtonian pull of the stars (:36-51, row 0) plus the 1PN sum; thread k < 3 holds component k
-        const int k = threadIdx.x;
         if (k < 3) {
             const double acc = a.pn1 ? fma(ic2, t, G[G_B3X + k]) : G[G_B3X + k];
             if (!isfinite(acc)) atomicOr(a.err, DEVERR_NONFINITE);
             if (a.a) a.a[(long long)k * a.ask] = acc;
-            if (a.stage) stage_update_k(a, 0, k, acc);
+            if (a.stage) stage_update_k(a, 0, k, acc, in);
         }
         if (k == 0) {
             if (a.fix_bad) *a.fix_bad = 0;
