@@ -681,6 +681,8 @@ def headline(args, rank, world, dist):
         line["fp64"] = {"value": inter_step / (sm64[0] * 1e-3), "unit": UNIT,
                         "ms_per_step": float(sm64[0]),
                         "peak_fp64_tflops": pn.probe_fma_peak(pn.PN_PREC_FP64),
+                        # (70 flops per pair of the FP64 form; the default sweep forms the terms in fixed point
+                        # on the integer pipes, so this may exceed the FP64 peak)
                         "pair_tflops": float(ns) * ns * pn.flops_per_pair(1, 0) / (pm64[0] / 3 * 1e-3) / 1e12}
         line["mixed_over_fp64"] = value / world / line["fp64"]["value"]
         acc = {}

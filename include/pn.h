@@ -51,7 +51,8 @@ typedef enum {
 } pn_status;
 
 typedef enum {
-    PN_PREC_FP64 = 0,  /* every pair term in FP64: parity with the reference */
+    PN_PREC_FP64 = 0,  /* pair terms to FP64 accuracy (in fixed point where the system's range allows
+                          it, else in FP64), the rest in FP64: parity with the reference */
     PN_PREC_MIXED = 1  /* FP32 pair terms (per-tile FP64 origin, compensated sums), FP64 rest */
 } pn_precision;
 

@@ -8,13 +8,13 @@
 // for the sums themselves, which are added to FP64 totals in shared memory at the tile's end.
 //
 // Why: FP64 issues one warp instruction per 64 cycles and scheduler here and k_pair<double>'s 51 per
-// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 725 and is bound by the
-// multiply-add pipe, beside the FP64 pipe's 6 operations per pair. One force evaluation at
-// N = 65,536: 385 -> 77.3 ms, N = 10,000: 9.3 -> 2.0 ms.  Its error against long double sums is below
+// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 672, of which the
+// multiply-add pipe is busy 71 % and the FP64 pipe 59 % (6 operations per pair). One force evaluation at
+// N = 65,536: 385 -> 71.7 ms, N = 10,000: 9.3 -> 1.85 ms.  Its error against long double sums is below
 // the FP64 sweep's (medians at N = 2,049: 1.46e-16 against 2.22e-16 at c = 1000, 5.2e-16 against
 // 7.4e-16 at c = 1).  Measured on the way there, at N = 65,536: every product in integers and C's sum
 // in FP64 (4 conversions and 5 FMA per pair) 104 ms; the dot products' small parts in FP32, Phi and U in
-// FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms; the sums' small parts in FP32
+// FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms, carry additions 71.7 ms; the sums' small parts in FP32
 // too (before that) 76 against 88 ms, but with twice the FP64 sweep's error at c = 1.
 //
 // The integer range covers the systems that k_prep has checked star by star (positions within

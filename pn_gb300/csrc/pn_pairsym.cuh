@@ -26,7 +26,7 @@
 // one system (N = 8,100 to 32,767, inv_c2 = 1e-6; 0.75 to 0.85 at 1); for ensembles of 128 to 4,000 stars
 // the error of the whole vector is 0.95 of k_pair2's in the mean (with 128 terms it was 1.15 of it).
 //
-// Bound by the FP32 FMA pipe (71 % active at N = 16,384) and, with two warps per scheduler, by the latency
+// Bound by the FP32 FMA pipe (75 % active at N = 16,384) and, with two warps per scheduler, by the latency
 // between its instructions.  Per step of a warp that pipe takes 300 cycles, the shared-memory pipe of
 // the SM 144 (16 wavefronts of loads and 20 shuffles for each of four warps): with half the rows it
 // would be the limit.  Measured at N = 65,536: stars as pairs of equal values in shared memory (twice the
