@@ -134,13 +134,24 @@ static int cluster_gsplit(const pn_ens *e, int c) {
 // Tables and work items of the sweep over unordered pairs; false (and the packed sweep) where its
 // partial sums would take more than SYM_ENS_BYTES or there is no memory for them.  Tiles per item as for
 // one system (pn_api.cu, choose_sym), over the work of all clusters.
+// Small clusters leave most of a 512-star row block empty and few tiles that serve both sides, so the
+// packed sweep keeps them: compared by operations per 256 stars and tile (25 packed there; here 102 for 512
+// rows in both orders, 150 for both sides) over the share of the FMA pipe that each sweep keeps busy (85 and
+// 73 %), unless the packed sweep's items are fewer than the SMs.  Measured (us per step, packed and this one):
+// 200 clusters of 400 stars 571 / 634, 100 of 1,000 861 / 933, 60 of 1,500 1,126 / 1,061, 40 of 2,500 1,733 /
+// 1,691, 16 of 5,000 3,103 / 2,298, 4 of 1,000 669 / 276.
 constexpr size_t SYM_ENS_BYTES = (size_t)2 << 30;
 static bool ens_build_sym(pn_ens *e) {
-    long long units = 0;
+    long long units = 0, packed_items = 0;
+    double cost = 0.0, packed = 0.0;
     for (int c = 0; c < e->nc; ++c) {
-        const long long nt = (e->n[c] + 126) / 128, nb = (nt + 3) / 4;
-        units += nb * nt - 2 * nb * (nb - 1);
+        const long long nt = (e->n[c] + 126) / 128, nb = (nt + 3) / 4, u = nb * nt - 2 * nb * (nb - 1);
+        units += u;
+        cost += (51.0 * nt + 75.0 * (u - nt)) / 0.73;  // (every tile is once a tile of its own rows)
+        packed += 25.0 * (double)((nt + 1) / 2 * nt) / 0.85;
+        packed_items += (nt + 1) / 2 * cluster_gsplit(e, c);
     }
+    if (cost >= packed && packed_items >= e->sms) return false;
     const int chunk = (int)std::min<long long>(8, std::max<long long>(1, (units + 12 * e->sms - 1) / (12 * e->sms)));
     size_t bytes = 0;
     for (int c = 0; c < e->nc; ++c) bytes += sym_ens_bytes(e->n[c] - 1, chunk);
