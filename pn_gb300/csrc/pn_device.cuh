@@ -155,6 +155,12 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// Orders this thread's ordinary accesses of shared memory before later bulk copies to the same place
+// (which a barrier alone does not: the copies are another proxy's).  Every thread that stored into a stage
+// calls it, ahead of the barrier after which the stage is refilled.
+__device__ __forceinline__ void fence_before_bulk() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),

@@ -152,6 +152,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                 const B2 wx = slower(g5.x, g5.y, sft), wy = slower(g5.z, g5.w, sft), wz = slower(g6.x, g6.y, sft);
                 q[0] = make_uint4((unsigned)wx.h, (unsigned)wx.l, (unsigned)wy.h, (unsigned)wy.l);
                 q[TJ] = make_uint4((unsigned)wz.h, (unsigned)wz.l, g6.z, g6.w);
+                fence_before_bulk();  // (the stage is refilled by a bulk copy)
                 __syncthreads();
             }
         }
