@@ -256,6 +256,12 @@ int pn::ensure_acc(pn_ctx *c, int splits) {
     return PN_OK;
 }
 
+// Room for the partial sums of every sweep at this size, whichever runs first: a force evaluation that a caller
+// has captured holds the buffer's address, so a later energy must not move it.
+static int ensure_sums(pn_ctx *c) {
+    return ensure_acc(c, std::max({acc_splits(c->cfg_force), c->cfg_energy.gsplit, c->cfg_fused.gsplit}));
+}
+
 // Room for the partial sums of the sweep over unordered pairs; the packed sweep takes its place where
 // there is none.
 void pn::ensure_sym(pn_ctx *c) {
@@ -424,7 +430,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     ensure_sym(c);
     const PairCfg &k = with_energy ? c->cfg_fused : c->cfg_force;
     const bool sym = is_f32(c) && k.x2 == 4;
-    int rc = ensure_acc(c, acc_splits(k));
+    int rc = ensure_sums(c);
     if (rc) return rc;
     const double eps2 = c->p.eps * c->p.eps;
 
@@ -624,9 +630,8 @@ static int build_step_graph(pn_ctx *c, bool timed = false) {
     if (valid) return PN_OK;
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     refresh_cfg(c);
-    // allocate before capture, for the energy sweep too (a later allocation would make the step stale)
-    ensure_sym(c);
-    int rc = ensure_acc(c, std::max({acc_splits(c->cfg_force), c->cfg_energy.gsplit, c->cfg_fused.gsplit}));
+    ensure_sym(c);  // (allocated before capture)
+    int rc = ensure_sums(c);
     if (rc) return rc;
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -809,7 +814,7 @@ static int enqueue_energy(pn_ctx *c, const double *x, const double *v, const dou
     const int nstar = c->n - 1;
     refresh_cfg(c);
     const PairCfg &k = c->cfg_energy;
-    int rc = ensure_acc(c, k.gsplit);
+    int rc = ensure_sums(c);
     if (rc) return rc;
     const double eps2 = c->p.eps * c->p.eps;
     cudaStream_t s = c->stream;
