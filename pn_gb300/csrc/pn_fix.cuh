@@ -273,6 +273,18 @@ PNF int speed_exp(double v2) {
     return be == 0 || e < -EV_MAX ? -EV_MAX : e;
 }
 
+// Whether the sweep covers a star of mass m at s with |v|^2 = v2 beside a BH of mass m0 (a star outside sends the
+// whole system to the FP64 sweep): |s| < 2^POS_BITS in units, speeds below 2^EV_MAX and (for the FP32 sums of C's
+// magnitudes) |v|^2 below 2^60 m0 / 2^eL, the star's mass 0 or 2^-32 .. 2^59 of the BH's, whose own is positive;
+// infinities and NaN are outside.
+PNF bool in_range(const double *s, double v2, double m, double m0, int eL) {
+    auto e = [](double x) { return (int)((bits_of(x) >> 52) & 0x7ff); };
+    const int e0 = expo(m0);
+    bool in = !(bits_of(m0) >> 63) && e(m0) > 60 && e(m0) < 1986 && e(v2) < 1023 + 2 * EV_MAX - 10 && e(v2) < 1023 + 60 + e0 - eL;
+    for (int k = 0; k < 3; ++k) in = in && e(s[k]) < 1023 + POS_BITS + eL;
+    return in && !(bits_of(m) >> 63) && (m == 0.0 || (e(m) >= 1023 + e0 - 32 && e(m) < 1023 + e0 + 59));
+}
+
 // ------------------------------------------------------------------ one pair
 enum : int { F_NEWTON = 0, F_FORCE = 1, F_ENERGY = 2, F_FORCE_ENERGY = 3 };  // as PairMode
 

@@ -114,12 +114,7 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     using namespace fix;
     const FixUnits &u = a.fu;
     const int e0 = expo(m0);
-    auto ebits = [](double d) { return (__double2hiint(d) >> 20) & 0x7ff; };  // 0x7ff: not finite
-    bool in = ebits(m0) > 60 && ebits(m0) < 1986 && ebits(v2) < 1023 + 2 * EV_MAX - 10 &&
-              ebits(v2) < 1023 + 60 + e0 - u.eL;  // (|v|^2 beside the FP32 range of g1f)
-    for (int k = 0; k < 3; ++k) in = in && ebits(s[k]) < 1023 + POS_BITS + u.eL;
-    // m: 0, or 2^-32 .. 2^59 of m0
-    in = in && (__double2hiint(m) >= 0) && (m == 0.0 || (ebits(m) >= 1023 + e0 - 32 && ebits(m) < 1023 + e0 + 59));
+    const bool in = in_range(s, v2, m, m0, u.eL);
     if (real && !in) atomicOr(a.fix_bad, 1);
     if (!in) return;
     float hi[3], lo[3];
