@@ -49,7 +49,8 @@ typedef unsigned long long u64;
 
 // limits of the fixed-point range (host constants of the units, checked per star by k_prep)
 constexpr int POS_BITS = 24;   // |s| / 2^eL < 2^24 (the FP32 seed then stays within 2^-20)
-constexpr int EV_MAX = 300;    // speeds below 2^300 (slower ones than 2^-300 count as at rest)
+constexpr int EV_MAX = 200;    // speeds below 2^200 (slower ones than 2^-200 count as at rest)
+constexpr int E0_MAX = 300;    // the BH's mass within 2^-300 .. 2^300
 constexpr double W_SCALE = 1.7320508075688772935;  // w / v
 constexpr u64 W_MANT = 0xDDB3D742C265539DULL;      // sqrt(3) 2^63
 constexpr u64 U_MANT = 0x93CD3A2C8198E269ULL;      // 4 / sqrt(3) 2^62
@@ -275,12 +276,19 @@ PNF int speed_exp(double v2) {
 
 // Whether the sweep covers a star of mass m at s with |v|^2 = v2 beside a BH of mass m0 (a star outside sends the
 // whole system to the FP64 sweep): |s| < 2^POS_BITS in units, speeds below 2^EV_MAX and (for the FP32 sums of C's
-// magnitudes) |v|^2 below 2^60 m0 / 2^eL, the star's mass 0 or 2^-32 .. 2^59 of the BH's, whose own is positive;
-// infinities and NaN are outside.
+// magnitudes) |v|^2 below 2^60 m0 / 2^eL, the star's mass 0 or 2^-32 .. 2^59 of the BH's, whose own is positive
+// and within 2^-E0_MAX .. 2^E0_MAX; infinities and NaN are outside.
+// The units of a tile's integer sums are then powers of two that a double holds (the sweep's pow2): with the BH's mass
+// about 2^e0, |e0| <= 300, |eL| <= 60, a tile's FP32 sum of m Q^2 below 2^67 (2^-126 stands for none), -200 <= ev
+// and ev < 200, their exponents lie within
+//   G, S0      e0 - 2 eL - 188 .. e0 - 3 eL + 7          -608 .. 487
+//   C + H      2 e0 - 3 eL - 187 .. 2 e0 - 3 eL + 67     -967 .. 847
+//   ct, ct w   e0 - 2 eL - 200 + 2 ev .. e0 - 2 eL + 5 + 2 ev    -1020 .. 825
 PNF bool in_range(const double *s, double v2, double m, double m0, int eL) {
     auto e = [](double x) { return (int)((bits_of(x) >> 52) & 0x7ff); };
     const int e0 = expo(m0);
-    bool in = !(bits_of(m0) >> 63) && e(m0) > 60 && e(m0) < 1986 && e(v2) < 1023 + 2 * EV_MAX - 10 && e(v2) < 1023 + 60 + e0 - eL;
+    bool in = !(bits_of(m0) >> 63) && e0 >= -E0_MAX && e0 <= E0_MAX && e(v2) < 1023 + 2 * EV_MAX - 10 &&
+              e(v2) < 1023 + 60 + e0 - eL;
     for (int k = 0; k < 3; ++k) in = in && e(s[k]) < 1023 + POS_BITS + eL;
     return in && !(bits_of(m) >> 63) && (m == 0.0 || (e(m) >= 1023 + e0 - 32 && e(m) < 1023 + e0 + 59));
 }

@@ -71,3 +71,17 @@ def test_negative_bh_mass(pn, ic2):
     x[7] = x[0] + 1e-3
     m[0] = -m[0]
     _same(_device(pn, x, v, m, ic2), _device(pn, x, v, m, ic2, **FP64))
+
+
+@pytest.mark.parametrize("mass,length", [(-500, 0), (-340, 50), (340, -50), (480, 0), (-294, -54), (-294, 66),
+                                         (-290, 0), (290, 0), (306, 66), (306, -54)])
+def test_extreme_units(pn, mass, length):
+    """Units far from 1 (masses and lengths times powers of two), inside the range and outside."""
+    x, v, m = _system(300, 13)
+    x[5] = x[0] + 1e-4
+    v[1:129] *= 1e-3
+    s = 2.0 ** ((mass - length) // 2)
+    a, b = (_device(pn, x * 2.0 ** length, v * s, m * 2.0 ** mass, 1e-2 / s ** 2, eps=EPS * 2.0 ** length, **kw)
+            for kw in ({}, FP64))
+    assert np.isfinite(b).all() and np.abs(b).max() > 0
+    _same(a, b)

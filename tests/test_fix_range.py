@@ -27,3 +27,29 @@ def test_signs_and_values(inside):
     assert inside(m=0.02 * 2.0 ** -31) and not inside(m=0.02 * 2.0 ** -33)
     assert inside(m=0.02 * 2.0 ** 57) and not inside(m=0.02 * 2.0 ** 60)
     assert inside(s=(2.0 ** 17.9, 0, 0)) and not inside(s=(2.0 ** 18.1, 0, 0))
+
+
+def test_units_that_a_double_holds(inside):
+    """The exponents of a tile's sums (the kernel's formulas) at the limits that the check lets through."""
+    def largest(ok, lo, hi):  # the last k from lo on towards hi that is inside
+        step = 1 if hi > lo else -1
+        k = lo
+        while k != hi and ok(k + step):
+            k += step
+        return k
+
+    def star(e0, eL, k):  # at rest next to the BH, of the BH's mass, v^2 = 2^k
+        return inside(m0=2.0 ** e0, m=2.0 ** e0, v2=2.0 ** k, s=(2.0 ** (eL - 3), 0, 0), eL=eL)
+
+    for eL in (-60, 0, 60):
+        lo = largest(lambda e: star(e, eL, -1000), 0, -1000)
+        hi = largest(lambda e: star(e, eL, -1000), 0, 1000)
+        for e0 in (lo, hi):
+            ev = largest(lambda k: star(e0, eL, k), -1000, 1000) // 2 + 2
+            for e in (ev, -200):  # the fastest star, one at rest
+                for g in (-126, 67):  # exponent of a tile's sum of m Q^2: none, the heaviest
+                    gn = g + e0 - 2 * eL
+                    h = g + e0 - 2 * eL + 2 + 2 * e
+                    units = [gn - 62, gn - eL - 60, gn + 2 - 2 - 62 + 2 * e, gn + 2 - 14 - 62 + 2 * e, gn + 2 - 14 - 62 + e]
+                    units += [max(c + 2 * e0 - 3 * eL, h - lift) + 1 - 62 for c in (-126, 128) for lift in (2, 18)]
+                    assert min(units) >= -1022 and max(units) <= 1023, (e0, eL, e, g, units)
