@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "pn_ctx.h"
+#include "pn_fix.cuh"
 #include "pn_tune.h"
 
 using namespace pn;
@@ -85,7 +86,7 @@ extern "C" void pn_params_default(pn_params *p) {
 bool pn::is_f32(const pn_ctx *c) { return c->p.precision == PN_PREC_MIXED; }
 int pn::force_mode(const pn_ctx *c) { return c->p.inv_c2 != 0.0 ? MODE_FORCE : MODE_NEWTON; }
 
-bool pn::fix_units(double eps, FixUnits *u) {
+bool pn::fix_units(double eps, double inv_c2, FixUnits *u) {
     *u = FixUnits{};
     if (!std::isfinite(eps)) return false;
     u->eL = std::ilogb(eps);
@@ -95,6 +96,7 @@ bool pn::fix_units(double eps, FixUnits *u) {
     u->inv_len = std::ldexp(1.0, -u->eL);
     u->inv_eps = 1.0 / eps;
     u->inv_eps3 = (double)(1.0L / ((long double)eps * eps * eps));
+    u->ev_max = fix::velocity_limit(inv_c2);
     return true;
 }
 
@@ -187,7 +189,7 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
     const int pv = c->p.pair_variant;
     PairCfg tuned;
     FixUnits fu;
-    const bool fix = !f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, &fu);
+    const bool fix = !f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, c->p.inv_c2, &fu);
     // (an FP64 shape tuned for the other of its two sweeps does not apply: 3.5 to 4.5 times slower, or
     // outside the fixed-point one's range)
     if (!explicit_shape && pv == PN_PAIR_AUTO && nstar > 0 &&
@@ -448,7 +450,7 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
         if (k.x2) pa.pack = nullptr;  // the packed sweep reads the paired pack only
     }
     FixUnits fu{};
-    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
+    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, c->p.inv_c2, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
     if (!pa.f32 && k.x2) { pa.fpack = c->fpack; pa.fix_bad = c->fix_bad; pa.fu = fu; }
     pa.part = c->part; pa.glob = c->glob; pa.ticket = &c->tickets[0];
     CU(launch_prep(pa, s));
@@ -825,7 +827,7 @@ static int enqueue_energy(pn_ctx *c, const double *x, const double *v, const dou
     pa.pack = c->pack; pa.torg = c->torg; pa.spos = c->spos;
     if (pa.f32) { pa.pack2 = c->pack2; pa.ipack = c->ipack; }
     FixUnits fu{};
-    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
+    if (!pa.f32 && k.x2 && !fix_units(c->p.eps, c->p.inv_c2, &fu)) return set_err(PN_ERR_STATE, "fixed-point units");
     if (!pa.f32 && k.x2) { pa.fpack = c->fpack; pa.fix_bad = c->fix_bad; pa.fu = fu; }
     pa.part = c->part; pa.glob = c->glob; pa.ticket = &c->tickets[0];
     CU(launch_prep(pa, s));
@@ -1203,7 +1205,7 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
     refresh_cfg(c);
     const bool f32 = is_f32(c);
     FixUnits fu;
-    const bool fix = !f32 && fix_units(c->p.eps, &fu);
+    const bool fix = !f32 && fix_units(c->p.eps, c->p.inv_c2, &fu);
     const int modes[2] = {force_mode(c), MODE_ENERGY};
     for (int which = 0; which < 2; ++which) {
         if (!(sweeps & (1 << which))) continue;

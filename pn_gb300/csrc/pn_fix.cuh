@@ -274,23 +274,36 @@ PNF int speed_exp(double v2) {
     return be == 0 || e < -EV_MAX ? -EV_MAX : e;
 }
 
+// The largest velocity unit 2^ev of a system whose 1PN terms have the weight inv_c2: inv_c2 4^ev <= 64, which every
+// speed up to that of light is within (and up to 2.8 times it at inv_c2 = 1).  The velocity terms' rounding, 2^-58 of
+// the unit's square and 2^-55 of the unit times the star's own speed for each m Q^2, does not shrink with
+// the slow stars of a tile that holds a fast one.
+// Median errors of W over sum m Q^2 |n| of 128 stars of speeds about 0.3 and one light fast one, in units of 2^-53
+// (inv_c2 = 1; here and in FP64): speed 1: 0.50, 0.70; 2.8: 1.3, 0.80; 11: 6.8, 1.0; 45: 124, 0.4; 300: 6,100, 0.4.
+inline int velocity_limit(double inv_c2) {
+    if (!(inv_c2 > 0.0)) return EV_MAX;  // (no velocity terms)
+    const double lim = 64.0 / inv_c2;
+    const int e = lim > 0.0 ? __builtin_ilogb(lim) >> 1 : -EV_MAX - 1;
+    return e < EV_MAX ? e : EV_MAX;
+}
+
 // Whether the sweep covers a star of mass m at s with |v|^2 = v2 beside a BH of mass m0 (a star outside sends the
 // whole system to the FP64 sweep): |s| < 2^POS_BITS in units, speeds below 2^EV_MAX and (for the FP32 sums of C's
-// magnitudes) |v|^2 below 2^60 m0 / 2^eL, the star's mass 0 or 2^-32 .. 2^59 of the BH's, whose own is positive
-// and within 2^-E0_MAX .. 2^E0_MAX; infinities and NaN are outside.
+// magnitudes) |v|^2 below 2^60 m0 / 2^eL, the star's mass 0 or 2^-32 .. 2^59 of the BH's, the speed within
+// velocity_limit, the BH's mass positive and within 2^-E0_MAX .. 2^E0_MAX; infinities and NaN are outside.
 // The units of a tile's integer sums are then powers of two that a double holds (the sweep's pow2): with the BH's mass
 // about 2^e0, |e0| <= 300, |eL| <= 60, a tile's FP32 sum of m Q^2 below 2^67 (2^-126 stands for none), -200 <= ev
 // and ev < 200, their exponents lie within
 //   G, S0      e0 - 2 eL - 188 .. e0 - 3 eL + 7          -608 .. 487
 //   C + H      2 e0 - 3 eL - 187 .. 2 e0 - 3 eL + 67     -967 .. 847
 //   ct, ct w   e0 - 2 eL - 200 + 2 ev .. e0 - 2 eL + 5 + 2 ev    -1020 .. 825
-PNF bool in_range(const double *s, double v2, double m, double m0, int eL) {
+PNF bool in_range(const double *s, double v2, double m, double m0, int eL, int ev_max) {
     auto e = [](double x) { return (int)((bits_of(x) >> 52) & 0x7ff); };
     const int e0 = expo(m0);
     bool in = !(bits_of(m0) >> 63) && e0 >= -E0_MAX && e0 <= E0_MAX && e(v2) < 1023 + 2 * EV_MAX - 10 &&
               e(v2) < 1023 + 60 + e0 - eL;
     for (int k = 0; k < 3; ++k) in = in && e(s[k]) < 1023 + POS_BITS + eL;
-    return in && !(bits_of(m) >> 63) && (m == 0.0 || (e(m) >= 1023 + e0 - 32 && e(m) < 1023 + e0 + 59));
+    return in && speed_exp(v2) <= ev_max && !(bits_of(m) >> 63) && (m == 0.0 || (e(m) >= 1023 + e0 - 32 && e(m) < 1023 + e0 + 59));
 }
 
 // ------------------------------------------------------------------ one pair

@@ -30,8 +30,8 @@ cudaError_t launch_pair_f64(int mode, const PairCfg &c, const PairArgs &a, cudaS
 // tiles of 128.
 cudaError_t launch_pair_fix(int mode, const PairCfg &c, const PairArgs &a, cudaStream_t s);
 constexpr int FIX_GROUPS = 13;  // 16-byte groups per star of its pack
-// Its units for a softening; false where its range does not cover it.
-bool fix_units(double eps, FixUnits *u);
+// Its units for a softening and a weight of the 1PN terms; false where its range does not cover the softening.
+bool fix_units(double eps, double inv_c2, FixUnits *u);
 bool pair_shape_supported(int ipt, int js);
 // The mixed force sweep over unordered pairs (PairCfg::x2 = 4; pn_pair_sym.cu), whose partial sums take
 // sym_bytes of work, at most SYM_PANEL_BYTES (or one panel of 4 tiles).

@@ -114,7 +114,7 @@ __device__ __forceinline__ void prep_fix(const PrepArgs &a, int j, bool real, co
     using namespace fix;
     const FixUnits &u = a.fu;
     const int e0 = expo(m0);
-    const bool in = in_range(s, v2, m, m0, u.eL);
+    const bool in = in_range(s, v2, m, m0, u.eL, u.ev_max);
     if (real && !in) atomicOr(a.fix_bad, 1);
     if (!in) return;
     float hi[3], lo[3];

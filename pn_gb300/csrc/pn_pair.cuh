@@ -32,9 +32,9 @@ template <> struct PackVec<float> { using V = float4; };
 template <> struct PackVec<double> { using V = double2; };
 
 // Units of the fixed-point sweep (pn_fix.cuh): lengths 2^eL; eps60 = eps^2 in them with 60 fraction
-// bits; inv_len = 2^-eL; inv_eps, inv_eps3 = 1 / eps, 1 / eps^3.
+// bits; inv_len = 2^-eL; inv_eps, inv_eps3 = 1 / eps, 1 / eps^3; ev_max: the largest velocity unit.
 struct FixUnits {
-    int eL;
+    int eL, ev_max;
     unsigned long long eps60;
     double inv_len, inv_eps, inv_eps3;
 };

@@ -85,3 +85,14 @@ def test_extreme_units(pn, mass, length):
             for kw in ({}, FP64))
     assert np.isfinite(b).all() and np.abs(b).max() > 0
     _same(a, b)
+
+
+@pytest.mark.parametrize("speed", [0.5, 3.0, 10.0, 30.0, 1e2, 1e3, 1e4, 1e5])
+def test_one_fast_star(pn, speed):
+    """One light star far faster than the rest, and than c: the slow rows keep their velocity sums."""
+    x, v, m = _system(300, 17)
+    m[40] = m[0] * 2.0 ** -31
+    v[40] = speed * np.array([0.6, 0.0, 0.8])
+    new, old = (_run(pn, x, v, m, 1.0, **kw) for kw in ({}, FP64))
+    assert relerr(new[0], old[0]).max() <= 1e-12
+    assert np.abs(new[1] - old[1]).max() <= 1e-12 * np.abs(old[1]).max()
