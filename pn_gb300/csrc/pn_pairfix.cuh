@@ -17,6 +17,12 @@
 // FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms, carry additions 71.7 ms; the sums' small parts in FP32
 // too (before that) 76 against 88 ms, but with twice the FP64 sweep's error at c = 1.
 //
+// n = d Q has an absolute error of 2^-61, whatever d: G's is up to 2^-61 sum m Q^2, where FP64's is about 2^-53 of
+// the terms, sum m Q^2 |n|.  So a row whose stars (of its j-range, weighted by m Q^2) lie so far inside the softening
+// that the mean of |n|^2 may be below 1 / 128 is formed once more in FP64, by the whole CTA, before it leaves: two
+// stars 1e-8 eps apart and alone kept 5e-11 of their force without that.  For one such pair to dominate a
+// row its stars have to be within 0.13 eps; of N = 65,536 stars at eps = 0.04 / N^(1/3), one in a hundred systems has one.
+//
 // The integer range covers the systems that k_prep has checked star by star (positions within
 // 2^24 eps, masses zero or 2^-32 .. 2^59 of the BH's, all finite); for any other
 // the same launch runs k_pair<double>'s block instead.
@@ -28,6 +34,8 @@
 namespace pn {
 
 constexpr int FIX_TJ = 128;
+// Rows with sum m Q^2 |n|^2 < sum m Q^2 / NEAR go to FP64 (fix_row_fp64).
+constexpr float NEAR = 128.f;
 
 template <int MODE> struct FixInfo {
     static constexpr int NG = MODE == MODE_NEWTON ? 5 : MODE == MODE_ENERGY ? 8 : 11;  // streamed 16-byte groups
@@ -37,7 +45,7 @@ template <int MODE> struct FixInfo {
 
 template <int MODE>
 __host__ __device__ constexpr size_t fix_tot_bytes() {
-    return (size_t)FixInfo<MODE>::NT * PAIR_NT * sizeof(double);
+    return (size_t)PAIR_NT * (FixInfo<MODE>::NT * sizeof(double) + sizeof(float));
 }
 template <int MODE>
 inline size_t fix_smem_bytes() {
@@ -56,6 +64,43 @@ __device__ __forceinline__ int mag_exp(float x) {
 }
 __device__ __forceinline__ double pow2(int e) {  // 2^e, -1022 <= e <= 1023
     return __hiloint2double((e + 1023) << 20, 0);
+}
+
+// Row i's sums with the stars j0 .. j1 - 1 in FP64, by the whole CTA, to out[slot * npad].  red: 4 NACC doubles of
+// shared memory.
+template <int MODE>
+__device__ __noinline__ void fix_row_fp64(const double2 *pk, int npad, int i, int j0, int j1, double eps2, double *red,
+                                          double *out) {
+    constexpr int NACC = ModeInfo<MODE>::NACC;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto grp = [&](int g, int j) { return pk[(size_t)g * npad + j]; };
+    IState<double> I{};
+    I.ex = grp(0, i).x;
+    I.ey = grp(0, i).y;
+    I.ez = grp(1, i).x;
+    I.vx = grp(2, i).x;
+    I.vy = grp(2, i).y;
+    I.vz = grp(3, i).x;
+    I.qe = grp(5, i).y;
+    I.vi2 = pn_fma(I.vz, I.vz, pn_fma(I.vy, I.vy, I.vx * I.vx));
+    double acc[NACC];
+#pragma unroll
+    for (int q = 0; q < NACC; ++q) acc[q] = 0.0;
+#pragma unroll 1
+    for (int j = j0 + tid; j < j1; j += PAIR_NT) {
+        const double2 g0 = grp(0, j), g1 = grp(1, j), g2 = grp(2, j), g3 = grp(3, j), g4 = grp(4, j), g5 = grp(5, j);
+        pair_accumulate<MODE, double>(acc, I, g0.x, g0.y, g1.x, 0.0, 0.0, 0.0, g1.y, g2.x, g2.y, g3.x, g3.y, g4.x, g4.y,
+                                      g5.x, eps2);
+    }
+#pragma unroll
+    for (int q = 0; q < NACC; ++q) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
+        if (lane == 0) red[warp * NACC + q] = acc[q];
+    }
+    __syncthreads();
+    if (tid < NACC) out[(size_t)tid * npad] = (red[tid] + red[NACC + tid]) + (red[2 * NACC + tid] + red[3 * NACC + tid]);
+    __syncthreads();  // red is free again
 }
 
 template <int MODE, int JS>
@@ -108,6 +153,9 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         sl[k] = (float)(s - (double)sh[k]);
     }
     Sums A;
+    // sum of m Q^2 (units; without S0, of m Q^2 (1 - NEAR |n|^2)) over this lane's stars
+    float &near = reinterpret_cast<float *>(tot + FixInfo<MODE>::NT * NT)[tid];
+    near = 0.f;
     if (sub == 0)
 #pragma unroll
         for (int q = 0; q < FixInfo<MODE>::NT; ++q) tot[q * NT + grp] = 0.0;
@@ -176,7 +224,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
         // ---- the tile's sums in FP32: their exponents
         Scale E;
         {
-            float mg = 0.f, mc = 0.f, mh = 0.f, mt = 0.f;
+            float mg = 0.f, mb = 0.f, mc = 0.f, mh = 0.f, mt = 0.f;
             const float down = FORCE ? exp2f((float)(__float_as_int(a.torg[t].pad0) - ev)) : 0.f;  // w to units of 2^ev
 #pragma unroll 4
             for (int j = sub; j < TJ; j += JS) {
@@ -185,6 +233,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                 const float my = j == jself ? 0.f : h.w * y;
                 const float my2 = my * y;
                 mg += MODE == MODE_ENERGY ? my : my2;
+                if constexpr (MODE == MODE_NEWTON) mb = fmaf(my2, y * y, mb);
                 if constexpr (FORCE) {
                     const float4 g7 = reinterpret_cast<const float4 *>(b)[7 * TJ + j];
                     mc += j == jself ? 0.f : fmaf(fmaf(g7.z, qef, g7.y), y * y, g7.w);
@@ -193,6 +242,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                     mt = fmaf(my2, I.fd + wn, mt);
                 }
             }
+            if constexpr (MODE == MODE_NEWTON) near = fmaf(NEAR * epsf, mb, fmaf(1.f - NEAR, mg, near));
 #pragma unroll
             for (int off = JS / 2; off > 0; off >>= 1) {
                 mg += __shfl_xor_sync(0xffffffffu, mg, off);
@@ -202,6 +252,7 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                     mt += __shfl_xor_sync(0xffffffffu, mt, off);
                 }
             }
+            if constexpr (FORCE) near += mg;
             E.g = mag_exp(mg);
             E.q = -eL;
             E.lh = lift(E.g, mag_exp(mh), LIFT_H);
@@ -324,6 +375,30 @@ __device__ __forceinline__ bool fix_block(const PairArgs &a, int ibase, int spli
                 out(A_WX + k, ::fma(cs, v[k], T(8 + k)) + ::fma(-vi2, g, T(4 + k)));
             }
             if constexpr (MODE == MODE_FORCE_ENERGY) out(A_PSI, T(13));
+        }
+    }
+    if constexpr (MODE != MODE_ENERGY) {
+        // rows whose stars lie far inside the softening: in FP64 (above), by |n|^2 = 1 - eps^2 Q^2 or, at no cost per
+        // pair, by |n|^2 >= 1 - eps Q and S0 = sum m Q^2 Q (without the star itself)
+        bool lost = sub == 0 && valid;
+        if constexpr (FORCE) {
+            lost = lost && tot[3 * NT + grp] > (double)(near * (1.f - 1.f / NEAR)) * pow2(eg) * a.fu.inv_eps;
+        } else {
+            float w = near;
+#pragma unroll
+            for (int off = JS / 2; off > 0; off >>= 1) w += __shfl_xor_sync(0xffffffffu, w, off);
+            lost = lost && w > 0.f;
+        }
+        if (__syncthreads_or(lost)) {
+            int *flag = reinterpret_cast<int *>(buf);  // (every copy to the stages has been consumed)
+            double *red = reinterpret_cast<double *>(buf + PAIR_NT);
+            if (sub == 0) flag[grp] = lost;
+            __syncthreads();
+#pragma unroll 1
+            for (int r = 0; r < NI; ++r)
+                if (flag[r])
+                    fix_row_fp64<MODE>(static_cast<const double2 *>(a.pack), a.npad, ibase + r, t0 * TJ, min(t1 * TJ, a.nstar),
+                                       a.eps2, red, a.out + (size_t)split * NACC * a.npad + ibase + r);
         }
     }
     seq += (uint32_t)(t1 - t0 > 0 ? t1 - t0 : 0);

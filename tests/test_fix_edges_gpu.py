@@ -96,3 +96,45 @@ def test_one_fast_star(pn, speed):
     new, old = (_run(pn, x, v, m, 1.0, **kw) for kw in ({}, FP64))
     assert relerr(new[0], old[0]).max() <= 1e-12
     assert np.abs(new[1] - old[1]).max() <= 1e-12 * np.abs(old[1]).max()
+
+
+@pytest.mark.parametrize("ic2", [0.0, 1.0])
+@pytest.mark.parametrize("sep", [1e-1, 1e-2, 1e-4, 1e-6, 1e-8, 1e-10])
+@pytest.mark.parametrize("n", [3, 5])
+def test_close_pair_that_dominates(pn, n, sep, ic2):
+    """Two stars far below the softening apart, beside a BH too light to matter, alone or with a third one far
+    off: the pair's force keeps FP64's relative accuracy.  (An energy in between: one sweep serves both.)"""
+    rng = np.random.default_rng(n)
+    x = np.zeros((n, 3))
+    x[1] = [0.25, -0.125, 0.5]
+    x[2] = x[1] + sep * EPS * np.array([0.6, 0.0, 0.8])
+    x[3:] = rng.uniform(-1, 1, (n - 3, 3)) * 1e3
+    v = rng.normal(0, 0.3, (n, 3))
+    m = np.full(n, 1.0)
+    m[0] = 2.0 ** -50
+    out = []
+    for kw in ({}, FP64):
+        with pn.Context(n, eps=EPS, inv_c2=ic2, dt=1e-3, **kw) as c:
+            c.set_state(x, v, m)
+            a = c.force()
+            e = np.array(c.steps_energy(1))
+            out.append((a, e, c.get_state()[1] - v))
+    new, old = out
+    assert relerr(new[0][1:], old[0][1:]).max() <= 1e-14
+    assert np.abs(new[1] - old[1]).max() <= 1e-12 * np.abs(old[1]).max()
+
+
+@pytest.mark.parametrize("ic2", [0.0, 1.0])
+@pytest.mark.parametrize("n", [130, 300, 1026, 2500, 9001])
+def test_close_pairs_among_others(pn, n, ic2):
+    """Four heavy pairs, each 1e-7 eps wide, at the ends and in the middle of the rows, among light stars."""
+    x, v, m = _system(n, n)
+    m[:] = 1e-12
+    corners = np.array([[1.0, 1.0, 1.0], [1.0, -1.0, -1.0], [-1.0, 1.0, -1.0], [-1.0, -1.0, 1.0]])
+    rng = np.random.default_rng(n)
+    for k, (i, j) in enumerate([(1, 2), (5, 129), (n // 2, n - 2), (n // 3, n - 1)]):
+        x[i] = corners[k]
+        x[j] = x[i] + 1e-7 * EPS * rng.normal(size=3)
+        m[[i, j]] = 1.0
+    new, old = (_run(pn, x, v, m, ic2, **kw) for kw in ({}, FP64))
+    assert relerr(new[0], old[0]).max() <= 1e-12
