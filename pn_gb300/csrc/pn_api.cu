@@ -363,8 +363,8 @@ extern "C" int pn_create(pn_ctx **out, int nmax, const pn_params *p) {
     if (cudaMalloc(&c->pack2, 7 * (np / 2) * 16) != cudaSuccess) return fail("pack2");
     if (cudaMalloc(&c->ipack, np * 16) != cudaSuccess) return fail("ipack");
     if (cudaMalloc(&c->fpack, FIX_GROUPS * np * 16) != cudaSuccess) return fail("fpack");
-    if (cudaMalloc(&c->fix_bad, sizeof(int)) != cudaSuccess) return fail("fix_bad");
-    if (cudaMemset(c->fix_bad, 0, sizeof(int)) != cudaSuccess) return fail("memset");
+    if (cudaMalloc(&c->fix_bad, 2 * sizeof(int)) != cudaSuccess) return fail("fix_bad");
+    if (cudaMemset(c->fix_bad, 0, 2 * sizeof(int)) != cudaSuccess) return fail("memset");
     if (cudaMemset(c->pack2, 0, 7 * (np / 2) * 16) != cudaSuccess) return fail("memset");
     if (cudaMalloc(&c->torg, (np / 32 + 1) * sizeof(TileOrigin)) != cudaSuccess) return fail("torg");
     const size_t nblk = on_blocks(c->npad);

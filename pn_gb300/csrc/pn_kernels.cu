@@ -262,6 +262,7 @@ __device__ __forceinline__ void prep_body(const PrepArgs &a, int blk, int nblk) 
         pk[4 * a.npad + j] = make_double2(c1, c3);
         pk[5 * a.npad + j] = make_double2(k35, qe);
         if (a.fpack) {
+            if (j == 0) a.fix_bad[1] = 0;
             // the tile's velocity unit (a block is one tile of 128)
             static_assert(ON_NT == 128, "one tile per block");
             __shared__ int wev[4];

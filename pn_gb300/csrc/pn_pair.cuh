@@ -54,9 +54,9 @@ struct PairArgs {
     int gsplit;           // j-range splits (gridDim.y)
     double eps2;
     // the fixed-point FP64 sweep (pn_pairfix.cuh): its pack [13][npad], the flag that k_prep raises
-    // for a system outside its range, the state's masses and velocities, and its units
+    // for a system outside its range and the item that the FP64 sweep then takes next, the state's masses and velocities, and its units
     const uint4 *fpack;
-    const int *fix_bad;
+    int *fix_bad;
     const double *m, *v;
     long long vsp, vsk;
     FixUnits fu;

@@ -34,6 +34,7 @@
 namespace pn {
 
 constexpr int FIX_TJ = 128;
+constexpr int FIX_GENERAL_JS = 16;  // lanes per star in k_pair<double>'s block
 // Rows with sum m Q^2 |n|^2 < sum m Q^2 / NEAR go to FP64 (fix_row_fp64).
 constexpr float NEAR = 128.f;
 
@@ -69,7 +70,7 @@ __device__ __forceinline__ double pow2(int e) {  // 2^e, -1022 <= e <= 1023
 // Row i's sums with the stars j0 .. j1 - 1 in FP64, by the whole CTA, to out[slot * npad].  red: 4 NACC doubles of
 // shared memory.
 template <int MODE>
-__device__ __noinline__ void fix_row_fp64(const double2 *pk, int npad, int i, int j0, int j1, double eps2, double *red,
+__device__ __forceinline__ void fix_row_fp64(const double2 *pk, int npad, int i, int j0, int j1, double eps2, double *red,
                                           double *out) {
     constexpr int NACC = ModeInfo<MODE>::NACC;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -417,13 +418,27 @@ __global__ void __launch_bounds__(PAIR_NT, 3) k_pair_fix(const PairArgs a) {
     __syncthreads();
     uint32_t seq = 0;
     const int ibase = blockIdx.x * (PAIR_NT / JS);
-    if (*a.fix_bad == 0) {
-        double *tot = reinterpret_cast<double *>(smem + 128);
-        uint4 *buf = reinterpret_cast<uint4 *>(smem + 128 + fix_tot_bytes<MODE>());
-        fix_block<MODE, JS>(a, ibase, blockIdx.y, bars, tot, buf, seq);
-    } else {
-        pair_block<double, MODE, 1, JS>(a, ibase, blockIdx.y, bars, reinterpret_cast<double2 *>(smem + 128), seq);
+    if (__builtin_expect(*a.fix_bad != 0, 0)) {
+        // The launch's shape fits the sweep below, whose CTAs are few and unequally many per SM; in FP64 the fullest SM
+        // then sets the time, so the CTAs take smaller items in turn (N = 3,000 1,026 -> 892 us, 9,000 7.96 -> 7.53 ms,
+        // 30,000 82.8 -> 80.6 ms; 8 lanes per star: 872 us, 7.58 and 80.5 ms, but 64 stars 42 -> 55 us).
+        constexpr int BI = PAIR_NT / FIX_GENERAL_JS;
+        int &cur = *reinterpret_cast<int *>(smem + 64);  // (behind the barriers)
+        const int items = (a.nstar + BI - 1) / BI * a.gsplit;
+        for (;;) {
+            if (threadIdx.x == 0) cur = atomicAdd(a.fix_bad + 1, 1);
+            __syncthreads();
+            const int w = cur;
+            __syncthreads();  // everyone has read cur before thread 0 fetches the next item
+            if (w >= items) break;
+            if (!pair_block<double, MODE, 1, FIX_GENERAL_JS>(a, w / a.gsplit * BI, w % a.gsplit, bars,
+                                                             reinterpret_cast<double2 *>(smem + 128), seq)) break;
+        }
+        return;
     }
+    double *tot = reinterpret_cast<double *>(smem + 128);
+    uint4 *buf = reinterpret_cast<uint4 *>(smem + 128 + fix_tot_bytes<MODE>());
+    fix_block<MODE, JS>(a, ibase, blockIdx.y, bars, tot, buf, seq);
 }
 
 }  // namespace pn

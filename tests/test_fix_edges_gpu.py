@@ -138,3 +138,23 @@ def test_close_pairs_among_others(pn, n, ic2):
         m[[i, j]] = 1.0
     new, old = (_run(pn, x, v, m, ic2, **kw) for kw in ({}, FP64))
     assert relerr(new[0], old[0]).max() <= 1e-12
+
+
+@pytest.mark.parametrize("n", [2, 9, 17, 129, 1026, 4099, 9001])
+def test_general_block_of_any_size(pn, n):
+    """A system outside the range, its FP64 items shared out among the CTAs: the sums of the FP64-pipe sweep,
+    the same each time, in force, energy and step."""
+    x, v, m = _system(n, n)
+    m[n // 2 or 1] = m[0] * 2.0 ** -40
+    out = []
+    for kw in ({}, {}, FP64):
+        with pn.Context(n, eps=EPS, inv_c2=1e-2, dt=1e-3, **kw) as c:
+            c.set_state(x, v, m)
+            a, again = c.force(), c.force()
+            assert np.array_equal(a, again)
+            out.append((a, np.array(c.energy()), np.array(c.steps_energy(2)), *c.get_state()))
+    for p, q in zip(out[0], out[1]):
+        assert np.array_equal(p, q)
+    assert relerr(out[0][0], out[2][0]).max() <= 1e-12
+    for p, q in zip(out[0][1:], out[2][1:]):
+        assert np.abs(p - q).max() <= 1e-12 * np.abs(q).max()
