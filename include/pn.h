@@ -74,7 +74,9 @@ typedef struct {
 } pn_params;
 
 enum { PN_PAIR_AUTO = 0, PN_PAIR_SCALAR = 1, PN_PAIR_F32X2 = 2, PN_PAIR_F32X2_OCC3 = 3, PN_PAIR_F32X2_OCC4 = 4,
-       PN_PAIR_F32X2_SYM = 5 /* reported only: the packed sweep that forms every pair once */ };
+       PN_PAIR_F32X2_SYM = 5, /* reported only: the packed sweep that forms every pair once */
+       PN_PAIR_FIX64 = 6      /* reported only: FP64's sweep in fixed point, or its FP64 form in the same
+                                 launch where the system's values are outside its range */ };
 enum { PN_INT_REFERENCE = 0, PN_INT_RK4 = 1 };
 
 /* Energies as the reference prints them (Limit-sticky9.c:561-562, :702-703). */
@@ -91,8 +93,9 @@ typedef struct {
     double total_ms;         /* whole force evaluation */
     double interactions;     /* star-star pairs evaluated by that launch */
     int tile_j, i_per_thread, j_split, grid_split, threads; /* launch shape used */
-    int pair_variant;        /* PN_PAIR_SCALAR, PN_PAIR_F32X2, _OCC3, _OCC4 or _SYM (where grid_split
-                                counts the panels of the j-range, swept and summed in turn): the kernel used */
+    int pair_variant;        /* the kernel used: PN_PAIR_SCALAR, PN_PAIR_F32X2, _OCC3, _OCC4 or _SYM (where
+                                grid_split counts the panels of the j-range, swept and summed in turn),
+                                PN_PAIR_FIX64 */
 } pn_stats;
 
 /* ------------------------------------------------------------------ 1. drop-in entry points */

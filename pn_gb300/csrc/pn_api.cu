@@ -505,10 +505,11 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
     c->stats.tile_j = k.tj; c->stats.i_per_thread = k.ipt; c->stats.j_split = k.js;
     c->stats.grid_split = sym ? sym_panels(nstar, k.gsplit) : k.gsplit; c->stats.threads = PAIR_NT;
     c->stats.pair_variant = sym         ? PN_PAIR_F32X2_SYM
+                            : !k.x2       ? PN_PAIR_SCALAR
+                            : !is_f32(c)  ? PN_PAIR_FIX64
                             : k.x2 == 3   ? PN_PAIR_F32X2_OCC4
-                            : k.x2 == 2 ? PN_PAIR_F32X2_OCC3
-                            : k.x2      ? PN_PAIR_F32X2
-                                        : PN_PAIR_SCALAR;
+                            : k.x2 == 2   ? PN_PAIR_F32X2_OCC3
+                                          : PN_PAIR_F32X2;
     c->stats.interactions = (double)nstar * (double)nstar;
     return PN_OK;
 }

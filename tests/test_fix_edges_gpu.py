@@ -158,3 +158,14 @@ def test_general_block_of_any_size(pn, n):
     assert relerr(out[0][0], out[2][0]).max() <= 1e-12
     for p, q in zip(out[0][1:], out[2][1:]):
         assert np.abs(p - q).max() <= 1e-12 * np.abs(q).max()
+
+
+@pytest.mark.parametrize("kw,variant", [
+    ({}, 6), (FP64, 1), ({"eps": 1e-25}, 1),
+    ({"precision": 1, "pair_variant": 3, "i_per_thread": 2}, 3), ({"precision": 1, "pair_variant": 1}, 1)])
+def test_the_kernel_used_is_reported(pn, kw, variant):
+    x, v, m = _system(5000, 1)
+    with pn.Context(5000, **{"eps": EPS, "inv_c2": 1e-2, **kw}) as c:
+        c.set_state(x, v, m)
+        c.force()
+        assert c.stats().pair_variant == variant
