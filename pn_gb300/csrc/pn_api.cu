@@ -189,7 +189,7 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
     const int pv = c->p.pair_variant;
     PairCfg tuned;
     FixUnits fu;
-    const bool fix = !f32 && !explicit_shape && nstar > 0 && fix_units(c->p.eps, c->p.inv_c2, &fu);
+    const bool fix = !f32 && !explicit_shape && nstar > 0 && !c->fix_off && fix_units(c->p.eps, c->p.inv_c2, &fu);
     // (an FP64 shape tuned for the other of its two sweeps does not apply: 3.5 to 4.5 times slower, or
     // outside the fixed-point one's range)
     if (!explicit_shape && pv == PN_PAIR_AUTO && nstar > 0 &&
@@ -283,6 +283,11 @@ void pn::ensure_sym(pn_ctx *c) {
     }
 }
 
+// After another size or other parameters: shapes and captured steps are of the old ones (and there may be memory now).
+static void forget_cfg(pn_ctx *c) {
+    c->cfg_set = c->step_valid = c->timed_valid = c->fix_off = false;
+}
+
 static void free_ctx(pn_ctx *c) {
     if (!c) return;
     free_adjoint(c);
@@ -362,7 +367,6 @@ extern "C" int pn_create(pn_ctx **out, int nmax, const pn_params *p) {
     if (cudaMalloc(&c->pack, 6 * np * 16) != cudaSuccess) return fail("pack");
     if (cudaMalloc(&c->pack2, 7 * (np / 2) * 16) != cudaSuccess) return fail("pack2");
     if (cudaMalloc(&c->ipack, np * 16) != cudaSuccess) return fail("ipack");
-    if (cudaMalloc(&c->fpack, FIX_GROUPS * np * 16) != cudaSuccess) return fail("fpack");
     if (cudaMalloc(&c->fix_bad, 2 * sizeof(int)) != cudaSuccess) return fail("fix_bad");
     if (cudaMemset(c->fix_bad, 0, 2 * sizeof(int)) != cudaSuccess) return fail("memset");
     if (cudaMemset(c->pack2, 0, 7 * (np / 2) * 16) != cudaSuccess) return fail("memset");
@@ -399,8 +403,7 @@ extern "C" int pn_destroy(pn_ctx *c) {
 extern "C" int pn_set_params(pn_ctx *c, const pn_params *p) {
     if (!c || validate_params(p) != PN_OK) return set_err(PN_ERR_INVALID, "pn_set_params");
     c->p = *p;
-    c->cfg_set = false;
-    c->step_valid = c->timed_valid = false;
+    forget_cfg(c);
     return PN_OK;
 }
 
@@ -418,6 +421,22 @@ void pn::refresh_cfg(pn_ctx *c) {
     c->cfg_set = true;
 }
 
+// The shapes of this size and the buffers that their sweeps need (208 bytes per star for the fixed-point sweep's pack,
+// which mixed contexts and given shapes do without; the FP64 sweep takes its place where there is no memory for it).
+static int ensure_work(pn_ctx *c) {
+    refresh_cfg(c);
+    if (!is_f32(c) && !c->fpack && (c->cfg_force.x2 || c->cfg_energy.x2) &&
+        cudaMalloc(&c->fpack, FIX_GROUPS * (size_t)c->npad * 16) != cudaSuccess) {
+        cudaGetLastError();
+        c->fpack = nullptr;
+        c->fix_off = true;
+        c->cfg_set = false;
+        refresh_cfg(c);
+    }
+    ensure_sym(c);
+    return ensure_sums(c);
+}
+
 // One force evaluation.  x, v, m: particle p component k at [p*sp + k*sk] (device).
 // a_out: optional device output (AoS when asp=3, ask=1).  stage: fused integration stage.
 // with_energy: the same sweep also accumulates the energy's Psi, and the energies of the state
@@ -427,13 +446,11 @@ int pn::eval_force(pn_ctx *c, const double *x, const double *v, const double *m,
                    cudaStream_t s, bool timed, int tslot, double *sums_out, bool with_energy) {
     const int n = c->n;
     const int nstar = n - 1;
-    refresh_cfg(c);
     const int mode = with_energy ? (int)MODE_FORCE_ENERGY : force_mode(c);
-    ensure_sym(c);
+    int rc = ensure_work(c);
+    if (rc) return rc;
     const PairCfg &k = with_energy ? c->cfg_fused : c->cfg_force;
     const bool sym = is_f32(c) && k.x2 == 4;
-    int rc = ensure_sums(c);
-    if (rc) return rc;
     const double eps2 = c->p.eps * c->p.eps;
 
     PrepArgs pa{};
@@ -551,7 +568,7 @@ extern "C" int pn_set_state(pn_ctx *c, int n, const double *x, const double *v, 
     cudaError_t e4 = cudaStreamSynchronize(c->stream);
     cudaFreeHost(h);
     if (e1 || e2 || e3 || e4) return set_err(PN_ERR_CUDA, "pn_set_state: copy failed");
-    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
+    if (n != c->n) forget_cfg(c);
     c->n = n;
     c->time = 0.0;
     c->have_state = true;
@@ -598,7 +615,7 @@ extern "C" int pn_force_device(pn_ctx *c, int n, const double *d_x, const double
     if (!c || n < 1 || n > c->nmax || !d_x || !d_v || !d_m || !d_a)
         return set_err(PN_ERR_INVALID, "pn_force_device");
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
+    if (n != c->n) forget_cfg(c);
     c->n = n;
     return eval_force(c, d_x, d_v, d_m, 3, 1, d_a, 3, 1, 0, s, false);
 }
@@ -632,9 +649,7 @@ static int build_step_graph(pn_ctx *c, bool timed = false) {
     bool &valid = timed ? c->timed_valid : c->step_valid;
     if (valid) return PN_OK;
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
-    refresh_cfg(c);
-    ensure_sym(c);  // (allocated before capture)
-    int rc = ensure_sums(c);
+    int rc = ensure_work(c);  // (allocated before capture)
     if (rc) return rc;
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -815,10 +830,9 @@ extern "C" int pn_load_checkpoint(pn_ctx *c, const char *path, double *eouttime,
 static int enqueue_energy(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,
                           long long sk) {
     const int nstar = c->n - 1;
-    refresh_cfg(c);
-    const PairCfg &k = c->cfg_energy;
-    int rc = ensure_sums(c);
+    int rc = ensure_work(c);
     if (rc) return rc;
+    const PairCfg &k = c->cfg_energy;
     const double eps2 = c->p.eps * c->p.eps;
     cudaStream_t s = c->stream;
     PrepArgs pa{};
@@ -936,7 +950,7 @@ static int drop_upload(pn_ctx *c, const double *x, const double *v, const double
     std::memcpy(g_drop_h + 3 * w, v, 3 * w * sizeof(double));
     std::memcpy(g_drop_h + 6 * w, m, w * sizeof(double));
     CU(cudaMemcpyAsync(c->in_aos, g_drop_h, 7 * w * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    if (n != c->n) { c->cfg_set = false; c->step_valid = c->timed_valid = false; }
+    if (n != c->n) forget_cfg(c);
     c->n = n;
     return PN_OK;
 }

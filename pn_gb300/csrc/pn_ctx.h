@@ -24,7 +24,8 @@ struct pn_ctx {
     void *pack = nullptr;
     float4 *pack2 = nullptr;      // paired pack of the f32x2 sweep [7][npad/2]
     float4 *ipack = nullptr;      // [npad] (v.xyz, qe)
-    uint4 *fpack = nullptr;       // pack of the fixed-point FP64 sweep [FIX_GROUPS][npad]
+    uint4 *fpack = nullptr;       // pack of the fixed-point FP64 sweep [FIX_GROUPS][npad] (on first use)
+    bool fix_off = false;         // there was no memory for it
     int *fix_bad = nullptr;       // raised by k_prep for a system outside that sweep's range; the next item of the sweep that then runs
     pn::TileOrigin *torg = nullptr;
     void *sym_work = nullptr;     // partial sums of the sweep over unordered pairs (on first use)

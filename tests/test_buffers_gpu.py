@@ -50,3 +50,58 @@ def test_captured_force_outlives_other_calls(pn, precision, n):
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(a, da)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_context_allocates_what_it_uses(pn, precision):
+    """State 152 bytes per particle, results and staging 80, BH-relative positions 24, packs 168, tile origins 2,
+    partial sums 1; the fixed-point pack (208) only once its sweep runs."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 20
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    with pn.Context(n, eps=EPS, precision=precision):
+        taken = free - torch.cuda.mem_get_info()[0]
+    assert taken <= 440 * n + (32 << 20)  # (allocations are rounded up to 2 MiB)
+
+
+class _NoMemory:
+    """Takes the GPU's free memory, but for a few MiB."""
+
+    def __enter__(self):
+        import torch
+        self.held, size = [], torch.cuda.mem_get_info()[0]
+        while size >= 2 << 20:
+            try:
+                self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                size //= 2
+            size = min(size, torch.cuda.mem_get_info()[0])
+        return self
+
+    def __exit__(self, *a):
+        import torch
+        self.held.clear()
+        torch.cuda.empty_cache()
+
+
+def test_no_memory_for_the_fixed_point_pack(pn):
+    """The FP64 sweep takes over, and gives way again once there is memory and the parameters are set anew."""
+    pytest.importorskip("torch")
+    n = 40001
+    x, v, m = _system(n)
+    with pn.Context(n, eps=EPS, inv_c2=1e-2) as c:  # (its kernels are loaded)
+        c.set_state(x, v, m)
+        a = c.force()
+        assert c.stats().pair_variant == 6
+    with pn.Context(n, eps=EPS, inv_c2=1e-2, i_per_thread=1, grid_split=16) as c:  # (so are its sums)
+        c.set_state(x, v, m)
+        b = c.force()
+        with _NoMemory():
+            c.set_params(i_per_thread=0, grid_split=0)
+            d = c.force()
+            assert c.stats().pair_variant == 1
+        c.set_params()
+        assert np.array_equal(c.force(), a) and c.stats().pair_variant == 6
+    for f in (b, d):
+        assert (np.linalg.norm(f - a, axis=1) <= 1e-12 * np.linalg.norm(a, axis=1).max()).all()
