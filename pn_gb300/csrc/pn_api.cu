@@ -265,7 +265,7 @@ static int ensure_sums(pn_ctx *c) {
 }
 
 // Room for the partial sums of the sweep over unordered pairs; the packed sweep takes its place where
-// there is none.
+// there is none, until the shapes are chosen anew.
 void pn::ensure_sym(pn_ctx *c) {
     if (!is_f32(c) || c->cfg_force.x2 != 4) return;
     const size_t need = sym_bytes(c->n - 1, c->cfg_force.gsplit);
@@ -278,7 +278,6 @@ void pn::ensure_sym(pn_ctx *c) {
         c->sym_have = need;
     } else {
         cudaGetLastError();
-        c->sym_off = true;
         c->cfg_force = c->cfg_fused;
     }
 }
@@ -416,7 +415,6 @@ void pn::refresh_cfg(pn_ctx *c) {
     if (is_f32(c) && c->cfg_force.x2 == 4) {
         choose_packed(&c->cfg_fused, nstar, c->sms);
         c->cfg_fused.x2 = c->cfg_fused.ipt == 2 ? 2 : 1;
-        if (c->sym_off) c->cfg_force = c->cfg_fused;
     }
     c->cfg_set = true;
 }
@@ -1217,10 +1215,15 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
     if (!c || !c->have_state) return set_err(PN_ERR_STATE, "pn_autotune: no state");
     const int nstar = c->n - 1;
     if (nstar < 1) return PN_OK;
-    refresh_cfg(c);
+    int rc = ensure_work(c);
+    if (rc) return rc;
     const bool f32 = is_f32(c);
     FixUnits fu;
-    const bool fix = !f32 && fix_units(c->p.eps, c->p.inv_c2, &fu);
+    const bool fix = !f32 && !c->fix_off && fix_units(c->p.eps, c->p.inv_c2, &fu);
+    auto give_up = [&](int status) {  // (not with a candidate's shape)
+        c->cfg_set = false;
+        return status;
+    };
     const int modes[2] = {force_mode(c), MODE_ENERGY};
     for (int which = 0; which < 2; ++which) {
         if (!(sweeps & (1 << which))) continue;
@@ -1231,14 +1234,18 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
         for (const PairCfg &k : cands) {
             // a whole evaluation (prep, pair sweep, finish), so that the finishing kernel's reads of the
             // j-range partial sums (72 B per star and split) count against the shapes with many splits
-            (which == 0 ? c->cfg_force : c->cfg_energy) = k;
+            PairCfg &used = which == 0 ? c->cfg_force : c->cfg_energy;
+            used = k;
             c->cfg_set = true;
+            rc = ensure_work(c);
+            if (rc) return give_up(rc);
+            if (used.x2 != k.x2) continue;  // (no memory for it)
             float t = 1e30f;
             for (int rep = 0; rep < 3; ++rep) {  // first evaluation warms up; best of two
                 CU(cudaEventRecord(c->ev0, c->stream));
-                int rc = which == 0 ? eval_force(c, c->st.x, c->st.v, c->st.m, 1, c->ld, nullptr, 3, 1, 0, c->stream, false)
-                                    : enqueue_energy(c, c->st.x, c->st.v, c->st.m, 1, c->ld);
-                if (rc) return rc;
+                rc = which == 0 ? eval_force(c, c->st.x, c->st.v, c->st.m, 1, c->ld, nullptr, 3, 1, 0, c->stream, false)
+                                : enqueue_energy(c, c->st.x, c->st.v, c->st.m, 1, c->ld);
+                if (rc) return give_up(rc);
                 CU(cudaEventRecord(c->ev1, c->stream));
                 CU(cudaEventSynchronize(c->ev1));
                 float ms = 0.f;
@@ -1253,8 +1260,8 @@ extern "C" int pn_autotune(pn_ctx *c, int sweeps, double *best_ms) {
                 best = k;
             }
         }
-        int rc = check_device_err(c);
-        if (rc) return rc;
+        rc = check_device_err(c);
+        if (rc) return give_up(rc);
         tune_store(c->p.precision, mode, nstar, best, best_t);
         if (best_ms) best_ms[which] = best_t;
     }

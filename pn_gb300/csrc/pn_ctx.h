@@ -30,7 +30,6 @@ struct pn_ctx {
     pn::TileOrigin *torg = nullptr;
     void *sym_work = nullptr;     // partial sums of the sweep over unordered pairs (on first use)
     size_t sym_have = 0;
-    bool sym_off = false;         // there was no memory for them
     double *acc = nullptr;
     int acc_splits = 0;
     double *part = nullptr;  // partial sums (prep / finish / energy share one buffer region each)

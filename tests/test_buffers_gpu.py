@@ -105,3 +105,41 @@ def test_no_memory_for_the_fixed_point_pack(pn):
         assert np.array_equal(c.force(), a) and c.stats().pair_variant == 6
     for f in (b, d):
         assert (np.linalg.norm(f - a, axis=1) <= 1e-12 * np.linalg.norm(a, axis=1).max()).all()
+
+
+def test_no_memory_for_the_unordered_sweep(pn):
+    """The packed sweep takes over, also while shapes are tuned (none is kept for the sweep that did not run), and
+    gives way again once there is memory."""
+    pytest.importorskip("torch")
+    n = 20001
+    x, v, m = _system(n)
+    kw = dict(eps=EPS, inv_c2=1e-2, precision=1)
+    with pn.Context(n, **kw) as c:
+        c.set_state(x, v, m)
+        a = c.force()
+        assert c.stats().pair_variant == 5
+    try:
+        with pn.Context(n, grid_split=32, **kw) as c:  # (its sums are allocated)
+            c.set_state(x, v, m)
+            c.force()
+            c.autotune(1)  # (every kernel is loaded)
+            pn.lib().pn_autotune_clear()
+        with pn.Context(n, grid_split=32, **kw) as c:
+            c.set_state(x, v, m)
+            c.force()
+            with _NoMemory():
+                c.set_params(grid_split=0)
+                b = c.force()
+                assert c.stats().pair_variant in (2, 3)
+                c.autotune(1)
+                c.force()
+                assert c.stats().pair_variant != 5
+            c.set_params(dt=1e-3)
+            c.force()
+            assert c.stats().pair_variant != 5  # (a tuned shape)
+            pn.lib().pn_autotune_clear()
+            c.set_params(dt=2e-3)
+            assert np.array_equal(c.force(), a) and c.stats().pair_variant == 5
+    finally:
+        pn.lib().pn_autotune_clear()
+    assert np.sqrt(((a - b) ** 2).sum() / (a ** 2).sum()) <= 2e-6  # (each within 1e-6 of FP64)
