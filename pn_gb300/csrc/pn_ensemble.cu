@@ -141,6 +141,12 @@ static int cluster_gsplit(const pn_ens *e, int c) {
 // 200 clusters of 400 stars 571 / 634, 100 of 1,000 861 / 933, 60 of 1,500 1,126 / 1,061, 40 of 2,500 1,733 /
 // 1,691, 16 of 5,000 3,103 / 2,298, 4 of 1,000 669 / 276.
 constexpr size_t SYM_ENS_BYTES = (size_t)2 << 30;
+static void ens_free_sym(pn_ens *e) {
+    for (void **p : {&e->sym_work, (void **)&e->t_sym, (void **)&e->sym_items}) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+    }
+}
 static bool ens_build_sym(pn_ens *e) {
     long long units = 0, packed_items = 0;
     double cost = 0.0, packed = 0.0;
@@ -156,10 +162,7 @@ static bool ens_build_sym(pn_ens *e) {
     size_t bytes = 0;
     for (int c = 0; c < e->nc; ++c) bytes += sym_ens_bytes(e->n[c] - 1, chunk);
     if (bytes > SYM_ENS_BYTES) return false;
-    for (void **p : {&e->sym_work, (void **)&e->t_sym, (void **)&e->sym_items}) {
-        if (*p) cudaFree(*p);
-        *p = nullptr;
-    }
+    ens_free_sym(e);
     std::vector<Pair2SymArgs> tab(e->nc);
     std::vector<int4> items;
     if (cudaMalloc(&e->sym_work, std::max<size_t>(1, bytes)) != cudaSuccess) {
@@ -204,15 +207,18 @@ static int ens_build_tables(pn_ens *e) {
     const bool f32 = ens_f32(e);
     const int mode = ens_mode(e);
     const int nc = e->nc;
+    e->step_valid = false;  // (a captured step holds the old buffers, also where a new one cannot be had)
     int gmax = 1;
     for (int c = 0; c < nc; ++c) gmax = std::max(gmax, cluster_gsplit(e, c));
     if (gmax > e->acc_splits) {
         if (e->acc) cudaFree(e->acc);
         e->acc = nullptr;
+        e->acc_splits = 0;
         ECU(cudaMalloc(&e->acc, (size_t)gmax * NACC_MAX * e->S * sizeof(double)));
         e->acc_splits = gmax;
     }
     if (e->sym) e->sym = ens_build_sym(e);
+    if (!e->sym) ens_free_sym(e);
     std::vector<PrepArgs> tp(3 * nc);
     std::vector<FinishArgs> tf(4 * nc);
     std::vector<EnergyArgs> te(nc);
@@ -356,7 +362,6 @@ static int ens_build_tables(pn_ens *e) {
     ECU(cudaMemcpy(e->t_fin, tf.data(), tf.size() * sizeof(FinishArgs), cudaMemcpyHostToDevice));
     ECU(cudaMemcpy(e->t_en, te.data(), te.size() * sizeof(EnergyArgs), cudaMemcpyHostToDevice));
     ECU(cudaMemcpy(e->t_pair, tq.data(), tq.size() * sizeof(PairArgs), cudaMemcpyHostToDevice));
-    e->step_valid = false;
     return PN_OK;
 }
 

@@ -143,3 +143,22 @@ def test_no_memory_for_the_unordered_sweep(pn):
     finally:
         pn.lib().pn_autotune_clear()
     assert np.sqrt(((a - b) ** 2).sum() / (a ** 2).sum()) <= 2e-6  # (each within 1e-6 of FP64)
+
+
+class _Cluster:
+    def __init__(self, n):
+        self.x, self.v, self.m = _system(n)
+
+
+def test_ensemble_gives_its_sums_back(pn):
+    """The partial sums of the unordered sweep (150 MB here) go when another sweep is asked for."""
+    torch = pytest.importorskip("torch")
+    clusters = [_Cluster(16385) for _ in range(4)]
+    with pn.Ensemble(clusters, [EPS] * 4, precision=1, inv_c2=1e-2, dt=1e-3) as e:
+        e.steps(1)
+        e.get_state()
+        free = torch.cuda.mem_get_info()[0]
+        e.set_shape(2, 1)
+        assert torch.cuda.mem_get_info()[0] - free > 100 << 20
+        e.steps(1)
+        e.get_state()
