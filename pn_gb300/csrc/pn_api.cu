@@ -129,11 +129,11 @@ static void choose_fix(PairCfg *k, int nstar, int sms) {
 // per split in the finishing kernel.  Measured against the former rule (2 i per thread from N = 4096,
 // about 32 CTAs per SM, the 2-CTA build): N = 1,001 pair 28.6 -> 12.5 us, 4,096: 75.9 -> 42.5,
 // 12,000: 281 -> 234, 16,384: 424 either way, 65,536: 6.57 -> 6.33 ms, 262,144: 101.2 -> 100.3 ms.
-static void choose_packed(PairCfg *k, int nstar, int sms) {
+static void choose_packed(PairCfg *k, int nstar, int sms, int ipt_min = 1) {
     static const double busy[2][4] = {{0.40, 0.70, 0.85, 0.92}, {0.62, 0.88, 1.0, 1.0}};
     k->js = 1;
     double best = 1e300;
-    for (int ipt = 1; ipt <= 2; ++ipt) {
+    for (int ipt = ipt_min; ipt <= 2; ++ipt) {
         const int tj = 128 * ipt, ntiles = (nstar + tj - 1) / tj, nib = (nstar + 128 * ipt - 1) / (128 * ipt);
         for (int g = 1; g <= 32 && g <= ntiles; ++g) {
             const int n = (nib * g + sms - 1) / sms;
@@ -215,9 +215,17 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
             choose_sym(&k, nstar, c->sms);
             return k;
         }
-        choose_packed(&k, nstar, c->sms);
-        k.x2 = k.ipt == 2 && mode_has_force(mode) ? 2 : 1;
-        return k;
+        // The Newtonian and the energy sweep need fewer registers and have more resident CTAs than that model, whose few
+        // large CTAs leave them a long last wave: N = 20,000 Newtonian 322 us against 306 in the general shape below,
+        // 37,000 975 / 922, energy 1,454 / 1,365 (from 65,536 stars on that has too few splits, 2,884 / 2,771, and
+        // below 16,000 unequal ones: 13,750 170 / 158); and two stars per thread from N = 12,000 on (12,120 137 -> 131).
+        if (mode_has_force(mode) || nstar < 16000 || nstar >= 65536) {
+            choose_packed(&k, nstar, c->sms, mode_has_force(mode) || nstar < 12000 ? 1 : 2);
+            k.x2 = k.ipt == 2 && mode_has_force(mode) ? 2 : 1;
+            return k;
+        }
+        k.ipt = 2;
+        k.x2 = 1;
     } else {
         k.x2 = 0;  // scalar sweep: FP64, PN_PAIR_SCALAR, or an explicit shape without the variant
     }
