@@ -272,22 +272,32 @@ static int ensure_sums(pn_ctx *c) {
     return ensure_acc(c, std::max({acc_splits(c->cfg_force), c->cfg_energy.gsplit, c->cfg_fused.gsplit}));
 }
 
+// Memory that a sweep can do without.  none: there is none left (and only that: where the call itself is refused, as
+// while a caller captures, it is an error, not a reason for another sweep in all calls that follow).
+static int optional_alloc(void **p, size_t bytes, bool *none) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    *none = e == cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) return PN_OK;
+    cudaGetLastError();
+    *p = nullptr;
+    return *none ? PN_OK : set_err(PN_ERR_CUDA, "work buffer: %s", cudaGetErrorString(e));
+}
+
 // Room for the partial sums of the sweep over unordered pairs; the packed sweep takes its place where
 // there is none, until the shapes are chosen anew.
-void pn::ensure_sym(pn_ctx *c) {
-    if (!is_f32(c) || c->cfg_force.x2 != 4) return;
+int pn::ensure_sym(pn_ctx *c) {
+    if (!is_f32(c) || c->cfg_force.x2 != 4) return PN_OK;
     const size_t need = sym_bytes(c->n - 1, c->cfg_force.gsplit);
-    if (need <= c->sym_have) return;
+    if (need <= c->sym_have) return PN_OK;
     if (c->sym_work) cudaFree(c->sym_work);
     c->sym_work = nullptr;
     c->sym_have = 0;
     c->step_valid = c->timed_valid = false;  // captured steps hold the old buffer
-    if (cudaMalloc(&c->sym_work, need) == cudaSuccess) {
-        c->sym_have = need;
-    } else {
-        cudaGetLastError();
-        c->cfg_force = c->cfg_fused;
-    }
+    bool none;
+    const int rc = optional_alloc(&c->sym_work, need, &none);
+    if (none) c->cfg_force = c->cfg_fused;
+    else if (!rc) c->sym_have = need;
+    return rc;
 }
 
 // After another size or other parameters: shapes and captured steps are of the old ones (and there may be memory now).
@@ -431,16 +441,16 @@ void pn::refresh_cfg(pn_ctx *c) {
 // which mixed contexts and given shapes do without; the FP64 sweep takes its place where there is no memory for it).
 static int ensure_work(pn_ctx *c) {
     refresh_cfg(c);
-    if (!is_f32(c) && !c->fpack && (c->cfg_force.x2 || c->cfg_energy.x2) &&
-        cudaMalloc(&c->fpack, FIX_GROUPS * (size_t)c->npad * 16) != cudaSuccess) {
-        cudaGetLastError();
-        c->fpack = nullptr;
-        c->fix_off = true;
-        c->cfg_set = false;
-        refresh_cfg(c);
+    if (!is_f32(c) && !c->fpack && (c->cfg_force.x2 || c->cfg_energy.x2)) {
+        const int rc = optional_alloc((void **)&c->fpack, FIX_GROUPS * (size_t)c->npad * 16, &c->fix_off);
+        if (rc) return rc;
+        if (c->fix_off) {
+            c->cfg_set = false;
+            refresh_cfg(c);
+        }
     }
-    ensure_sym(c);
-    return ensure_sums(c);
+    const int rc = ensure_sym(c);
+    return rc ? rc : ensure_sums(c);
 }
 
 // One force evaluation.  x, v, m: particle p component k at [p*sp + k*sk] (device).

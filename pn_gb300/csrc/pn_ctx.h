@@ -69,7 +69,7 @@ bool is_f32(const pn_ctx *c);
 int force_mode(const pn_ctx *c);
 void refresh_cfg(pn_ctx *c);
 int ensure_acc(pn_ctx *c, int splits);
-void ensure_sym(pn_ctx *c);
+int ensure_sym(pn_ctx *c);
 int check_device_err(pn_ctx *c);
 // One force evaluation; see pn_api.cu.  sums_out (optional) receives the per-star pair sums.
 int eval_force(pn_ctx *c, const double *x, const double *v, const double *m, long long sp,

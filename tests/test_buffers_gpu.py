@@ -162,3 +162,48 @@ def test_ensemble_gives_its_sums_back(pn):
         assert torch.cuda.mem_get_info()[0] - free > 100 << 20
         e.steps(1)
         e.get_state()
+
+
+REFUSED = r"""
+import sys
+import numpy as np
+import torch
+import pn_gb300 as pn
+sys.path.insert(0, sys.argv[1])
+from test_buffers_gpu import EPS, _system
+for precision, kw, variant in ((0, dict(i_per_thread=1, grid_split=32), 6), (1, dict(grid_split=32), 5)):
+    n = 9001
+    x, v, m = _system(n)
+    with pn.Context(n, eps=EPS, inv_c2=1e-2, precision=precision, **kw) as c:
+        c.set_state(x, v, m)
+        c.force()
+        c.set_params(**{k: 0 for k in kw})
+        d = [torch.tensor(q, device="cuda") for q in (x, v, m)]
+        a = torch.zeros(n, 3, dtype=torch.float64, device="cuda")
+        s = torch.cuda.Stream()
+        refused = None
+        try:
+            with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=s):  # (capture that allows no allocation)
+                try:
+                    c.force_device(n, *(q.data_ptr() for q in d), a.data_ptr(), s.cuda_stream)
+                except pn.PNError as e:
+                    refused = e.status
+        except RuntimeError:
+            pass
+        assert refused == -2, refused
+        c.force()
+        assert c.stats().pair_variant == variant
+print("ok")
+"""
+
+
+def test_an_allocation_refused_while_capturing_is_an_error(pn):
+    """... and no reason to take a slower sweep from then on.  (In a process of its own: the capture is broken off.)"""
+    pytest.importorskip("torch")
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(here))
+    r = subprocess.run([sys.executable, "-c", REFUSED, here], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
