@@ -642,8 +642,8 @@ def headline(args, rank, world, dist):
         sym = st.pair_variant == 5
         gs = 1 if sym else st.grid_split
         # k_prep reads x, v, m (56 B) and writes spos, the paired pack, the i-side pack (96 B; the
-        # scalar pack's 64 B too when the scalar sweep runs; 64 B in all for the sweep that forms every
-        # pair once); k_finish reads v, m, spos (56 B) and
+        # scalar pack's 64 B too when the scalar sweep runs; spos and a pack of 64 B, 88 B in all, for the
+        # sweep that forms every pair once); k_finish reads v, m, spos (56 B) and
         # the j-range partial sums (9 doubles per split), and reads/writes the stage state (168 B)
         moved = 56 + (88 if sym else 96 if st.pair_variant in (2, 3, 4) else 160) + 56 + 72 * gs + 168
         algo = 104 + 144                  # BH-star O(N) terms + one stage update, per star

@@ -132,14 +132,14 @@ static int cluster_gsplit(const pn_ens *e, int c) {
 }
 
 // Tables and work items of the sweep over unordered pairs; false (and the packed sweep) where its
-// partial sums would take more than SYM_ENS_BYTES or there is no memory for them.  Tiles per item as for
-// one system (pn_api.cu, choose_sym), over the work of all clusters.
+// partial sums would take more than SYM_ENS_BYTES (0.14 n^2 bytes per cluster, so four of 65,536 stars do) or there
+// is no memory for them.  Tiles per item as for one system (pn_api.cu, choose_sym), over the work of all clusters.
 // Small clusters leave most of a 512-star row block empty and few tiles that serve both sides, so the
-// packed sweep keeps them: compared by operations per 256 stars and tile (25 packed there; here 102 for 512
-// rows in both orders, 150 for both sides) over the share of the FMA pipe that each sweep keeps busy (85 and
-// 73 %), unless the packed sweep's items are fewer than the SMs.  Measured (us per step, packed and this one):
-// 200 clusters of 400 stars 571 / 634, 100 of 1,000 861 / 933, 60 of 1,500 1,126 / 1,061, 40 of 2,500 1,733 /
-// 1,691, 16 of 5,000 3,103 / 2,298, 4 of 1,000 669 / 276.
+// packed sweep keeps them: compared by a thread's packed operations for a row block and a tile of 128 stars (25 x 256
+// for 256 rows there; here, for 512 rows, 51 x 256 in one order and 75 x 256 where both sides are served) over the
+// share of the FMA pipe that each sweep keeps busy (85 and 73 %), unless the packed sweep's items are fewer than the
+// SMs.  Measured (us per step, packed and this one): 200 clusters of 400 stars 571 / 634, 100 of 1,000 861 / 933, 60
+// of 1,500 1,126 / 1,061, 40 of 2,500 1,733 / 1,691, 16 of 5,000 3,103 / 2,298, 4 of 1,000 669 / 276.
 constexpr size_t SYM_ENS_BYTES = (size_t)2 << 30;
 static void ens_free_sym(pn_ens *e) {
     for (void **p : {&e->sym_work, (void **)&e->t_sym, (void **)&e->sym_items}) {

@@ -30,6 +30,8 @@
 // so the smallest kept bit is 2^-62 of that sum; the tile sums are added in FP64.  The pair of a star
 // with itself (d = 0: no G, no W) would raise that scale to m / eps^2; it is left out of the integer
 // sums and its S0, and in the energy sweep Phi and Psi, added in FP64.
+// Two of these errors do not shrink with their term, as FP64's do: n's, 2^-61 also where d is far below eps (the
+// sweep forms such rows again in FP64), and the velocity terms' in the unit of a tile's fastest star (velocity_limit).
 #pragma once
 
 #include <cstdint>
@@ -140,7 +142,7 @@ PNF u64 shr(u64 a, int s) {
 
 // Sums of a product and a 32-bit part as carry additions of their halves: as the addend of a multiply-add the
 // part would have to be moved and extended into a register pair, by moves on the pipe that bounds the
-// sweep (N = 65,536: 77.3 -> 71.3 ms).
+// sweep (N = 65,536: 77.3 -> 71.7 ms).
 // a + (c >> 32)
 PNF i64 plus_hi(i64 a, i64 c) {
 #ifdef __CUDA_ARCH__

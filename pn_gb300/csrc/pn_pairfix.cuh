@@ -7,15 +7,15 @@
 // passed twice: in FP32 for the magnitude of the tile's sums (the integer sums' exponents), then
 // for the sums themselves, which are added to FP64 totals in shared memory at the tile's end.
 //
-// Why: FP64 issues one warp instruction per 64 cycles and scheduler here and k_pair<double>'s 51 per
-// pair keep that pipe busy for 3580 cycles per warp of pairs; this form takes 672, of which the
+// Why: FP64 issues one warp instruction per 64 cycles and scheduler here, so k_pair<double>'s 51 per
+// pair take that pipe 3,264 cycles per warp of pairs (3,610 measured); this form takes 672, of which the
 // multiply-add pipe is busy 71 % and the FP64 pipe 59 % (6 operations per pair). One force evaluation at
-// N = 65,536: 385 -> 71.7 ms, N = 10,000: 9.3 -> 1.85 ms.  Its error against long double sums is below
+// N = 65,536: 385 -> 71.5 ms, N = 10,000: 9.3 -> 1.85 ms.  Its error against long double sums is below
 // the FP64 sweep's (medians at N = 2,049: 1.46e-16 against 2.22e-16 at c = 1000, 5.2e-16 against
 // 7.4e-16 at c = 1).  Measured on the way there, at N = 65,536: every product in integers and C's sum
 // in FP64 (4 conversions and 5 FMA per pair) 104 ms; the dot products' small parts in FP32, Phi and U in
-// FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms, carry additions 71.7 ms; the sums' small parts in FP32
-// too (before that) 76 against 88 ms, but with twice the FP64 sweep's error at c = 1.
+// FP64 and C's sum in integers 88.2 ms; one sum along n for C and H 77.3 ms, carry additions 71.7 ms; the sums' small
+// parts in FP32 too (before that) 76 against 88 ms, but with twice the FP64 sweep's error at c = 1.
 //
 // n = d Q has an absolute error of 2^-61, whatever d: G's is up to 2^-61 sum m Q^2, where FP64's is about 2^-53 of
 // the terms, sum m Q^2 |n|.  So a row whose stars (of its j-range, weighted by m Q^2) lie so far inside the softening
@@ -23,9 +23,9 @@
 // stars 1e-8 eps apart and alone kept 5e-11 of their force without that.  For one such pair to dominate a
 // row its stars have to be within 0.13 eps; of N = 65,536 stars at eps = 0.04 / N^(1/3), one in a hundred systems has one.
 //
-// The integer range covers the systems that k_prep has checked star by star (positions within
-// 2^24 eps, masses zero or 2^-32 .. 2^59 of the BH's, all finite); for any other
-// the same launch runs k_pair<double>'s block instead.
+// The integer range covers the systems that k_prep has checked star by star (fix::in_range: positions within
+// 2^24 eps, masses zero or 2^-32 .. 2^59 of the BH's, which is positive and not extreme, speeds up to that of light
+// and somewhat beyond, all finite); for any other the same launch runs k_pair<double>'s block instead.
 #pragma once
 
 #include "pn_fix.cuh"
