@@ -149,6 +149,24 @@ static void choose_packed(PairCfg *k, int nstar, int sms, int ipt_min = 1) {
     }
 }
 
+// j-range splits of a large Newtonian or energy sweep (tiles and row blocks of 256 stars): at least ten CTAs per SM, of a
+// number that is a multiple of the SMs' as nearly as may be, as they end when the last SM does, and with partial
+// sums (8 bytes each per star and split) of no more than 2^21 stars times one split, or 8 splits.  N = 65,536 Newtonian: 7,
+// 8, 9 and 16 splits 2,837, 2,884, 2,929 and 2,770 us; 80,000: 8, 16 and 18 4,255, 4,122 and 4,196.
+static int choose_whole(int nstar, int sms) {
+    const int nb = (nstar + 255) / 256, most = std::min({32, std::max(8, (1 << 21) / nstar), nb});
+    int best = most;
+    double cost = 1e300;
+    for (int g = 1; g <= most; ++g) {
+        const double per = (double)nb * g / sms, waste = std::ceil(per) / per + 0.0005 * g;
+        if ((per >= 10.0 || g == most) && waste < cost) {
+            cost = waste;
+            best = g;
+        }
+    }
+    return best;
+}
+
 // Tiles per CTA of the sweep over unordered pairs: about 6 CTAs per resident one (2 per SM), so that the last
 // ones end together, at most 8 tiles (a CTA's set-up is then a few percent of its time), and one tile
 // where that takes no more CTAs than are resident.  Measured, N = 6,000: 1 tile 70 us, 2 tiles 117;
@@ -217,15 +235,19 @@ static PairCfg choose_cfg(const pn_ctx *c, int mode, int nstar) {
         }
         // The Newtonian and the energy sweep need fewer registers and have more resident CTAs than that model, whose few
         // large CTAs leave them a long last wave: N = 20,000 Newtonian 322 us against 306 in the general shape below,
-        // 37,000 975 / 922, energy 1,454 / 1,365 (from 65,536 stars on that has too few splits, 2,884 / 2,771, and
-        // below 16,000 unequal ones: 13,750 170 / 158); and two stars per thread from N = 12,000 on (12,120 137 -> 131).
-        if (mode_has_force(mode) || nstar < 16000 || nstar >= 65536) {
+        // 37,000 975 / 922, energy 1,454 / 1,365, but below 16,000 unequal ones: 13,750 158 / 170; and two stars per
+        // thread from N = 12,000 on (12,120 137 -> 131).  From 65,536 stars on (below) by whole CTAs per SM.
+        if (mode_has_force(mode) || nstar < 16000) {
             choose_packed(&k, nstar, c->sms, mode_has_force(mode) || nstar < 12000 ? 1 : 2);
             k.x2 = k.ipt == 2 && mode_has_force(mode) ? 2 : 1;
             return k;
         }
         k.ipt = 2;
         k.x2 = 1;
+        if (nstar >= 65536) {
+            k.gsplit = choose_whole(nstar, c->sms);
+            return k;
+        }
     } else {
         k.x2 = 0;  // scalar sweep: FP64, PN_PAIR_SCALAR, or an explicit shape without the variant
     }
